@@ -37,6 +37,12 @@ struct DevThd {
   double Wc[IZEM_NSMAX], Wc_i[IZEM_NSMAX];
   double tpolymin[IZEM_NSMAX], tpolymax[IZEM_NSMAX], tpolylim[IZEM_NSMAX];
   double hc[IZEM_NSMAX][2][7];
+  // h_k and gam2 Wc_i,k cp_k/R as polynomials of the code-unit temperature,
+  // [range][species][power]; with tcommon every species shares the middle
+  // temperature tc_lim and is inside its own fit on [tc_lo, tc_hi) K
+  int tcommon;
+  double tc_lo, tc_lim, tc_hi;
+  double hk[2][IZEM_NSMAX][6], ck[2][IZEM_NSMAX][5];
   double cofd[IZEM_NSMAX][IZEM_NSMAX][IZEM_NPOLY];
   double coflam[IZEM_NSMAX][IZEM_NPOLY];
   double cofeta[IZEM_NSMAX][IZEM_NPOLY];

@@ -713,6 +713,27 @@ int izem_gpu_init(const izem_cfg* cfg, const izem_thd* thd, const izem_adi* adi,
     std::memcpy(h.cofeta[k], thd->cofeta[k], sizeof(h.cofeta[k]));
     h.Kd[k] = 1.0e-4 * thd->p0 / (thd->pinf * thd->dinf[k]);
   }
+  // the fits in code units: t = tinf T folded into the coefficients
+  h.tcommon = 1;
+  h.tc_lo = thd->tpolymin[0];
+  h.tc_hi = thd->tpolymax[0];
+  h.tc_lim = thd->tpolylim[0];
+  for (int k = 0; k < thd->nspc; ++k) {
+    h.tc_lo = std::max(h.tc_lo, thd->tpolymin[k]);
+    h.tc_hi = std::min(h.tc_hi, thd->tpolymax[k]);
+    if (thd->tpolylim[k] != h.tc_lim) h.tcommon = 0;
+    for (int r = 0; r < 2; ++r) {
+      const double* a = h.hc[k][r];
+      double tp = 1.0;   // tinf^j
+      for (int j = 0; j < 5; ++j) {
+        h.ck[r][k][j] = h.gam2 * h.Wc_i[k] * a[j] * tp;
+        h.hk[r][k][j] = h.Wc_i[k] * a[j] * tp / (j + 1);
+        tp *= h.tinf;
+      }
+      h.hk[r][k][5] = h.Wc_i[k] * a[5] / h.tinf;
+    }
+  }
+  if (!(h.tc_lo > 0.0 && h.tc_lo <= h.tc_lim && h.tc_lim <= h.tc_hi)) h.tcommon = 0;
   h.Kl = 0.5 * 1.0e-5 / thd->laminf;
   h.Ku = 1.0e-1 / thd->muinf;
   h.sqgmr = adi->sqgmr;

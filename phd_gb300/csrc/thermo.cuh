@@ -55,6 +55,35 @@ __device__ __forceinline__ double th_species(int is, double T, double* cpk) {
   }
 }
 
+// The range of the fits that holds at code temperature T: 0 or 1 when every
+// species takes its low or its high polynomial there, -1 when th_species has
+// to choose per species.  The comparisons are those of th_species, made on
+// the bit patterns (ordered like the values for positive doubles; negative
+// temperatures and NaN fall out of [lo, hi)) to leave the FP64 pipe alone.
+__device__ __forceinline__ int th_range(double T) {
+  const long long t = __double_as_longlong(T * c_thd.tinf);
+  if (!c_thd.tcommon || t < __double_as_longlong(c_thd.tc_lo) || t >= __double_as_longlong(c_thd.tc_hi)) return -1;
+  return t < __double_as_longlong(c_thd.tc_lim) ? 0 : 1;
+}
+// h_k and gam2 Wc_i,k cp_k/R inside the common range r: nine FP64 operations
+// a species (Horner's rule on the code-unit coefficients), against 35 of
+// th_species with its range tests and the caller's scaling
+__device__ __forceinline__ double th_h_fast(int r, int is, double T) {
+  const double* a = c_thd.hk[r][is];
+  return fma(T, fma(T, fma(T, fma(T, fma(T, a[4], a[3]), a[2]), a[1]), a[0]), a[5]);
+}
+__device__ __forceinline__ double th_cp_fast(int r, int is, double T) {
+  const double* a = c_thd.ck[r][is];
+  return fma(T, fma(T, fma(T, fma(T, a[4], a[3]), a[2]), a[1]), a[0]);
+}
+
+// th_species out of line, for the points outside the common range
+__device__ __noinline__ double2 th_species_call(int is, double T) {
+  double cpk;
+  const double h = th_species(is, T, &cpk);
+  return make_double2(h, cpk);
+}
+
 // cp_scalar: cp = sum_k Y_k gam2 Wc_i,k cp_k/R
 template <int NRV>
 __device__ __forceinline__ double th_cp_mix(double T, const double* Y) {
@@ -72,11 +101,20 @@ __device__ __forceinline__ double th_cp_mix(double T, const double* Y) {
 template <int NRV>
 __device__ __forceinline__ double th_cp_ha(double T, const double* Y, double* ha) {
   double cp = 0.0;
+  const int r = th_range(T);
+  if (r >= 0) {
+#pragma unroll
+    for (int is = 0; is < NRV; ++is) {
+      ha[is] = th_h_fast(r, is, T);
+      cp = fma(Y[is], th_cp_fast(r, is, T), cp);
+    }
+    return cp;
+  }
 #pragma unroll
   for (int is = 0; is < NRV; ++is) {
-    double cpk;
-    ha[is] = th_species(is, T, &cpk);
-    cp = cp + Y[is] * c_thd.gam2 * c_thd.Wc_i[is] * cpk;
+    const double2 q = th_species_call(is, T);
+    ha[is] = q.x;
+    cp = cp + Y[is] * c_thd.gam2 * c_thd.Wc_i[is] * q.y;
   }
   return cp;
 }
