@@ -26,6 +26,7 @@
 #include "../../include/izem_gpu.h"
 #include "chem.h"
 #include "atomics.cuh"
+#include "fmath.cuh"
 
 // This source builds two translation units, compiled in parallel:
 // IZEM_CHEM_UNIT 0 (chem.cu) holds the host side and the kernels that walk
@@ -50,7 +51,8 @@ __constant__ int c_need_eqk_dev;   // some reaction uses the equilibrium reverse
 // Mechanism constants of the device right-hand side (ck_fun_fast).
 struct ChemFast {
   double wt_inv[IZEM_NSMAX];          // 1 / W_k
-  double ru_wt[IZEM_NSMAX];           // RU / W_k
+  double cvp[IZEM_NSMAX][2][5];       // species c_v in powers of T (mass basis)
+  double up[IZEM_NSMAX][2][6];        // molar internal energy: RU T (..) of five powers, constant last
   double troe_inv[IZEM_MAXREAC][2];   // 1 / T***, 1 / T*
   double sri_cinv[IZEM_MAXREAC];      // 1 / c of the SRI form
 };
@@ -69,6 +71,7 @@ ChemFast c_fast_host;
 izem_mech c_mech_host;
 int c_need_eqk_host = 0;
 #define HD __host__ __device__
+#define HD_NOINLINE __host__ __device__ __noinline__
 #ifdef __CUDA_ARCH__
 #define c_mech c_mech_dev
 #define c_need_eqk c_need_eqk_dev
@@ -78,11 +81,71 @@ int c_need_eqk_host = 0;
 #endif
 #else
 #define HD __device__
+#define HD_NOINLINE __device__ __noinline__
 #define c_mech c_mech_dev
 #define c_need_eqk c_need_eqk_dev
 #endif
 
 constexpr int MXSP = 6;
+
+// Reciprocal, quotient and x^(1/l) of the integrator: on the device those of
+// fmath.cuh (5, 4 and 100 FP64 operations fewer than the library's), in a host
+// build the plain operations, which the oracle performs too.
+HD __forceinline__ double c_rcp(double x) {
+#ifdef __CUDA_ARCH__
+  return fm_rcp(x);
+#else
+  return 1.0 / x;
+#endif
+}
+HD __forceinline__ double c_div(double a, double x) {
+#ifdef __CUDA_ARCH__
+  return fm_div(a, x);
+#else
+  return a / x;
+#endif
+}
+__constant__ double c_inv_dev[9] = {0.0, 1.0, 0.5, 1.0 / 3.0, 0.25, 0.2, 1.0 / 6.0, 1.0 / 7.0, 0.125};
+// 1 / n, n = 1..8
+HD __forceinline__ double c_inv(int n) {
+#ifdef __CUDA_ARCH__
+  return c_inv_dev[n];
+#else
+  return 1.0 / double(n);
+#endif
+}
+HD __forceinline__ double c_root(double x, int n) {   // x^(1/n)
+#ifdef __CUDA_ARCH__
+  return fm_root(x, c_inv_dev[n]);
+#else
+  return pow(x, 1.0 / double(n));
+#endif
+}
+// exp and log of the right-hand side, one copy each in a kernel: inlined at
+// their 30 uses they push the BDF kernels out of the instruction cache
+#ifdef __CUDA_ARCH__
+__device__ __noinline__ double c_exp(double x) { return fm_exp(x); }
+__device__ __noinline__ double c_log(double x) { return fm_log(x); }
+#else
+inline double c_exp(double x) { return fm_exp(x); }
+inline double c_log(double x) { return fm_log(x); }
+#endif
+// |a| > b for b >= 0, and a != 0: comparisons of bit patterns on the device,
+// which the FP64 pipe would make at the price of an addition each
+HD __forceinline__ bool c_abs_gt(double a, double b) {
+#ifdef __CUDA_ARCH__
+  return __double_as_longlong(fabs(a)) > __double_as_longlong(b);
+#else
+  return fabs(a) > b;
+#endif
+}
+HD __forceinline__ bool c_nonzero(double a) {
+#ifdef __CUDA_ARCH__
+  return (__double_as_longlong(a) << 1) != 0;
+#else
+  return a != 0.0;
+#endif
+}
 // exponents of the Landau-Teller factor exp(B / T^(1/3) + C / T^(2/3))
 // (CKRATT's PM_V_1 and PM_V_2, vode.f:975-976)
 constexpr double kLtP1 = 1.0 / 3.0;
@@ -242,7 +305,17 @@ inline ChemFast chem_fast_constants(const izem_mech& m) {
   ChemFast f{};
   for (int k = 0; k < m.kk && k < IZEM_NSMAX; ++k) {
     f.wt_inv[k] = 1.0 / m.wt[k];
-    f.ru_wt[k] = m.ru / m.wt[k];
+    const double ru_wt = m.ru / m.wt[k];
+    for (int q = 0; q < 2; ++q) {
+      const double* a = m.a[k][q];
+      f.cvp[k][q][0] = ru_wt * (a[0] - 1.0);
+      f.up[k][q][0] = m.ru * (a[0] - 1.0);
+      for (int j = 1; j < 5; ++j) {
+        f.cvp[k][q][j] = ru_wt * a[j];
+        f.up[k][q][j] = m.ru * a[j] / double(j + 1);
+      }
+      f.up[k][q][5] = m.ru * a[5];
+    }
   }
   for (int i = 0; i < m.ii && i < IZEM_MAXREAC; ++i) {
     f.troe_inv[i][0] = m.troe[i][1] != 0.0 ? 1.0 / m.troe[i][1] : 0.0;
@@ -252,36 +325,56 @@ inline ChemFast chem_fast_constants(const izem_mech& m) {
   return f;
 }
 
-// The temperature-only terms of ck_fun_fast: species c_v and h, the forward
-// and reverse rate constants, and the fall-off low-pressure rates and
-// log10 F_cent.  The finite-difference Jacobian perturbs one variable per
-// column, so its nine species columns share the temperature of the call
-// before them and can reuse these terms (rc_drive).
+// What one reactor's right-hand sides share: its density, 1 / rho, and the
+// factors from mass fractions to concentrations.
+template <int KK>
+struct Cell {
+  double rho, rho_i;
+  double rw[KK];   // rho / W_k
+};
+template <int KK>
+HD __forceinline__ void cell_set(double rho, Cell<KK>& c) {
+  c.rho = rho;
+  c.rho_i = c_rcp(rho);
+#pragma unroll
+  for (int k = 0; k < KK; ++k) c.rw[k] = rho * c_fast.wt_inv[k];
+}
+
+// The temperature-only terms of ck_fun_fast: species c_v and internal
+// energies, the forward and reverse rate constants, and of a fall-off
+// reaction the ratio of its low- to its high-pressure rate constant and the
+// Troe terms that hold no concentration.  The finite-difference Jacobian
+// perturbs one variable per column, so its nine species columns share the
+// temperature of the call before them and can reuse these terms (rc_drive).
 template <int KK>
 struct FunT {
   double T;                                    // temperature the entries belong to
-  double rut;                                  // RU * T
-  double cvk[KK], h[KK];
+  double cvk[KK], u[KK];                       // c_v (mass), internal energy (molar)
   double kf[IZEM_MAXREAC], kr[IZEM_MAXREAC];   // before third-body and fall-off factors
-  double klow[IZEM_MAXREAC], fclog[IZEM_MAXREAC];
+  double kratio[IZEM_MAXREAC];
+  double lnfc[IZEM_MAXREAC];                   // ln F_cent (SRI: ln(a exp(-b/T) + exp(-T/c)))
+  double trc[IZEM_MAXREAC], trn[IZEM_MAXREAC]; // ln 10 (0.4 + 0.67 log10 F_cent), ln 10 (0.75 - 1.27 log10 F_cent)
 };
+
+constexpr double kLn10 = 2.302585092994045684, kInvLn10 = 0.4342944819032518277;
+constexpr double kTroeC = 0.4 * kLn10, kTroeN = 0.75 * kLn10;
 
 template <int KK>
 HD void fun_tpart(double T, FunT<KK>& t) {
-  const double Tinv = 1.0 / T;
-  const double alogt = log(T);
-  const double T2 = T * T, T3 = T * T2, T4 = T2 * T2;
+  const double Tinv = c_rcp(T);
+  const double alogt = c_log(T);
   t.T = T;
-  t.rut = T * c_mech.ru;
   double smh[KK];
 #pragma unroll
   for (int k = 0; k < KK; ++k) {
-    const double* a = c_mech.a[k][T > c_mech.tmid[k] ? 1 : 0];
-    const double cps = a[0] + T * a[1] + T2 * a[2] + T3 * a[3] + T4 * a[4];
-    t.cvk[k] = c_fast.ru_wt[k] * (cps - 1.0);
-    const double hs = a[0] + (0.5 * T) * a[1] + (T2 * (1.0 / 3.0)) * a[2] + (0.25 * T3) * a[3] + (0.2 * T4) * a[4];
-    t.h[k] = t.rut * (hs + a[5] * Tinv) * c_fast.wt_inv[k];
+    const int q = T > c_mech.tmid[k] ? 1 : 0;
+    const double* c = c_fast.cvp[k][q];
+    const double* e = c_fast.up[k][q];
+    t.cvk[k] = c[0] + T * (c[1] + T * (c[2] + T * (c[3] + T * c[4])));
+    t.u[k] = e[5] + T * (e[0] + T * (e[1] + T * (e[2] + T * (e[3] + T * e[4]))));
     if (c_need_eqk) {
+      const double* a = c_mech.a[k][q];
+      const double T2 = T * T, T3 = T * T2, T4 = T2 * T2;
       const double sv = (alogt - 1.0) * a[0] + (0.5 * T) * a[1] + (T2 * (1.0 / 6.0)) * a[2] +
                         (T3 * (1.0 / 12.0)) * a[3] + (T4 * 0.05) * a[4];
       smh[k] = sv + a[6] - a[5] * Tinv;
@@ -289,9 +382,9 @@ HD void fun_tpart(double T, FunT<KK>& t) {
   }
   const int ii = c_mech.ii;
   for (int i = 0; i < ii; ++i) {
-    double rkft = c_mech.par[i][0] * exp(c_mech.par[i][1] * alogt - c_mech.par[i][2] * Tinv);
+    double rkft = c_mech.par[i][0] * c_exp(c_mech.par[i][1] * alogt - c_mech.par[i][2] * Tinv);
     if (c_mech.lt[i][0] != 0.0 || c_mech.lt[i][1] != 0.0)   // Landau-Teller
-      rkft = rkft * exp(c_mech.lt[i][0] / pow(T, kLtP1) + c_mech.lt[i][1] / pow(T, kLtP2));
+      rkft = rkft * c_exp(c_mech.lt[i][0] / pow(T, kLtP1) + c_mech.lt[i][1] / pow(T, kLtP2));
     double rkrt = 0.0;
     const int rv = c_mech.rev[i];
     if (rv == 1) {
@@ -302,44 +395,54 @@ HD void fun_tpart(double T, FunT<KK>& t) {
         if (kk >= 0) sumsmh = sumsmh + double(c_mech.nu[i][n]) * smh[kk];
         nus += c_mech.nu[i][n];
       }
-      double eqk = sumsmh != 0.0 ? exp(fmin(sumsmh, 690.77552789821368)) : 1.0;
+      double eqk = sumsmh != 0.0 ? c_exp(fmin(sumsmh, 690.77552789821368)) : 1.0;
       eqk = eqk * powi(c_mech.patm * Tinv / c_mech.ru, nus);
-      rkrt = rkft / fmax(eqk, 1.0e-300);
+      rkrt = c_div(rkft, fmax(eqk, 1.0e-300));
     } else if (rv == 2) {
-      rkrt = c_mech.rpar[i][0] * exp(c_mech.rpar[i][1] * alogt - c_mech.rpar[i][2] * Tinv);
+      rkrt = c_mech.rpar[i][0] * c_exp(c_mech.rpar[i][1] * alogt - c_mech.rpar[i][2] * Tinv);
     }
     if (c_mech.rlt[i][0] != 0.0 || c_mech.rlt[i][1] != 0.0)   // reverse Landau-Teller
-      rkrt = rkrt * exp(c_mech.rlt[i][0] / pow(T, kLtP1) + c_mech.rlt[i][1] / pow(T, kLtP2));
+      rkrt = rkrt * c_exp(c_mech.rlt[i][0] / pow(T, kLtP1) + c_mech.rlt[i][1] / pow(T, kLtP2));
     t.kf[i] = rkft;
     t.kr[i] = rkrt;
     const int fo = c_mech.fall[i];
     if (fo) {
-      t.klow[i] = c_mech.low[i][0] * exp(c_mech.low[i][1] * alogt - c_mech.low[i][2] * Tinv);
-      if (fo == 2) {   // SRI: ln(a exp(-b/T) + exp(-T/c)) in the fclog slot
+      t.kratio[i] = c_div(c_mech.low[i][0] * c_exp(c_mech.low[i][1] * alogt - c_mech.low[i][2] * Tinv), rkft);
+      if (fo == 2) {
         const double* sr = c_mech.sri[i];
-        t.fclog[i] = log(sr[0] * exp(-sr[1] * Tinv) + exp(-T * c_fast.sri_cinv[i]));
+        t.lnfc[i] = c_log(sr[0] * c_exp(-sr[1] * Tinv) + c_exp(-T * c_fast.sri_cinv[i]));
       } else if (fo > 1) {
-        constexpr double kInvLn10 = 0.4342944819032518277;
         const double ta = c_mech.troe[i][0];
-        double fcent = (1.0 - ta) * exp(-T * c_fast.troe_inv[i][0]) + ta * exp(-T * c_fast.troe_inv[i][1]);
-        if (fo == 4) fcent = fcent + exp(-c_mech.troe[i][3] * Tinv);
-        t.fclog[i] = log(fmax(fcent, 1.0e-300)) * kInvLn10;
+        double fcent = (1.0 - ta) * c_exp(-T * c_fast.troe_inv[i][0]) + ta * c_exp(-T * c_fast.troe_inv[i][1]);
+        if (fo == 4) fcent = fcent + c_exp(-c_mech.troe[i][3] * Tinv);
+        const double lnfc = c_log(fmax(fcent, 1.0e-300));
+        t.lnfc[i] = lnfc;
+        t.trc[i] = kTroeC + 0.67 * lnfc;
+        t.trn[i] = kTroeN - 1.27 * lnfc;
       }
     }
   }
 }
 
+// Troe's broadening factor from ln P_r: with x = ln P_r - c and d = n - 0.14 x,
+// log F = log F_cent / (1 + (x / d)^2), the same in natural logarithms
+HD_NOINLINE double troe_factor(double pr, double lnfc, double trc, double trn) {
+  const double x = c_log(fmax(pr, 1.0e-300)) - trc;
+  const double d = trn - 0.14 * x;
+  const double d2 = d * d;
+  return c_exp(c_div(lnfc * d2, d2 + x * x));
+}
+
 // The composition-dependent rest of ck_fun_fast, from the temperature terms t.
 template <int KK>
-HD void fun_cpart(double rho, const double* z, const FunT<KK>& t, double* zp) {
-  constexpr double kLn10 = 2.302585092994045684, kInvLn10 = 0.4342944819032518277;
+HD void fun_cpart(const Cell<KK>& cell, const double* z, const FunT<KK>& t, double* zp) {
   const double* Y = z + 1;
   double cv = 0.0, C[KK], wdot[KK];
   double ctot = 0.0;
 #pragma unroll
   for (int k = 0; k < KK; ++k) {
     cv = cv + Y[k] * t.cvk[k];
-    C[k] = rho * Y[k] * c_fast.wt_inv[k];
+    C[k] = Y[k] * cell.rw[k];
     ctot = ctot + C[k];
     wdot[k] = 0.0;
   }
@@ -356,21 +459,15 @@ HD void fun_cpart(double rho, const double* z, const FunT<KK>& t, double* zp) {
     const int fo = c_mech.fall[i];
     if (fo) {
       const int kf = c_mech.kfal[i];   // collider: (+M), or species kf - 1 alone
-      const double pr = t.klow[i] * (kf ? C[kf - 1] : ctb) / rkft;
+      const double pr = t.kratio[i] * (kf ? C[kf - 1] : ctb);
       if (!kf) ctb = 1.0;
-      double pcor = pr / (1.0 + pr);
+      double pcor = c_div(pr, 1.0 + pr);
       if (fo == 2) {
-        const double prlog = log(fmax(pr, 1.0e-300)) * kInvLn10;
-        const double xp = 1.0 / (1.0 + prlog * prlog);
-        pcor = exp(xp * t.fclog[i]) * c_mech.sri[i][3] * pow(t.T, c_mech.sri[i][4]) * pcor;
+        const double prlog = c_log(fmax(pr, 1.0e-300)) * kInvLn10;
+        const double xp = c_rcp(1.0 + prlog * prlog);
+        pcor = c_exp(xp * t.lnfc[i]) * c_mech.sri[i][3] * pow(t.T, c_mech.sri[i][4]) * pcor;
       } else if (fo > 1) {
-        const double prlog = log(fmax(pr, 1.0e-300)) * kInvLn10;
-        const double fclog = t.fclog[i];
-        const double xn = 0.75 - 1.27 * fclog;
-        const double cprlog = prlog - (0.4 + 0.67 * fclog);
-        const double q = cprlog / (xn - 0.14 * cprlog);
-        const double flog = fclog / (1.0 + q * q);
-        pcor = exp(flog * kLn10) * pcor;
+        pcor = troe_factor(pr, t.lnfc[i], t.trc[i], t.trn[i]) * pcor;
       }
       rkft = rkft * pcor;
       rkrt = rkrt * pcor;
@@ -397,29 +494,33 @@ HD void fun_cpart(double rho, const double* z, const FunT<KK>& t, double* zp) {
       const int k = c_mech.nuk[i][n];
       if (k >= 0) wdot[k] = wdot[k] + rop[i] * double(c_mech.nu[i][n]);
     }
-  const double rho_i = 1.0 / rho;
   double sum = 0.0;
 #pragma unroll
   for (int k = 0; k < KK; ++k) {
-    zp[k + 1] = wdot[k] * c_mech.wt[k] * rho_i;
-    sum = sum + t.h[k] * wdot[k] * c_mech.wt[k] + (-t.rut) * wdot[k];
+    zp[k + 1] = wdot[k] * c_mech.wt[k] * cell.rho_i;
+    sum = sum + t.u[k] * wdot[k];
   }
-  zp[0] = -sum / (rho * cv);
+  zp[0] = -c_div(sum, cell.rho * cv);
 }
 
-// The constant-volume reactor right-hand side of ck_fun with the divisions
-// by T, by the molar masses and by the Troe and SRI temperatures replaced by
-// multiplications with reciprocals, and 10^x / log10 by exp / log: the same
-// CHEMKIN expressions (CKCVBS, CKHMS, CKRATT, CKRATX, CKWYR) with different
-// rounding (a few ulp per term) and about a sixth of the FP64 instructions
-// of the divisions.  The BDF kernels call it in two parts (fun_tpart,
+// The constant-volume reactor right-hand side of ck_fun with everything that
+// depends only on the mechanism, on the reactor or on the temperature moved
+// out of the composition part, the enthalpy and pressure terms of the energy
+// balance joined (u_k = h_k W_k - RU T), and the exponentials, logarithms and
+// quotients of fmath.cuh: the same CHEMKIN expressions (CKCVBS, CKHMS, CKRATT,
+// CKRATX, CKWYR) with different rounding (a few ulp per term).  The FP64 pipe
+// bounds the BDF kernels: 13.6 k -> 7.3 k FP64 instructions a reactor of the
+// mixing layer with this form and the integrator's quotients, 195 -> 114 ms a half
+// step of 7.5 M reactors.  The BDF kernels call it in two parts (fun_tpart,
 // fun_cpart); ck_fun above keeps the reference's operation order for the
 // host build that is compared with the oracle bit for bit.
 template <int KK>
 HD void ck_fun_fast(double rho, const double* z, double* zp) {
   FunT<KK> t;
+  Cell<KK> c;
+  cell_set<KK>(rho, c);
   fun_tpart<KK>(z[0], t);
-  fun_cpart<KK>(rho, z, t, zp);
+  fun_cpart<KK>(c, z, t, zp);
 }
 
 // The generated right-hand side: the shipped mechanism's, or another one
@@ -439,16 +540,18 @@ HD void ck_fun_fast(double rho, const double* z, double* zp) {
 template <int KK>
 struct RhsTables {
   using Terms = FunT<KK>;
+  static HD __forceinline__ void cell(double rho, Cell<KK>& c) { cell_set<KK>(rho, c); }
   static HD __forceinline__ void tpart(double T, Terms& t) { fun_tpart<KK>(T, t); }
-  static HD __forceinline__ void cpart(double rho, const double* z, const Terms& t, double* zp) {
-    fun_cpart<KK>(rho, z, t, zp);
+  static HD __forceinline__ void cpart(const Cell<KK>& c, const double* z, const Terms& t, double* zp) {
+    fun_cpart<KK>(c, z, t, zp);
   }
 };
 struct RhsGenerated {
   using Terms = chem_gen::FunT;
+  static HD __forceinline__ void cell(double rho, Cell<chem_gen::KK>& c) { chem_gen::cell_set(rho, c); }
   static HD __forceinline__ void tpart(double T, Terms& t) { chem_gen::tpart(T, t); }
-  static HD __forceinline__ void cpart(double rho, const double* z, const Terms& t, double* zp) {
-    chem_gen::cpart(rho, z, t, zp);
+  static HD __forceinline__ void cpart(const Cell<chem_gen::KK>& c, const double* z, const Terms& t, double* zp) {
+    chem_gen::cpart(c, z, t, zp);
   }
 };
 
@@ -473,7 +576,11 @@ HD __forceinline__ double dvnorm(const double* v, const double* w) {
   double s = 0.0;
 #pragma unroll
   for (int i = 0; i < N; ++i) { const double x = v[i] * w[i]; s = s + x * x; }
+#ifdef __CUDA_ARCH__
+  return sqrt(s * (1.0 / double(N)));
+#else
   return sqrt(s / double(N));
+#endif
 }
 
 // LINPACK DGEFA/DGESL (vode.f:7033/7630).  The outer loops stay rolled: the
@@ -487,24 +594,24 @@ HD int dgefa(double* a, int* ipvt) {
     int l = k;
     double dmax = fabs(a[k + k * N]);
     for (int i = k + 1; i < N; ++i) {
-      const double v = fabs(a[i + k * N]);
-      if (v > dmax) { dmax = v; l = i; }
+      const double v = a[i + k * N];
+      if (c_abs_gt(v, dmax)) { dmax = fabs(v); l = i; }
     }
     ipvt[k] = l;
-    if (a[l + k * N] == 0.0) { info = k + 1; continue; }
+    if (!c_nonzero(a[l + k * N])) { info = k + 1; continue; }
     if (l != k) { const double t = a[l + k * N]; a[l + k * N] = a[k + k * N]; a[k + k * N] = t; }
-    const double t = -1.0 / a[k + k * N];
+    const double t = -c_rcp(a[k + k * N]);
     for (int i = k + 1; i < N; ++i) a[i + k * N] = t * a[i + k * N];
 #pragma unroll 1
     for (int j = k + 1; j < N; ++j) {
       double tj = a[l + j * N];
       if (l != k) { a[l + j * N] = a[k + j * N]; a[k + j * N] = tj; }
-      if (tj != 0.0)
+      if (c_nonzero(tj))
         for (int i = k + 1; i < N; ++i) a[i + j * N] = a[i + j * N] + tj * a[i + k * N];
     }
   }
   ipvt[N - 1] = N - 1;
-  if (a[(N - 1) + (N - 1) * N] == 0.0) info = N;
+  if (!c_nonzero(a[(N - 1) + (N - 1) * N])) info = N;
   return info;
 }
 
@@ -515,14 +622,14 @@ HD void dgesl(const double* a, const int* ipvt, double* b) {
     const int l = ipvt[k];
     const double t = b[l];
     if (l != k) { b[l] = b[k]; b[k] = t; }
-    if (t != 0.0)
+    if (c_nonzero(t))
       for (int i = k + 1; i < N; ++i) b[i] = b[i] + t * a[i + k * N];
   }
 #pragma unroll 1
   for (int k = N - 1; k >= 0; --k) {
-    b[k] = b[k] / a[k + k * N];
+    b[k] = c_div(b[k], a[k + k * N]);
     const double t = -b[k];
-    if (t != 0.0)
+    if (c_nonzero(t))
       for (int i = 0; i < k; ++i) b[i] = b[i] + t * a[i + k * N];
   }
 }
@@ -538,17 +645,17 @@ HD void dvset(Dv<N>& d) {
   if (nq != 1) {
     for (int j = 1; j <= nq - 2; ++j) {
       hsum = hsum + d.tau[j - 1];
-      rxi = d.h / hsum;
-      alph0 = alph0 - 1.0 / double(j + 1);
+      rxi = c_div(d.h, hsum);
+      alph0 = alph0 - c_inv(j + 1);
       for (int iback = 1; iback <= j + 1; ++iback) {
         const int i = (j + 3) - iback;
         el[i - 1] = el[i - 1] + el[i - 2] * rxi;
       }
     }
-    alph0 = alph0 - 1.0 / double(nq);
+    alph0 = alph0 - c_inv(nq);
     rxis = -el[1] - alph0;
     hsum = hsum + d.tau[nq - 2];
-    rxi = d.h / hsum;
+    rxi = c_div(d.h, hsum);
     ahatn0 = -el[1] - rxi;
     for (int iback = 1; iback <= nq; ++iback) {
       const int i = (nq + 2) - iback;
@@ -557,19 +664,19 @@ HD void dvset(Dv<N>& d) {
   }
   const double t1 = 1.0 - ahatn0 + alph0;
   const double t2 = 1.0 + double(nq) * t1;
-  d.tq[1] = fabs(alph0 * t2 / t1);
-  d.tq[4] = fabs(t2 / (el[L - 1] * rxi / rxis));
+  d.tq[1] = fabs(c_div(alph0 * t2, t1));
+  d.tq[4] = fabs(c_div(t2, c_div(el[L - 1] * rxi, rxis)));
   if (d.nqwait == 1) {
-    const double cnqm1 = rxis / el[L - 1];
-    const double t3 = alph0 + 1.0 / double(nq);
+    const double cnqm1 = c_div(rxis, el[L - 1]);
+    const double t3 = alph0 + c_inv(nq);
     const double t4 = ahatn0 + rxi;
-    double elp = t3 / (1.0 - t4 + t3);
-    d.tq[0] = fabs(elp / cnqm1);
+    double elp = c_div(t3, 1.0 - t4 + t3);
+    d.tq[0] = fabs(c_div(elp, cnqm1));
     hsum = hsum + d.tau[nq - 1];
-    rxi = d.h / hsum;
-    const double t5 = alph0 - 1.0 / double(nq + 1);
+    rxi = c_div(d.h, hsum);
+    const double t5 = alph0 - c_inv(nq + 1);
     const double t6 = ahatn0 - rxi;
-    elp = t2 / (1.0 - t6 + t5);
+    elp = c_div(t2, 1.0 - t6 + t5);
     d.tq[2] = fabs(elp * rxi * (double(L) + 1.0) * t5);
   }
   d.tq[3] = 0.1 * d.tq[1];
@@ -644,6 +751,7 @@ enum : int {
 
 template <int N>
 struct Rc : Dv<N> {
+  Cell<N - 1> cell;                         // FUN's constants of this reactor (device)
   double y[N], fo[N];                       // FUN argument / result
   double tcur, tout;                        // REACTION_V's time and target
   double hg, hub, hlb, hnew;                // DVHIN
@@ -703,7 +811,7 @@ HD void rc_step_return(Rc<N>& r, int kflag) {
     return;
   }
   // DVINDY (K = 0)
-  const double s = (r.tout - r.tn) / r.h;
+  const double s = c_div(r.tout - r.tn, r.h);
   for (int i = 0; i < N; ++i) r.y[i] = r.yh[i + (r.l - 1) * N];
   for (int jb = 1; jb <= r.nq; ++jb) {
     const int j = r.nq - jb;
@@ -732,7 +840,7 @@ HD bool rc_nls_return(Rc<N>& r, int ret) {
     r.pc = ST_STEP_LOOP;
     return false;
   }
-  const double dsm = r.acnrm / r.tq[1];
+  const double dsm = c_div(r.acnrm, r.tq[1]);
   if (dsm <= 1.0) {
     r.kflag = 0;
     r.nst = r.nst + 1;
@@ -753,8 +861,7 @@ HD bool rc_nls_return(Rc<N>& r, int ret) {
       r.conp = r.tq[4];
     }
     if (r.etamax != 1.0) {
-      const double flotl = double(r.l);
-      r.etaq = 1.0 / (pow(6.0 * dsm, 1.0 / flotl) + 1.0e-6);
+      r.etaq = c_rcp(c_root(6.0 * dsm, r.l) + 1.0e-6);
       if (r.nqwait != 0) {
         r.eta = r.etaq;
         r.newq = r.nq;
@@ -764,15 +871,15 @@ HD bool rc_nls_return(Rc<N>& r, int ret) {
         if (r.nq != 1) {
           double col[N];
           for (int i = 0; i < N; ++i) col[i] = r.yh[i + (r.l - 1) * N];
-          const double ddn = dvnorm<N>(col, r.ewt) / r.tq[0];
-          r.etaqm1 = 1.0 / (pow(6.0 * ddn, 1.0 / (flotl - 1.0)) + 1.0e-6);
+          const double ddn = c_div(dvnorm<N>(col, r.ewt), r.tq[0]);
+          r.etaqm1 = c_rcp(c_root(6.0 * ddn, r.l - 1) + 1.0e-6);
         }
         double etaqp1 = 0.0;
         if (r.l != r.lmax) {
-          const double cnquot = (r.tq[4] / r.conp) * powi(r.h / r.tau[1], r.l);
+          const double cnquot = c_div(r.tq[4], r.conp) * powi(c_div(r.h, r.tau[1]), r.l);
           for (int i = 0; i < N; ++i) r.savf[i] = r.acor[i] - cnquot * r.yh[i + (r.lmax - 1) * N];
-          const double dup = dvnorm<N>(r.savf, r.ewt) / r.tq[2];
-          etaqp1 = 1.0 / (pow(10.0 * dup, 1.0 / (flotl + 1.0)) + 1.0e-6);
+          const double dup = c_div(dvnorm<N>(r.savf, r.ewt), r.tq[2]);
+          etaqp1 = c_rcp(c_root(10.0 * dup, r.l + 1) + 1.0e-6);
         }
         if (r.etaq >= etaqp1) {
           if (r.etaq < r.etaqm1) { r.eta = r.etaqm1; r.newq = r.nq - 1; }
@@ -790,7 +897,7 @@ HD bool rc_nls_return(Rc<N>& r, int ret) {
       r.newq = r.nq; r.newh = 0; r.eta = 1.0; r.hnew = r.h;
     }
     r.etamax = 10.0;   // ETAMX2 = ETAMX3 = 10
-    const double rr = 1.0 / r.tq[1];
+    const double rr = c_rcp(r.tq[1]);
     for (int i = 0; i < N; ++i) r.acor[i] = rr * r.acor[i];
     r.jstart = 1;
     rc_step_return(r, 0);
@@ -804,7 +911,7 @@ HD bool rc_nls_return(Rc<N>& r, int ret) {
     for (int i = r.nqnyh - jb * N; i < r.nqnyh; ++i) r.yh[i] = r.yh[i] - r.yh[i + N];
   r.etamax = 1.0;
   if (r.kflag > -3) {
-    r.eta = 1.0 / (pow(6.0 * dsm, 1.0 / double(r.l)) + 1.0e-6);
+    r.eta = c_rcp(c_root(6.0 * dsm, r.l) + 1.0e-6);
     r.eta = fmax(r.eta, 0.1);
     if (r.kflag <= -2 && r.eta > 0.2) r.eta = 0.2;
     r.sguard = r.sguard + 1;
@@ -876,7 +983,7 @@ HD bool rc_advance(Rc<N>& r) {
         for (int i = 0; i < N; ++i) r.yh[i] = r.y[i];
         r.nq = 1;
         r.h = 1.0;
-        for (int i = 0; i < N; ++i) r.ewt[i] = 1.0 / (kRtol * fabs(r.yh[i]) + kAtol);
+        for (int i = 0; i < N; ++i) r.ewt[i] = c_rcp(kRtol * fabs(r.yh[i]) + kAtol);
         // DVHIN
         const double tdist = fabs(r.tout - r.tcur);
         const double tround = kUround * fmax(fabs(r.tcur), fabs(r.tout));
@@ -886,7 +993,7 @@ HD bool rc_advance(Rc<N>& r) {
         for (int i = 0; i < N; ++i) {
           const double delyi = 0.1 * fabs(r.yh[i]) + kAtol;
           const double afi = fabs(r.yh[i + N]);
-          if (afi * r.hub > delyi) r.hub = delyi / afi;
+          if (afi * r.hub > delyi) r.hub = c_div(delyi, afi);
         }
         r.hg = sqrt(r.hlb * r.hub);
         r.hnew = r.hg;
@@ -902,13 +1009,18 @@ HD bool rc_advance(Rc<N>& r) {
       }
       case ST_HIN_F: {
         double ft[N];
+#ifdef __CUDA_ARCH__
+        const double hg_i = fm_rcp(r.hg);
+        for (int i = 0; i < N; ++i) ft[i] = (r.fo[i] - r.yh[i + N]) * hg_i;
+#else
         for (int i = 0; i < N; ++i) ft[i] = (r.fo[i] - r.yh[i + N]) / r.hg;
+#endif
         const double yddnrm = dvnorm<N>(ft, r.ewt);
-        r.hnew = (yddnrm * r.hub * r.hub > 2.0) ? sqrt(2.0 / yddnrm) : sqrt(r.hg * r.hub);
+        r.hnew = (yddnrm * r.hub * r.hub > 2.0) ? sqrt(c_div(2.0, yddnrm)) : sqrt(r.hg * r.hub);
         r.iter = r.iter + 1;
         bool done = r.iter >= 4;
         if (!done) {
-          const double hrat = r.hnew / r.hg;
+          const double hrat = c_div(r.hnew, r.hg);
           if (hrat > 0.5 && hrat < 2.0) done = true;
           else if (r.iter >= 2 && r.hnew > 2.0 * r.hg) { r.hnew = r.hg; done = true; }
         }
@@ -929,7 +1041,7 @@ HD bool rc_advance(Rc<N>& r) {
             rc_after_dvode(r, -1);
             break;
           }
-          for (int i = 0; i < N; ++i) r.ewt[i] = 1.0 / (kRtol * fabs(r.yh[i]) + kAtol);
+          for (int i = 0; i < N; ++i) r.ewt[i] = c_rcp(kRtol * fabs(r.yh[i]) + kAtol);
         }
         r.first = 0;
         if (kUround * dvnorm<N>(r.yh, r.ewt) > 1.0) {
@@ -990,8 +1102,8 @@ HD bool rc_advance(Rc<N>& r) {
         for (int jb = 1; jb <= r.nq; ++jb)
           for (int i = r.nqnyh - jb * N; i < r.nqnyh; ++i) r.yh[i] = r.yh[i] + r.yh[i + N];
         dvset<N>(r);
-        r.rl1 = 1.0 / r.el[1];
-        r.rc = r.rc * (r.rl1 / r.prl1);
+        r.rl1 = c_rcp(r.el[1]);
+        r.rc = r.rc * c_div(r.rl1, r.prl1);
         r.prl1 = r.rl1;
         // DVNLSD entry
         if (r.jstart == 0) r.nslp = 0;
@@ -1056,9 +1168,9 @@ HD bool rc_advance(Rc<N>& r) {
         // temperature column last (rc_drive reuses the temperature terms)
         const int j = (r.jcol + 1) % N;
         r.yj = r.y[j];
-        const double rj = fmax(srur * fabs(r.yj), r.r0 / r.ewt[j]);
+        const double rj = fmax(srur * fabs(r.yj), c_div(r.r0, r.ewt[j]));
         r.y[j] = r.y[j] + rj;
-        r.rfac = 1.0 / rj;
+        r.rfac = c_rcp(rj);
         r.pc = ST_JAC_COL_F;
         return true;
       }
@@ -1076,14 +1188,14 @@ HD bool rc_advance(Rc<N>& r) {
           for (int i = 0; i < N; ++i) r.y[i] = (r.rl1 * r.h) * r.savf[i] - (r.rl1 * r.yh[i + N] + r.acor[i]);
           dgesl<N>(r.wm, r.ipvt, r.y);
           if (r.rc != 1.0) {
-            const double cscale = 2.0 / (1.0 + r.rc);
+            const double cscale = c_div(2.0, 1.0 + r.rc);
             for (int i = 0; i < N; ++i) r.y[i] = cscale * r.y[i];
           }
           const double del = dvnorm<N>(r.y, r.ewt);
           for (int i = 0; i < N; ++i) r.acor[i] = r.acor[i] + r.y[i];
           for (int i = 0; i < N; ++i) r.y[i] = r.yh[i] + r.acor[i];
-          if (r.m != 0) r.crate = fmax(0.3 * r.crate, del / r.delp);
-          const double dcon = del * fmin(1.0, r.crate) / r.tq[3];
+          if (r.m != 0) r.crate = fmax(0.3 * r.crate, c_div(del, r.delp));
+          const double dcon = c_div(del * fmin(1.0, r.crate), r.tq[3]);
           if (dcon <= 1.0) {
             r.jcur = 0;
             r.icf = 0;
@@ -1176,6 +1288,7 @@ __device__ __forceinline__ void rc_drive(unsigned n, unsigned* counter, Load loa
       double rho, tf, z[N];
       load(q, rho, z, tf);
       rc_start<N>(r, rho, z, tf);
+      Rhs::cell(rho, r.cell);
       active = true;
       nfun = 0;
     }
@@ -1188,7 +1301,7 @@ __device__ __forceinline__ void rc_drive(unsigned n, unsigned* counter, Load loa
       // the warp wait for its slowest lane.  Reused terms are the bits the
       // recomputation would give.
       if (!__all_sync(__activemask(), r.y[0] == ft.T)) Rhs::tpart(r.y[0], ft);
-      Rhs::cpart(r.rho, r.y, ft, r.fo);
+      Rhs::cpart(r.cell, r.y, ft, r.fo);
     } else {
       store(q, r);
       active = false;
@@ -1263,21 +1376,27 @@ __global__ void k_chem_scatter(ChemField f, const double* T, const double* Y, Ch
 // CKWYR rates x molar mass x dt / rho, psr_simp_chemkin.f:31-42) and it is
 // neither the pure fuel nor the pure oxidiser (H2 and N2 both off by more
 // than 1e-6).  The selected reactors are appended to list.
-template <int KK>
+template <int KK, class Rhs>
 __global__ void k_chem_select(int n, const double* T, const double* rho, const double* Y, const double* dt,
                               ChemSkip sk, int* list, unsigned* count) {
   const int q = blockIdx.x * blockDim.x + threadIdx.x;
   if (q >= n) return;
-  double y[KK], w[KK];
+  // dY_k / dt at the initial state: production rate x molar mass / rho
+  double z[KK + 1], f[KK + 1];
+  z[0] = T[q];
 #pragma unroll
-  for (int l = 0; l < KK; ++l) y[l] = Y[(long long)q * KK + l];
-  ck_wyr<KK>(rho[q], T[q], y, w);
-  const double myc = dt[q] / rho[q];
+  for (int l = 0; l < KK; ++l) z[1 + l] = Y[(long long)q * KK + l];
+  typename Rhs::Terms t;
+  Cell<KK> cell;
+  Rhs::cell(rho[q], cell);
+  Rhs::tpart(z[0], t);
+  Rhs::cpart(cell, z, t, f);
+  const double dtq = dt[q];
   bool call_w = false;
 #pragma unroll
   for (int l = 0; l < KK; ++l)
-    if (fabs(w[l] * c_mech.wt[l] * myc) > 1.0e-12) call_w = true;
-  const double yh = y[sk.ih2], yn = y[sk.in2];
+    if (fabs(f[1 + l] * dtq) > 1.0e-12) call_w = true;
+  const double yh = Y[(long long)q * KK + sk.ih2], yn = Y[(long long)q * KK + sk.in2];
   const bool call_f = fabs(yh - sk.yf_h2) > 1.0e-6 && fabs(yn - sk.yf_n2) > 1.0e-6;
   const bool call_o = fabs(yh - sk.yo_h2) > 1.0e-6 && fabs(yn - sk.yo_n2) > 1.0e-6;
   if (call_w && call_f && call_o) list[atomicAdd(count, 1u)] = q;
@@ -1443,24 +1562,21 @@ struct GateArgs {
   int residual;                      // the networks predict the increment minus dt f(y0)
 };
 
-// Mean cv and species h at T (CKCVBS, CKHMS) with the reciprocal constants
-// of ck_fun_fast (the species loop of fun_tpart), and the mixture's specific
-// internal energy sum_k Y_k (h_k - RU T / W_k).  For the surrogate's decode:
-// a few ulp from Thermo's reference-order values, a third of its FP64 work.
+// Mean cv at T (CKCVBS) and the mixture's specific internal energy
+// sum_k Y_k u_k / W_k, with the polynomials of fun_tpart.  For the
+// surrogate's decode: a few ulp from Thermo's reference-order values, a
+// quarter of its FP64 work.
 template <int KK>
 __device__ __forceinline__ double thermo_fast_e(double T, const double* Y, double* cvb) {
-  const double Tinv = 1.0 / T;
-  const double T2 = T * T, T3 = T * T2, T4 = T2 * T2;
-  const double rut = T * c_mech.ru;
   double cv = 0.0, e = 0.0;
 #pragma unroll
   for (int k = 0; k < KK; ++k) {
-    const double* a = c_mech.a[k][T > c_mech.tmid[k] ? 1 : 0];
-    const double cps = a[0] + T * a[1] + T2 * a[2] + T3 * a[3] + T4 * a[4];
-    cv = cv + Y[k] * (c_fast.ru_wt[k] * (cps - 1.0));
-    const double hs = a[0] + (0.5 * T) * a[1] + (T2 * (1.0 / 3.0)) * a[2] + (0.25 * T3) * a[3] + (0.2 * T4) * a[4];
-    const double h = rut * (hs + a[5] * Tinv) * c_fast.wt_inv[k];
-    e = e + Y[k] * (h - c_fast.ru_wt[k] * T);
+    const int q = T > c_mech.tmid[k] ? 1 : 0;
+    const double* c = c_fast.cvp[k][q];
+    const double* a = c_fast.up[k][q];
+    cv = cv + Y[k] * (c[0] + T * (c[1] + T * (c[2] + T * (c[3] + T * c[4]))));
+    const double u = a[5] + T * (a[0] + T * (a[1] + T * (a[2] + T * (a[3] + T * a[4]))));
+    e = e + (Y[k] * c_fast.wt_inv[k]) * u;
   }
   *cvb = cv;
   return e;
@@ -1509,8 +1625,10 @@ __global__ void k_decode_gate(int n, const float* out, const float* out2, int ld
 #pragma unroll
     for (int k = 0; k < KK; ++k) z0[1 + k] = Y[(size_t)q * KK + k];
     typename Rhs::Terms t0;
+    Cell<KK> c0;
+    Rhs::cell(rho[q], c0);
     Rhs::tpart(T0, t0);
-    Rhs::cpart(rho[q], z0, t0, f0);
+    Rhs::cpart(c0, z0, t0, f0);
 #pragma unroll
     for (int k = 0; k < KK; ++k) dY[k] = dY[k] + dt[q] * f0[1 + k];
     dTp = dTp + dt[q] * f0[0];
@@ -1569,8 +1687,10 @@ __global__ void k_reactor_rhs(int n, const double* __restrict__ T, const double*
 #pragma unroll
   for (int k = 0; k < KK; ++k) z[1 + k] = Y[(size_t)q * KK + k];
   typename Rhs::Terms t;
+  Cell<KK> cell;
+  Rhs::cell(rho[q], cell);
   Rhs::tpart(z[0], t);
-  Rhs::cpart(rho[q], z, t, f);
+  Rhs::cpart(cell, z, t, f);
 #pragma unroll
   for (int c = 0; c <= KK; ++c) zdot[(size_t)q * (KK + 1) + c] = f[c];
 }
@@ -1719,7 +1839,8 @@ cudaError_t chem_launch_gather(const ChemField& f, double* T, double* rho, doubl
 cudaError_t chem_launch_select(int n, const double* T, const double* rho, const double* Y, const double* dt,
                                const ChemSkip& sk, int* list, unsigned* count, cudaStream_t s) {
   if (n <= 0) return cudaSuccess;
-  k_chem_select<9><<<(n + 127) / 128, 128, 0, s>>>(n, T, rho, Y, dt, sk, list, count);
+  auto kern = g_chem_gen ? k_chem_select<9, RhsGenerated> : k_chem_select<9, RhsTables<9>>;
+  kern<<<(n + 127) / 128, 128, 0, s>>>(n, T, rho, Y, dt, sk, list, count);
   return cudaGetLastError();
 }
 

@@ -12,204 +12,188 @@ constexpr int KK = 9;
 // species columns reuse them (rc_drive)
 struct FunT {
   double T;
-  double rut;
-  double cvk[9], h[9];
-  double kf[12];
-  double kr[6];   // reactions 0, 1, 2, 5, 7, 8
-  double klow[2];   // reactions 3, 11
-  double fclog[2];   // reactions 3, 11
+  double cvk[9], u[9];
+  double k[20];   // forward rate constants, then
+                 // reverse: k[12] of reaction 0, k[13] of reaction 1, k[14] of reaction 2, k[15] of reaction 5, k[16] of reaction 7, k[17] of reaction 8
+                 // low- over high-pressure: k[18] of reaction 3, k[19] of reaction 11
+  double lnfc[2], trc[2], trn[2];   // reactions 3, 11
 };
 
+HD __forceinline__ void cell_set(double rho, Cell<9>& c) {
+  c.rho = rho;
+  c.rho_i = c_rcp(rho);
+  c.rw[0] = rho * 0x1.fbf39e8ab06bdp-1;
+  c.rw[1] = rho * 0x1.fbf39e8ab06bdp-2;
+  c.rw[2] = rho * 0x1.000275060987dp-4;
+  c.rw[3] = rho * 0x1.000275060987dp-5;
+  c.rw[4] = rho * 0x1.e1ac6c774b6a9p-5;
+  c.rw[5] = rho * 0x1.c6b93cc1512cbp-5;
+  c.rw[6] = rho * 0x1.f0620d016f133p-6;
+  c.rw[7] = rho * 0x1.e1ac6c774b6a9p-6;
+  c.rw[8] = rho * 0x1.246e76057aa8cp-5;
+}
+
+// A, b, E/R of the Arrhenius expressions; c_v (5) and internal energy (6)
+// polynomials of the species below and above their middle temperature: in
+// constant memory, so that the loops over them stay small code
+#define CHEM_GEN_ARR {0x1.f438daa060000p+54, (-0x1.6666666666666p-1), 0x1.0c6f4493ef159p+13}, \
+  {0x1.8b50000000000p+15, 0x1.55c28f5c28f5cp+1, 0x1.8bb78dad5b973p+11}, \
+  {0x1.16f3220000000p+30, 0x1.4cccccccccccdp+0, 0x1.c94c533be761cp+10}, \
+  {0x1.0eaa664900000p+42, 0x1.c28f5c28f5c29p-2, 0.0}, \
+  {0x1.0191a36680000p+46, 0.0, 0x1.27e432c1d6dbcp+7}, \
+  {0x1.e31fa34e00000p+43, 0.0, 0x1.9da4e3b0f0481p+8}, \
+  {0x1.a48ce3be80000p+44, 0.0, (-0x1.f4328690d2d50p+7)}, \
+  {0x1.0f0cf064dd592p+75, (-0x1.0000000000000p+1), 0.0}, \
+  {0x1.20a871cc00200p+60, (-0x1.0000000000000p+0), 0.0}, \
+  {0x1.5f93037c00000p+41, 0.0, 0x1.5dbc4f266b3c5p+9}, \
+  {0x1.2dbf9ea000000p+37, 0x1.3851eb851eb85p-1, 0x1.784fcc6a9ac05p+13}, \
+  {0x1.6b99192fbb3c0p+64, (-0x1.63d70a3d70a3dp+0), 0x1.93845131294f1p+14}, \
+  {0x1.001d1bf800000p+46, (-0x1.0a3d70a3d70a4p-2), 0x1.1fd705d6afec6p+6}, \
+  {0x1.d970000000000p+14, 0x1.50a3d70a3d70ap+1, 0x1.3072327bb03a1p+11}, \
+  {0x1.7d78400000000p+33, 0x1.30a3d70a3d70ap+0, 0x1.2611369490098p+13}, \
+  {0x1.39283f4a00000p+41, 0x1.70a3d70a3d70ap-2, 0x1.b3c1120ab0336p+14}, \
+  {0x1.5cfa424ea9c92p+76, (-0x1.c000000000000p+0), 0x1.d22edd4d65d8ep+15}, \
+  {0x1.0e0198eaee000p+58, (-0x1.4cccccccccccdp-1), 0x1.96e5d98de8289p+15}, \
+  {0x1.8efc84ad0c7b0p+65, (-0x1.6666666666666p+0), 0.0}, \
+  {0x1.592a7a2071df8p+79, (-0x1.e666666666666p+0), 0x1.8626719ec5abbp+14}
+#define CHEM_GEN_NASA {{0x1.d7ff8e3825f4ap+26, 0x1.e80f506d97176p-15, (-0x1.618f1f2124b19p-23), 0x1.a159b3e796e12p-33, (-0x1.58a5073e4b9eap-44), 0x1.dbc2948000000p+26, 0x1.ebf31bfc7e509p-16, (-0x1.db2b52f348540p-25), 0x1.a4ad3a7f28bafp-35, (-0x1.15e9c4e98a5f0p-46), 0x1.ed233bd1877d7p+40},\
+   {0x1.a703bf36dacefp+25, 0x1.416ed353acc12p+18, (-0x1.91ad45f2464bap+9), 0x1.a9a81b1e64e16p-1, (-0x1.3eff45c69d9bbp-12), 0x1.aa62d459f3e8ap+26, 0x1.43fea64415103p+18, (-0x1.0deb369d99cf1p+9), 0x1.ad0c943d898adp-2, (-0x1.013b4d2d53f55p-13), (-0x1.1c5226d289a30p+36)},\
+   {0x1.57df0702624b6p+23, (-0x1.0a4760fffc8a1p+14), 0x1.142df148e6721p+5, (-0x1.04e222e912be3p-5), 0x1.7064d5077b11cp-17, 0x1.57dbba1b66128p+27, (-0x1.0a44d2be9b351p+17), 0x1.7039b8f006229p+7, (-0x1.04dfa1e972f78p-3), 0x1.26b43cb2fc852p-15, 0x1.19e28b1840f5cp+41},\
+   {0x1.b946efc4d2fdfp+22, (-0x1.e6aa8d36d2990p+12), 0x1.99648ecb16b96p+4, (-0x1.9c26a8265042ep-6), 0x1.1acfc9fa7224ep-17, 0x1.b942b38987df5p+27, (-0x1.e6a5e175c5a15p+16), 0x1.10eb15ef57eafp+8, (-0x1.9c22b37b551ccp-3), 0x1.c47b51c30b00dp-15, (-0x1.498ba52fa8e56p+36)},\
+   {0x1.be638f3b2cda6p+23, (-0x1.6edbe390f33afp+13), 0x1.69376e7fc9e9ap+4, (-0x1.36de921e0dd57p-6), 0x1.bf89d27355702p-18, 0x1.da7e6bc41fe43p+27, (-0x1.85f4e485c392bp+16), 0x1.fff1fd1306df8p+6, (-0x1.4a7123c5a5705p-4), 0x1.7c92918263fc0p-16, 0x1.17eef572b5062p+38},\
+   {0x1.c283f5413bf48p+23, (-0x1.25b50a5c47d8cp+13), 0x1.e17dce03933eep+4, (-0x1.9efa92b9c77c9p-6), 0x1.12695e1c4f3e1p-17, 0x1.fb430727354c2p+27, (-0x1.4ab3c229620eap+16), 0x1.696d238bf995fp+7, (-0x1.d33fbf6ec423bp-4), 0x1.ee5c9ff7dc3cep-16, (-0x1.253957b89215cp+41)},\
+   {0x1.fba6572f0804bp+22, (-0x1.75d97aeff7d43p+13), 0x1.aa631fd8dde89p+5, (-0x1.f4f71fad691fap-5), 0x1.88b6573d98807p-16, 0x1.05cf845b8a3e7p+28, (-0x1.819c8661bf38cp+17), 0x1.25338b451e123p+9, (-0x1.025cfd6548c8cp-1), 0x1.440dd8e369053p-13, 0x1.6d41439fa6a7fp+34},\
+   {0x1.e8c63adc28e02p+22, (-0x1.4bb7770fc3119p+10), 0x1.4739e99066e29p+5, (-0x1.b0116b1462c59p-5), 0x1.61b13612ab5e8p-16, 0x1.03c620d38a85cp+28, (-0x1.609a0c5c905d5p+14), 0x1.cfc57df369b17p+8, (-0x1.cb4575097b96ap-2), 0x1.2cc4cbc47d3f0p-13, (-0x1.56b30f9872b5cp+40)},\
+   {0x1.a06ada57d4d7ap+22, 0x1.053b974b3ad43p+12, (-0x1.786ac086d4cc8p+3), 0x1.12569ebcaabd9p-6, (-0x1.e6f8bd3e66063p-18), 0x1.6c8a22210be0ep+27, 0x1.c96049f42c623p+15, (-0x1.b75d027f34893p+6), 0x1.e05266401eba5p-4, (-0x1.550b13d1e1e8ap-15), (-0x1.3c3691c537d71p+36)}}, \
+  {{0x1.d7ff8e6cf0bc7p+26, (-0x1.f32aafd504c46p-10), 0x1.65bd8cc3415b3p-20, (-0x1.ad75cad3044dep-32), 0x1.7226f20725a00p-45, 0x1.dbc294b5367e4p+26, (-0x1.f72524c339726p-11), 0x1.e0c9efcea8c6bp-22, (-0x1.b0e20692518c4p-34), 0x1.2a7b56674e2dap-47, 0x1.ed233bd1877d7p+40},\
+   {0x1.6fbb06f3e5b32p+26, (-0x1.fd630b8827036p+10), 0x1.49979c41dcaacp+4, (-0x1.e55c2eb4b1988p-8), 0x1.bb6af52ee8c1dp-21, 0x1.72a95019fb3fap+27, (-0x1.00b92d53b22a4p+11), 0x1.baf5714c0eafbp+3, (-0x1.e93a782375008p-9), 0x1.658fbc3f4a5acp-22, (-0x1.264d47d19950bp+36)},\
+   {0x1.f1cc1306e88bfp+22, (-0x1.bec9823789650p+8), 0x1.be74cdd8008b8p-3, (-0x1.b4b6123cca757p-15), 0x1.b6a98c2072389p-28, 0x1.f1c74bec7dcbfp+26, (-0x1.bec538726c729p+11), 0x1.29a05897572fdp+0, (-0x1.b4b1e1396fa60p-13), 0x1.5eeaab74b0bd7p-26, 0x1.1acebcf72db48p+41},\
+   {0x1.69fe630cc6790p+22, 0x1.e1b415c971e27p+11, (-0x1.f830494f6138ep+0), 0x1.1d5ca031a53e9p-11, (-0x1.e3b66c62314f8p-25), 0x1.69fae99ebd1aap+27, 0x1.e1af7639f85a8p+15, (-0x1.501cf7007e109p+4), 0x1.1d59e30d0fa49p-8, (-0x1.82f49fe8c734fp-22), (-0x1.5123747d72c09p+36)},\
+   {0x1.383eb7ca8f9e3p+23, 0x1.4f24ac9f858fbp+11, 0x1.3ca61bd3dea24p-1, (-0x1.c2d5666ade5a7p-12), 0x1.ed105d8b5cab2p-25, 0x1.4be775538ca1dp+27, 0x1.643e7cb67d8dcp+14, 0x1.c0c7c61421cf8p+1, (-0x1.df37e693eaa6fp-10), 0x1.a349399963805p-23, 0x1.2acb74dfcaccdp+38},\
+   {0x1.1e7ac2e3eb2b5p+23, 0x1.39f7f9e39dfb2p+13, (-0x1.83b428cf6d1aap-1), (-0x1.d5a0b6e0c088ap-12), 0x1.4d69be610f4bap-24, 0x1.42906b9f5e9c1p+27, 0x1.618408b867c3ap+16, (-0x1.23068f00b550cp+2), (-0x1.086408eea1af8p-9), 0x1.2c53d604820a8p-22, (-0x1.226c28fd1c9aep+41)},\
+   {0x1.cfe50765d5f3fp+22, 0x1.60a2d88e7926dp+12, (-0x1.98a0e352280dap+0), 0x1.2dc519b6f1b6fp-12, (-0x1.d2fde84bdced8p-26), 0x1.de7d4fc00d068p+27, 0x1.6bbb08cadcb91p+16, (-0x1.18fd5d80accffp+4), 0x1.37439ab3dda05p-9, (-0x1.8158e87f20091p-23), 0x1.152bf1da0734dp+33},\
+   {0x1.d8328e3a08eebp+22, 0x1.76ee81a4eb6b3p+13, (-0x1.29747758d3647p+2), 0x1.dbb2980f7ec1ap-11, (-0x1.2e431299c67ecp-24), 0x1.f5ed65ced5474p+27, 0x1.8e89a02e0194ap+17, (-0x1.a593c329d7eecp+5), 0x1.f9a5d9eb3b548p-8, (-0x1.0108b9f4bd6f4p-21), (-0x1.59c80eb64f452p+40)},\
+   {0x1.5d055c59fd85cp+22, 0x1.14062c7d74511p+12, (-0x1.aff084fd00f68p+0), 0x1.3a3e0c993c2fbp-12, (-0x1.585b9e0d0a636p-26), 0x1.318a1a6ed9168p+27, 0x1.e345fad6614b2p+15, (-0x1.f82bac86184e0p+3), 0x1.1317fa46cc62bp-9, (-0x1.e254ecbc085e2p-24), (-0x1.1dd3b7ba6451fp+36)}}
+__constant__ double arr_dev[20][3] = {CHEM_GEN_ARR};
+__constant__ double nasa_dev[2][9][11] = {CHEM_GEN_NASA};
+#ifdef __CUDA_ARCH__
+#define CHEM_GEN_TAB(x) x##_dev
+#else
+static const double arr_host[20][3] = {CHEM_GEN_ARR};
+static const double nasa_host[2][9][11] = {CHEM_GEN_NASA};
+#define CHEM_GEN_TAB(x) x##_host
+#endif
+
 HD __forceinline__ void tpart(double T, FunT& t) {
-  const double Tinv = 1.0 / T;
-  const double alogt = log(T);
-  const double T2 = T * T, T3 = T * T2, T4 = T2 * T2;
+  const double Tinv = c_rcp(T);
+  const double alogt = c_log(T);
   t.T = T;
-  t.rut = T * 0x1.3d2c630000000p+26;
+  const int hi0 = T > 0x1.f400000000000p+9 ? 1 : 0;
   {   // species 0
-    const bool hi = T > 0x1.f400000000000p+9;
-    const double a0 = hi ? 0x1.40000015798eep+1 : 0x1.4000000000000p+1;
-    const double a1 = hi ? (-0x1.961a6ec6a1e45p-36) : 0x1.8d112bff6d580p-41;
-    const double a2 = hi ? 0x1.230b4c341c642p-46 : (-0x1.1fa470055807fp-49);
-    const double a3 = hi ? (-0x1.5d647fbe2e672p-58) : 0x1.538a620b2373fp-59;
-    const double a4 = hi ? 0x1.2d244e9510ba2p-71 : (-0x1.1863cffe0b329p-70);
-    const double a5 = hi ? 0x1.8e06a3bcd35a8p+14 : 0x1.8e06a3bcd35a8p+14;
-    const double cps = a0 + T * a1 + T2 * a2 + T3 * a3 + T4 * a4;
-    t.cvk[0] = 0x1.3aaa5ed0194dcp+26 * (cps - 1.0);
-    const double hs = a0 + (0.5 * T) * a1 + (T2 * (1.0 / 3.0)) * a2 + (0.25 * T3) * a3 + (0.2 * T4) * a4;
-    t.h[0] = t.rut * (hs + a5 * Tinv) * 0x1.fbf39e8ab06bdp-1;
+    const double* c = CHEM_GEN_TAB(nasa)[hi0][0];
+    t.cvk[0] = c[0] + T * (c[1] + T * (c[2] + T * (c[3] + T * c[4])));
+    t.u[0] = c[10] + T * (c[5] + T * (c[6] + T * (c[7] + T * (c[8] + T * c[9]))));
   }
   {   // species 1
-    const bool hi = T > 0x1.f400000000000p+9;
-    const double a0 = hi ? 0x1.ab2bf6fecf7e5p+1 : 0x1.2c130ac9b2911p+1;
-    const double a1 = hi ? (-0x1.9e6b00cea2ba4p-15) : 0x1.058175d02a941p-7;
-    const double a2 = hi ? 0x1.0c24d11e93b22p-21 : (-0x1.46ca05831775cp-16);
-    const double a3 = hi ? (-0x1.8adee4a4b6baep-33) : 0x1.5a4c582f87e3dp-26;
-    const double a4 = hi ? 0x1.68bf7de4136dcp-46 : (-0x1.03862939e564dp-37);
-    const double a5 = hi ? (-0x1.db14578e5c4ebp+9) : (-0x1.caf7b3bfb58d1p+9);
-    const double cps = a0 + T * a1 + T2 * a2 + T3 * a3 + T4 * a4;
-    t.cvk[1] = 0x1.3aaa5ed0194dcp+25 * (cps - 1.0);
-    const double hs = a0 + (0.5 * T) * a1 + (T2 * (1.0 / 3.0)) * a2 + (0.25 * T3) * a3 + (0.2 * T4) * a4;
-    t.h[1] = t.rut * (hs + a5 * Tinv) * 0x1.fbf39e8ab06bdp-2;
+    const double* c = CHEM_GEN_TAB(nasa)[hi0][1];
+    t.cvk[1] = c[0] + T * (c[1] + T * (c[2] + T * (c[3] + T * c[4])));
+    t.u[1] = c[10] + T * (c[5] + T * (c[6] + T * (c[7] + T * (c[8] + T * c[9]))));
   }
   {   // species 2
-    const bool hi = T > 0x1.f400000000000p+9;
-    const double a0 = hi ? 0x1.48e2c7b5e1a3dp+1 : 0x1.9589c6bdbf12dp+1;
-    const double a1 = hi ? (-0x1.689a006cdb509p-14) : (-0x1.add3ae5787a18p-9);
-    const double a2 = hi ? 0x1.6855a2fbdda5cp-25 : 0x1.bdcef845b6ae0p-18;
-    const double a3 = hi ? (-0x1.607823c010ceap-37) : (-0x1.a51e14d5c0503p-28);
-    const double a4 = hi ? 0x1.620b4436bd152p-50 : 0x1.2954967e1b470p-39;
-    const double a5 = hi ? 0x1.c88650ff97247p+14 : 0x1.c709096bb98c8p+14;
-    const double cps = a0 + T * a1 + T2 * a2 + T3 * a3 + T4 * a4;
-    t.cvk[2] = 0x1.3d2f6e558a183p+22 * (cps - 1.0);
-    const double hs = a0 + (0.5 * T) * a1 + (T2 * (1.0 / 3.0)) * a2 + (0.25 * T3) * a3 + (0.2 * T4) * a4;
-    t.h[2] = t.rut * (hs + a5 * Tinv) * 0x1.000275060987dp-4;
+    const double* c = CHEM_GEN_TAB(nasa)[hi0][2];
+    t.cvk[2] = c[0] + T * (c[1] + T * (c[2] + T * (c[3] + T * c[4])));
+    t.u[2] = c[10] + T * (c[5] + T * (c[6] + T * (c[7] + T * (c[8] + T * c[9]))));
   }
   {   // species 3
-    const bool hi = T > 0x1.f400000000000p+9;
-    const double a0 = hi ? 0x1.a42a332f575b8p+1 : 0x1.e42787ae5fa45p+1;
-    const double a1 = hi ? 0x1.84c851ecf574dp-10 : (-0x1.88c9b66c8c0dfp-9);
-    const double a2 = hi ? (-0x1.96ee255022a3dp-21) : 0x1.4a6bae1fdae75p-17;
-    const double a3 = hi ? 0x1.cca1706e20348p-33 : (-0x1.4ca5927ada53cp-27);
-    const double a4 = hi ? (-0x1.8667712a69c18p-46) : 0x1.c883a18b02bcdp-39;
-    const double a5 = hi ? (-0x1.101d4b48d3ae7p+10) : (-0x1.09fc63497b741p+10);
-    const double cps = a0 + T * a1 + T2 * a2 + T3 * a3 + T4 * a4;
-    t.cvk[3] = 0x1.3d2f6e558a183p+21 * (cps - 1.0);
-    const double hs = a0 + (0.5 * T) * a1 + (T2 * (1.0 / 3.0)) * a2 + (0.25 * T3) * a3 + (0.2 * T4) * a4;
-    t.h[3] = t.rut * (hs + a5 * Tinv) * 0x1.000275060987dp-5;
+    const double* c = CHEM_GEN_TAB(nasa)[hi0][3];
+    t.cvk[3] = c[0] + T * (c[1] + T * (c[2] + T * (c[3] + T * c[4])));
+    t.u[3] = c[10] + T * (c[5] + T * (c[6] + T * (c[7] + T * (c[8] + T * c[9]))));
   }
   {   // species 4
-    const bool hi = T > 0x1.f400000000000p+9;
-    const double a0 = hi ? 0x1.8be3be406d029p+1 : 0x1.fefa5c927d1abp+1;
-    const double a1 = hi ? 0x1.1f88fd8e1440ep-11 : (-0x1.3abed86e71c7dp-9);
-    const double a2 = hi ? 0x1.0faafc0d73234p-23 : 0x1.35e793e99fbcdp-18;
-    const double a3 = hi ? (-0x1.82ca91827ab6dp-34) : (-0x1.0ab59e9e67441p-28);
-    const double a4 = hi ? 0x1.a705cd746f5f8p-47 : 0x1.7ff6d2c211dd3p-40;
-    const double a5 = hi ? 0x1.e2550624dd2f2p+11 : 0x1.c3e293f290abbp+11;
-    const double cps = a0 + T * a1 + T2 * a2 + T3 * a3 + T4 * a4;
-    t.cvk[4] = 0x1.2a63031c056b1p+22 * (cps - 1.0);
-    const double hs = a0 + (0.5 * T) * a1 + (T2 * (1.0 / 3.0)) * a2 + (0.25 * T3) * a3 + (0.2 * T4) * a4;
-    t.h[4] = t.rut * (hs + a5 * Tinv) * 0x1.e1ac6c774b6a9p-5;
+    const double* c = CHEM_GEN_TAB(nasa)[hi0][4];
+    t.cvk[4] = c[0] + T * (c[1] + T * (c[2] + T * (c[3] + T * c[4])));
+    t.u[4] = c[10] + T * (c[5] + T * (c[6] + T * (c[7] + T * (c[8] + T * c[9]))));
   }
   {   // species 5
-    const bool hi = T > 0x1.f400000000000p+9;
-    const double a0 = hi ? 0x1.8459ddac6e07ap+1 : 0x1.0cb686e536fbfp+2;
-    const double a1 = hi ? 0x1.1d553f9364039p-9 : (-0x1.0aeb63b84c925p-9);
-    const double a2 = hi ? (-0x1.6057d217698d4p-23) : 0x1.b593a7c039b70p-18;
-    const double a3 = hi ? (-0x1.aacb906a5f7ccp-34) : (-0x1.7921667072d59p-28);
-    const double a4 = hi ? 0x1.2f01042cd6ffep-46 : 0x1.f2c47bce627b1p-40;
-    const double a5 = hi ? (-0x1.d4d1303afb7e9p+14) : (-0x1.d956e8240b780p+14);
-    const double cps = a0 + T * a1 + T2 * a2 + T3 * a3 + T4 * a4;
-    t.cvk[5] = 0x1.19b11bf5ba9e9p+22 * (cps - 1.0);
-    const double hs = a0 + (0.5 * T) * a1 + (T2 * (1.0 / 3.0)) * a2 + (0.25 * T3) * a3 + (0.2 * T4) * a4;
-    t.h[5] = t.rut * (hs + a5 * Tinv) * 0x1.c6b93cc1512cbp-5;
+    const double* c = CHEM_GEN_TAB(nasa)[hi0][5];
+    t.cvk[5] = c[0] + T * (c[1] + T * (c[2] + T * (c[3] + T * c[4])));
+    t.u[5] = c[10] + T * (c[5] + T * (c[6] + T * (c[7] + T * (c[8] + T * c[9]))));
   }
   {   // species 6
-    const bool hi = T > 0x1.f400000000000p+9;
-    const double a0 = hi ? 0x1.0119fbbf289f6p+2 : 0x1.1350a899bcaa1p+2;
-    const double a1 = hi ? 0x1.2593e46a1f9dfp-9 : (-0x1.373d054674594p-8);
-    const double a2 = hi ? (-0x1.5431502070c84p-21) : 0x1.62fa28e3a8ea6p-16;
-    const double a3 = hi ? 0x1.f675fa32f618cp-34 : (-0x1.a110b0905e0fcp-26);
-    const double a4 = hi ? (-0x1.84c80e71ea191p-47) : 0x1.46f1288fc5c1cp-37;
-    const double a5 = hi ? 0x1.bf6d462c343b7p+6 : 0x1.26cedbb59ddc2p+8;
-    const double cps = a0 + T * a1 + T2 * a2 + T3 * a3 + T4 * a4;
-    t.cvk[6] = 0x1.337fbd7576e8bp+21 * (cps - 1.0);
-    const double hs = a0 + (0.5 * T) * a1 + (T2 * (1.0 / 3.0)) * a2 + (0.25 * T3) * a3 + (0.2 * T4) * a4;
-    t.h[6] = t.rut * (hs + a5 * Tinv) * 0x1.f0620d016f133p-6;
+    const double* c = CHEM_GEN_TAB(nasa)[hi0][6];
+    t.cvk[6] = c[0] + T * (c[1] + T * (c[2] + T * (c[3] + T * c[4])));
+    t.u[6] = c[10] + T * (c[5] + T * (c[6] + T * (c[7] + T * (c[8] + T * c[9]))));
   }
   {   // species 7
-    const bool hi = T > 0x1.f400000000000p+9;
-    const double a0 = hi ? 0x1.0a8f681d1fcb7p+2 : 0x1.11abd48f63e0ap+2;
-    const double a1 = hi ? 0x1.41abe4bc5704bp-8 : (-0x1.1c98643a78c6ap-11);
-    const double a2 = hi ? (-0x1.fe66ae3495cc5p-20) : 0x1.18be22e62f026p-16;
-    const double a3 = hi ? 0x1.981f91177d524p-32 : (-0x1.72b101d35ae59p-26);
-    const double a4 = hi ? (-0x1.0353229ef325dp-45) : 0x1.2f72fba30b7c2p-37;
-    const double a5 = hi ? (-0x1.1717269ad42c4p+14) : (-0x1.149a541205bc0p+14);
-    const double cps = a0 + T * a1 + T2 * a2 + T3 * a3 + T4 * a4;
-    t.cvk[7] = 0x1.2a63031c056b1p+21 * (cps - 1.0);
-    const double hs = a0 + (0.5 * T) * a1 + (T2 * (1.0 / 3.0)) * a2 + (0.25 * T3) * a3 + (0.2 * T4) * a4;
-    t.h[7] = t.rut * (hs + a5 * Tinv) * 0x1.e1ac6c774b6a9p-6;
+    const double* c = CHEM_GEN_TAB(nasa)[hi0][7];
+    t.cvk[7] = c[0] + T * (c[1] + T * (c[2] + T * (c[3] + T * c[4])));
+    t.u[7] = c[10] + T * (c[5] + T * (c[6] + T * (c[7] + T * (c[8] + T * c[9]))));
   }
   {   // species 8
-    const bool hi = T > 0x1.f400000000000p+9;
-    const double a0 = hi ? 0x1.769c23b7952d2p+1 : 0x1.a63b0c4588a05p+1;
-    const double a1 = hi ? 0x1.86106ec5d7fc6p-10 : 0x1.712969da04050p-10;
-    const double a2 = hi ? (-0x1.3132bf1b89c39p-21) : (-0x1.09f7a2b098bd4p-18);
-    const double a3 = hi ? 0x1.bc128a9b8a724p-34 : 0x1.83ae94da0fe59p-28;
-    const double a4 = hi ? (-0x1.e6a15668d1fd9p-48) : (-0x1.581526048e0d6p-39);
-    const double a5 = hi ? (-0x1.cd661b089a027p+9) : (-0x1.fe732fec56d5dp+9);
-    const double cps = a0 + T * a1 + T2 * a2 + T3 * a3 + T4 * a4;
-    t.cvk[8] = 0x1.6a4f7c37c9782p+21 * (cps - 1.0);
-    const double hs = a0 + (0.5 * T) * a1 + (T2 * (1.0 / 3.0)) * a2 + (0.25 * T3) * a3 + (0.2 * T4) * a4;
-    t.h[8] = t.rut * (hs + a5 * Tinv) * 0x1.246e76057aa8cp-5;
+    const double* c = CHEM_GEN_TAB(nasa)[hi0][8];
+    t.cvk[8] = c[0] + T * (c[1] + T * (c[2] + T * (c[3] + T * c[4])));
+    t.u[8] = c[10] + T * (c[5] + T * (c[6] + T * (c[7] + T * (c[8] + T * c[9]))));
   }
-  t.kf[0] = 0x1.f438daa060000p+54 * exp((-0x1.6666666666666p-1) * alogt - 0x1.0c6f4493ef159p+13 * Tinv);
-  t.kr[0] = 0x1.001d1bf800000p+46 * exp((-0x1.0a3d70a3d70a4p-2) * alogt - 0x1.1fd705d6afec6p+6 * Tinv);
-  t.kf[1] = 0x1.8b50000000000p+15 * exp(0x1.55c28f5c28f5cp+1 * alogt - 0x1.8bb78dad5b973p+11 * Tinv);
-  t.kr[1] = 0x1.d970000000000p+14 * exp(0x1.50a3d70a3d70ap+1 * alogt - 0x1.3072327bb03a1p+11 * Tinv);
-  t.kf[2] = 0x1.16f3220000000p+30 * exp(0x1.4cccccccccccdp+0 * alogt - 0x1.c94c533be761cp+10 * Tinv);
-  t.kr[2] = 0x1.7d78400000000p+33 * exp(0x1.30a3d70a3d70ap+0 * alogt - 0x1.2611369490098p+13 * Tinv);
-  t.kf[3] = 0x1.0eaa664900000p+42 * exp(0x1.c28f5c28f5c29p-2 * alogt - 0.0 * Tinv);
-  t.klow[0] = 0x1.8efc84ad0c7b0p+65 * exp((-0x1.6666666666666p+0) * alogt - 0.0 * Tinv);
+#pragma unroll 2
+  for (int i = 0; i < 20; ++i) {
+    const double* p = CHEM_GEN_TAB(arr)[i];
+    t.k[i] = p[0] * fm_exp(p[1] * alogt - p[2] * Tinv);
+  }
+  t.k[18] = c_div(t.k[18], t.k[3]);
   {
     const double ta = 0x1.0000000000000p-1;
-    double fcent = (1.0 - ta) * exp(-T * 0x1.93e5939a08ce9p+99) + ta * exp(-T * 0x1.4484bfeebc29fp-100);
-    t.fclog[0] = log(fmax(fcent, 1.0e-300)) * 0.4342944819032518277;
+    double fcent = (1.0 - ta) * c_exp(-T * 0x1.93e5939a08ce9p+99) + ta * c_exp(-T * 0x1.4484bfeebc29fp-100);
+    const double lnfc = c_log(fmax(fcent, 1.0e-300));
+    t.lnfc[0] = lnfc;
+    t.trc[0] = kTroeC + 0.67 * lnfc;
+    t.trn[0] = kTroeN - 1.27 * lnfc;
   }
-  t.kf[4] = 0x1.0191a36680000p+46 * exp(0.0 * alogt - 0x1.27e432c1d6dbcp+7 * Tinv);
-  t.kf[5] = 0x1.e31fa34e00000p+43 * exp(0.0 * alogt - 0x1.9da4e3b0f0481p+8 * Tinv);
-  t.kr[3] = 0x1.39283f4a00000p+41 * exp(0x1.70a3d70a3d70ap-2 * alogt - 0x1.b3c1120ab0336p+14 * Tinv);
-  t.kf[6] = 0x1.a48ce3be80000p+44 * exp(0.0 * alogt - (-0x1.f4328690d2d50p+7) * Tinv);
-  t.kf[7] = 0x1.0f0cf064dd592p+75 * exp((-0x1.0000000000000p+1) * alogt - 0.0 * Tinv);
-  t.kr[4] = 0x1.5cfa424ea9c92p+76 * exp((-0x1.c000000000000p+0) * alogt - 0x1.d22edd4d65d8ep+15 * Tinv);
-  t.kf[8] = 0x1.20a871cc00200p+60 * exp((-0x1.0000000000000p+0) * alogt - 0.0 * Tinv);
-  t.kr[5] = 0x1.0e0198eaee000p+58 * exp((-0x1.4cccccccccccdp-1) * alogt - 0x1.96e5d98de8289p+15 * Tinv);
-  t.kf[9] = 0x1.5f93037c00000p+41 * exp(0.0 * alogt - 0x1.5dbc4f266b3c5p+9 * Tinv);
-  t.kf[10] = 0x1.2dbf9ea000000p+37 * exp(0x1.3851eb851eb85p-1 * alogt - 0x1.784fcc6a9ac05p+13 * Tinv);
-  t.kf[11] = 0x1.6b99192fbb3c0p+64 * exp((-0x1.63d70a3d70a3dp+0) * alogt - 0x1.93845131294f1p+14 * Tinv);
-  t.klow[1] = 0x1.592a7a2071df8p+79 * exp((-0x1.e666666666666p+0) * alogt - 0x1.8626719ec5abbp+14 * Tinv);
+  t.k[19] = c_div(t.k[19], t.k[11]);
   {
     const double ta = 0x1.7851eb851eb85p-1;
-    double fcent = (1.0 - ta) * exp(-T * 0x1.5c9882b931057p-7) + ta * exp(-T * 0x1.2a91c92f3c105p-11);
-    fcent = fcent + exp(-0x1.43e0000000000p+12 * Tinv);
-    t.fclog[1] = log(fmax(fcent, 1.0e-300)) * 0.4342944819032518277;
+    double fcent = (1.0 - ta) * c_exp(-T * 0x1.5c9882b931057p-7) + ta * c_exp(-T * 0x1.2a91c92f3c105p-11);
+    fcent = fcent + c_exp(-0x1.43e0000000000p+12 * Tinv);
+    const double lnfc = c_log(fmax(fcent, 1.0e-300));
+    t.lnfc[1] = lnfc;
+    t.trc[1] = kTroeC + 0.67 * lnfc;
+    t.trn[1] = kTroeN - 1.27 * lnfc;
   }
 }
 
-HD __forceinline__ void cpart(double rho, const double* z, const FunT& t, double* zp) {
+HD __forceinline__ void cpart(const Cell<9>& cell, const double* z, const FunT& t, double* zp) {
   const double* Y = z + 1;
   double cv = 0.0, ctot = 0.0;
   cv = cv + Y[0] * t.cvk[0];
-  const double C0 = rho * Y[0] * 0x1.fbf39e8ab06bdp-1;
+  const double C0 = Y[0] * cell.rw[0];
   ctot = ctot + C0;
   cv = cv + Y[1] * t.cvk[1];
-  const double C1 = rho * Y[1] * 0x1.fbf39e8ab06bdp-2;
+  const double C1 = Y[1] * cell.rw[1];
   ctot = ctot + C1;
   cv = cv + Y[2] * t.cvk[2];
-  const double C2 = rho * Y[2] * 0x1.000275060987dp-4;
+  const double C2 = Y[2] * cell.rw[2];
   ctot = ctot + C2;
   cv = cv + Y[3] * t.cvk[3];
-  const double C3 = rho * Y[3] * 0x1.000275060987dp-5;
+  const double C3 = Y[3] * cell.rw[3];
   ctot = ctot + C3;
   cv = cv + Y[4] * t.cvk[4];
-  const double C4 = rho * Y[4] * 0x1.e1ac6c774b6a9p-5;
+  const double C4 = Y[4] * cell.rw[4];
   ctot = ctot + C4;
   cv = cv + Y[5] * t.cvk[5];
-  const double C5 = rho * Y[5] * 0x1.c6b93cc1512cbp-5;
+  const double C5 = Y[5] * cell.rw[5];
   ctot = ctot + C5;
   cv = cv + Y[6] * t.cvk[6];
-  const double C6 = rho * Y[6] * 0x1.f0620d016f133p-6;
+  const double C6 = Y[6] * cell.rw[6];
   ctot = ctot + C6;
   cv = cv + Y[7] * t.cvk[7];
-  const double C7 = rho * Y[7] * 0x1.e1ac6c774b6a9p-6;
+  const double C7 = Y[7] * cell.rw[7];
   ctot = ctot + C7;
   cv = cv + Y[8] * t.cvk[8];
-  const double C8 = rho * Y[8] * 0x1.246e76057aa8cp-5;
+  const double C8 = Y[8] * cell.rw[8];
   ctot = ctot + C8;
   double rop0;
   {   // reaction 0
-    double rkft = t.kf[0];
-    double rkrt = t.kr[0];
+    double rkft = t.k[0];
+    double rkrt = t.k[12];
     double rkf = rkft * C0;
     double rkr = rkrt * C2;
     rkf = rkf * C3;
@@ -218,8 +202,8 @@ HD __forceinline__ void cpart(double rho, const double* z, const FunT& t, double
   }
   double rop1;
   {   // reaction 1
-    double rkft = t.kf[1];
-    double rkrt = t.kr[1];
+    double rkft = t.k[1];
+    double rkrt = t.k[13];
     double rkf = rkft * C1;
     double rkr = rkrt * C0;
     rkf = rkf * C2;
@@ -228,8 +212,8 @@ HD __forceinline__ void cpart(double rho, const double* z, const FunT& t, double
   }
   double rop2;
   {   // reaction 2
-    double rkft = t.kf[2];
-    double rkrt = t.kr[2];
+    double rkft = t.k[2];
+    double rkrt = t.k[14];
     double rkf = rkft * C1;
     double rkr = rkrt * C0;
     rkf = rkf * C4;
@@ -238,21 +222,13 @@ HD __forceinline__ void cpart(double rho, const double* z, const FunT& t, double
   }
   double rop3;
   {   // reaction 3
-    double rkft = t.kf[3];
+    double rkft = t.k[3];
     double ctb = ctot;
     ctb = ctb + 0x1.8000000000000p+0 * C1;
     ctb = ctb + 0x1.e000000000000p+3 * C5;
-    const double pr = t.klow[0] * ctb / rkft;
-    double pcor = pr / (1.0 + pr);
-    {
-      const double prlog = log(fmax(pr, 1.0e-300)) * 0.4342944819032518277;
-      const double fclog = t.fclog[0];
-      const double xn = 0.75 - 1.27 * fclog;
-      const double cprlog = prlog - (0.4 + 0.67 * fclog);
-      const double q = cprlog / (xn - 0.14 * cprlog);
-      const double flog = fclog / (1.0 + q * q);
-      pcor = exp(flog * 2.302585092994045684) * pcor;
-    }
+    const double pr = t.k[18] * ctb;
+    double pcor = c_div(pr, 1.0 + pr);
+    pcor = troe_factor(pr, t.lnfc[0], t.trc[0], t.trn[0]) * pcor;
     rkft = rkft * pcor;
     double rkf = rkft * C0;
     rkf = rkf * C3;
@@ -260,15 +236,15 @@ HD __forceinline__ void cpart(double rho, const double* z, const FunT& t, double
   }
   double rop4;
   {   // reaction 4
-    double rkft = t.kf[4];
+    double rkft = t.k[4];
     double rkf = rkft * C0;
     rkf = rkf * C6;
     rop4 = rkf;
   }
   double rop5;
   {   // reaction 5
-    double rkft = t.kf[5];
-    double rkrt = t.kr[3];
+    double rkft = t.k[5];
+    double rkrt = t.k[15];
     double rkf = rkft * C0;
     double rkr = rkrt * C1;
     rkf = rkf * C6;
@@ -277,15 +253,15 @@ HD __forceinline__ void cpart(double rho, const double* z, const FunT& t, double
   }
   double rop6;
   {   // reaction 6
-    double rkft = t.kf[6];
+    double rkft = t.k[6];
     double rkf = rkft * C4;
     rkf = rkf * C6;
     rop6 = rkf;
   }
   double rop7;
   {   // reaction 7
-    double rkft = t.kf[7];
-    double rkrt = t.kr[4];
+    double rkft = t.k[7];
+    double rkrt = t.k[16];
     double ctb = ctot;
     ctb = ctb + 0x1.8000000000000p+0 * C1;
     ctb = ctb + 0x1.6000000000000p+3 * C5;
@@ -298,8 +274,8 @@ HD __forceinline__ void cpart(double rho, const double* z, const FunT& t, double
   }
   double rop8;
   {   // reaction 8
-    double rkft = t.kf[8];
-    double rkrt = t.kr[5];
+    double rkft = t.k[8];
+    double rkrt = t.k[17];
     double ctb = ctot;
     ctb = ctb + 0x1.8000000000000p+0 * C1;
     ctb = ctb + 0x1.6000000000000p+3 * C5;
@@ -311,68 +287,65 @@ HD __forceinline__ void cpart(double rho, const double* z, const FunT& t, double
   }
   double rop9;
   {   // reaction 9
-    double rkft = t.kf[9];
+    double rkft = t.k[9];
     double rkf = rkft * (C6 * C6);
     rop9 = rkf;
   }
   double rop10;
   {   // reaction 10
-    double rkft = t.kf[10];
+    double rkft = t.k[10];
     double rkf = rkft * C1;
     rkf = rkf * C6;
     rop10 = rkf;
   }
   double rop11;
   {   // reaction 11
-    double rkft = t.kf[11];
+    double rkft = t.k[11];
     double ctb = ctot;
     ctb = ctb + 0x1.8000000000000p+0 * C1;
     ctb = ctb + 0x1.4000000000000p+2 * C5;
-    const double pr = t.klow[1] * ctb / rkft;
-    double pcor = pr / (1.0 + pr);
-    {
-      const double prlog = log(fmax(pr, 1.0e-300)) * 0.4342944819032518277;
-      const double fclog = t.fclog[1];
-      const double xn = 0.75 - 1.27 * fclog;
-      const double cprlog = prlog - (0.4 + 0.67 * fclog);
-      const double q = cprlog / (xn - 0.14 * cprlog);
-      const double flog = fclog / (1.0 + q * q);
-      pcor = exp(flog * 2.302585092994045684) * pcor;
-    }
+    const double pr = t.k[19] * ctb;
+    double pcor = c_div(pr, 1.0 + pr);
+    pcor = troe_factor(pr, t.lnfc[1], t.trc[1], t.trn[1]) * pcor;
     rkft = rkft * pcor;
     double rkf = rkft * C7;
     rop11 = rkf;
   }
-  const double wdot0 = (((((((((0.0 + rop0 * (-0x1.0000000000000p+0)) + rop3 * (-0x1.0000000000000p+0)) + rop4 * (-0x1.0000000000000p+0)) + rop5 * (-0x1.0000000000000p+0)) + rop7 * (-0x1.0000000000000p+0)) + rop8 * (-0x1.0000000000000p+1)) + rop1 * 0x1.0000000000000p+0) + rop2 * 0x1.0000000000000p+0) + rop10 * 0x1.0000000000000p+0);
-  const double wdot1 = (((((0.0 + rop1 * (-0x1.0000000000000p+0)) + rop2 * (-0x1.0000000000000p+0)) + rop10 * (-0x1.0000000000000p+0)) + rop5 * 0x1.0000000000000p+0) + rop8 * 0x1.0000000000000p+0);
-  const double wdot2 = ((0.0 + rop1 * (-0x1.0000000000000p+0)) + rop0 * 0x1.0000000000000p+0);
-  const double wdot3 = (((((0.0 + rop0 * (-0x1.0000000000000p+0)) + rop3 * (-0x1.0000000000000p+0)) + rop6 * 0x1.0000000000000p+0) + rop9 * 0x1.0000000000000p+0) + rop5 * 0x1.0000000000000p+0);
-  const double wdot4 = (((((((0.0 + rop6 * (-0x1.0000000000000p+0)) + rop2 * (-0x1.0000000000000p+0)) + rop7 * (-0x1.0000000000000p+0)) + rop4 * 0x1.0000000000000p+1) + rop11 * 0x1.0000000000000p+1) + rop0 * 0x1.0000000000000p+0) + rop1 * 0x1.0000000000000p+0);
-  const double wdot5 = (((0.0 + rop7 * 0x1.0000000000000p+0) + rop2 * 0x1.0000000000000p+0) + rop6 * 0x1.0000000000000p+0);
-  const double wdot6 = ((((((0.0 + rop9 * (-0x1.0000000000000p+1)) + rop4 * (-0x1.0000000000000p+0)) + rop5 * (-0x1.0000000000000p+0)) + rop6 * (-0x1.0000000000000p+0)) + rop10 * (-0x1.0000000000000p+0)) + rop3 * 0x1.0000000000000p+0);
-  const double wdot7 = (((0.0 + rop11 * (-0x1.0000000000000p+0)) + rop9 * 0x1.0000000000000p+0) + rop10 * 0x1.0000000000000p+0);
+  const double wdot0 = - rop0 - rop3 - rop4 - rop5 - rop7 - rop8 * 0x1.0000000000000p+1 + rop1 + rop2 + rop10;
+  const double wdot1 = - rop1 - rop2 - rop10 + rop5 + rop8;
+  const double wdot2 = - rop1 + rop0;
+  const double wdot3 = - rop0 - rop3 + rop6 + rop9 + rop5;
+  const double wdot4 = - rop6 - rop2 - rop7 + rop4 * 0x1.0000000000000p+1 + rop11 * 0x1.0000000000000p+1 + rop0 + rop1;
+  const double wdot5 = + rop7 + rop2 + rop6;
+  const double wdot6 = - rop9 * 0x1.0000000000000p+1 - rop4 - rop5 - rop6 - rop10 + rop3;
+  const double wdot7 = - rop11 + rop9 + rop10;
   const double wdot8 = 0.0;
-  const double rho_i = 1.0 / rho;
   double sum = 0.0;
-  zp[1] = wdot0 * 0x1.020a520000000p+0 * rho_i;
-  sum = sum + t.h[0] * wdot0 * 0x1.020a520000000p+0 + (-t.rut) * wdot0;
-  zp[2] = wdot1 * 0x1.020a520000000p+1 * rho_i;
-  sum = sum + t.h[1] * wdot1 * 0x1.020a520000000p+1 + (-t.rut) * wdot1;
-  zp[3] = wdot2 * 0x1.fffb160000000p+3 * rho_i;
-  sum = sum + t.h[2] * wdot2 * 0x1.fffb160000000p+3 + (-t.rut) * wdot2;
-  zp[4] = wdot3 * 0x1.fffb160000000p+4 * rho_i;
-  sum = sum + t.h[3] * wdot3 * 0x1.fffb160000000p+4 + (-t.rut) * wdot3;
-  zp[5] = wdot4 * 0x1.101e302000000p+4 * rho_i;
-  sum = sum + t.h[4] * wdot4 * 0x1.101e302000000p+4 + (-t.rut) * wdot4;
-  zp[6] = wdot5 * 0x1.203ed54000000p+4 * rho_i;
-  sum = sum + t.h[5] * wdot5 * 0x1.203ed54000000p+4 + (-t.rut) * wdot5;
-  zp[7] = wdot6 * 0x1.080ddd9000000p+5 * rho_i;
-  sum = sum + t.h[6] * wdot6 * 0x1.080ddd9000000p+5 + (-t.rut) * wdot6;
-  zp[8] = wdot7 * 0x1.101e302000000p+5 * rho_i;
-  sum = sum + t.h[7] * wdot7 * 0x1.101e302000000p+5 + (-t.rut) * wdot7;
-  zp[9] = wdot8 * 0x1.c036e20000000p+4 * rho_i;
-  sum = sum + t.h[8] * wdot8 * 0x1.c036e20000000p+4 + (-t.rut) * wdot8;
-  zp[0] = -sum / (rho * cv);
+  zp[1] = wdot0 * 0x1.020a520000000p+0 * cell.rho_i;
+  sum = sum + t.u[0] * wdot0;
+  zp[2] = wdot1 * 0x1.020a520000000p+1 * cell.rho_i;
+  sum = sum + t.u[1] * wdot1;
+  zp[3] = wdot2 * 0x1.fffb160000000p+3 * cell.rho_i;
+  sum = sum + t.u[2] * wdot2;
+  zp[4] = wdot3 * 0x1.fffb160000000p+4 * cell.rho_i;
+  sum = sum + t.u[3] * wdot3;
+  zp[5] = wdot4 * 0x1.101e302000000p+4 * cell.rho_i;
+  sum = sum + t.u[4] * wdot4;
+  zp[6] = wdot5 * 0x1.203ed54000000p+4 * cell.rho_i;
+  sum = sum + t.u[5] * wdot5;
+  zp[7] = wdot6 * 0x1.080ddd9000000p+5 * cell.rho_i;
+  sum = sum + t.u[6] * wdot6;
+  zp[8] = wdot7 * 0x1.101e302000000p+5 * cell.rho_i;
+  sum = sum + t.u[7] * wdot7;
+  zp[9] = 0.0;
+  zp[0] = -c_div(sum, cell.rho * cv);
+}
+
+// the same from the density alone
+HD __forceinline__ void cpart(double rho, const double* z, const FunT& t, double* zp) {
+  Cell<9> cell;
+  cell_set(rho, cell);
+  cpart(cell, z, t, zp);
 }
 
 // True when m is the mechanism this file was generated from (every table

@@ -78,7 +78,7 @@ __device__ __forceinline__ double th_cp_fast(int r, int is, double T) {
 }
 
 // th_species out of line, for the points outside the common range
-__device__ __noinline__ double2 th_species_call(int is, double T) {
+static __device__ __noinline__ double2 th_species_call(int is, double T) {
   double cpk;
   const double h = th_species(is, T, &cpk);
   return make_double2(h, cpk);

@@ -82,11 +82,29 @@ def generate(m, name="h2air9", source="phd_gb300/data/h2_sandiego12.inp"):
     eqk = any(r["rev"] == 1 for r in R)
     fall = [r["i"] for r in R if r["fall"]]
     troe = [r["i"] for r in R if r["fall"] > 1]
-    kr_slot = {i: q for q, i in enumerate(rev)}
-    lo_slot = {i: q for q, i in enumerate(fall)}
     tr_slot = {i: q for q, i in enumerate(troe)}
     wt_inv = [1.0 / m.wt[k] for k in range(kk)]
     ru_wt = [m.ru / m.wt[k] for k in range(kk)]
+
+    # the Arrhenius expressions A exp(b ln T - E/R / T) in one table: forward,
+    # explicit reverse and low-pressure rate constants
+    arr = [r["par"] for r in R]
+    kr_at, lo_at = {}, {}
+    for r in R:
+        if r["rev"] == 2:
+            kr_at[r["i"]] = len(arr)
+            arr.append(r["rpar"])
+    for r in R:
+        if r["rev"] == 1:   # from the equilibrium constant: a slot without an expression
+            kr_at[r["i"]] = None
+    for r in R:
+        if r["fall"]:
+            lo_at[r["i"]] = len(arr)
+            arr.append(r["low"])
+    n_exp = len(arr)
+    for i in [i for i in kr_at if kr_at[i] is None]:
+        kr_at[i] = len(arr)
+        arr.append(None)
     L = []
     w = L.append
     w("// Generated by phd_gb300/mechgen.py from %s -- do not edit." % source)
@@ -103,71 +121,103 @@ def generate(m, name="h2air9", source="phd_gb300/data/h2_sandiego12.inp"):
     w("// species columns reuse them (rc_drive)")
     w("struct FunT {")
     w("  double T;")
-    w("  double rut;")
-    w("  double cvk[%d], h[%d];" % (kk, kk))
-    w("  double kf[%d];" % m.ii)
+    w("  double cvk[%d], u[%d];" % (kk, kk))
+    w("  double k[%d];   // forward rate constants, then" % len(arr))
     if rev:
-        w("  double kr[%d];   // reactions %s" % (len(rev), ", ".join(map(str, rev))))
+        w("                 // reverse: " + ", ".join("k[%d] of reaction %d" % (kr_at[i], i) for i in rev))
     if fall:
-        w("  double klow[%d];   // reactions %s" % (len(fall), ", ".join(map(str, fall))))
+        w("                 // low- over high-pressure: " +
+          ", ".join("k[%d] of reaction %d" % (lo_at[i], i) for i in fall))
     if troe:
-        w("  double fclog[%d];   // reactions %s" % (len(troe), ", ".join(map(str, troe))))
+        w("  double lnfc[%d], trc[%d], trn[%d];   // reactions %s" % ((len(troe),) * 3 + (", ".join(map(str, troe)),)))
     w("};")
+    w("")
+    w("HD __forceinline__ void cell_set(double rho, Cell<%d>& c) {" % kk)
+    w("  c.rho = rho;")
+    w("  c.rho_i = c_rcp(rho);")
+    for k in range(kk):
+        w("  c.rw[%d] = rho * %s;" % (k, lit(wt_inv[k])))
+    w("}")
+    w("")
+    # ---------------------------------------------------------------- tables
+    w("// A, b, E/R of the Arrhenius expressions; c_v (5) and internal energy (6)")
+    w("// polynomials of the species below and above their middle temperature: in")
+    w("// constant memory, so that the loops over them stay small code")
+    rows = ["{%s}" % ", ".join(lit(x) for x in p) for p in arr[:n_exp]]
+    nasa = []
+    for q in range(2):
+        sp = []
+        for k in range(kk):
+            a = list(m.a[k][q])
+            c = [ru_wt[k] * (a[0] - 1.0)] + [ru_wt[k] * a[j] for j in range(1, 5)]
+            e = [m.ru * (a[0] - 1.0)] + [m.ru * a[j] / float(j + 1) for j in range(1, 5)] + [m.ru * a[5]]
+            sp.append("{%s}" % ", ".join(lit(x) for x in c + e))
+        nasa.append("{%s}" % ",\\\n   ".join(sp))
+    w("#define CHEM_GEN_ARR %s" % ", \\\n  ".join(rows))
+    w("#define CHEM_GEN_NASA %s" % ", \\\n  ".join(nasa))
+    w("__constant__ double arr_dev[%d][3] = {CHEM_GEN_ARR};" % n_exp)
+    w("__constant__ double nasa_dev[2][%d][11] = {CHEM_GEN_NASA};" % kk)
+    w("#ifdef __CUDA_ARCH__")
+    w("#define CHEM_GEN_TAB(x) x##_dev")
+    w("#else")
+    w("static const double arr_host[%d][3] = {CHEM_GEN_ARR};" % n_exp)
+    w("static const double nasa_host[2][%d][11] = {CHEM_GEN_NASA};" % kk)
+    w("#define CHEM_GEN_TAB(x) x##_host")
+    w("#endif")
     w("")
     # ---------------------------------------------------------------- tpart
     w("HD __forceinline__ void tpart(double T, FunT& t) {")
-    w("  const double Tinv = 1.0 / T;")
-    w("  const double alogt = log(T);")
-    w("  const double T2 = T * T, T3 = T * T2, T4 = T2 * T2;")
+    w("  const double Tinv = c_rcp(T);")
+    w("  const double alogt = c_log(T);")
     w("  t.T = T;")
-    w("  t.rut = T * %s;" % lit(m.ru))
     if eqk:
+        w("  const double T2 = T * T, T3 = T * T2, T4 = T2 * T2;")
         w("  double %s;   // S/R - H/RT (CKSMH)" % ", ".join("smh%d" % k for k in range(kk)))
+    tm = sorted(set(m.tmid[k] for k in range(kk)))
+    for q, x in enumerate(tm):
+        w("  const int hi%d = T > %s ? 1 : 0;" % (q, lit(x)))
     for k in range(kk):
         lo, hi = list(m.a[k][0]), list(m.a[k][1])
         w("  {   // species %d" % k)
-        w("    const bool hi = T > %s;" % lit(m.tmid[k]))
-        for j in range(7 if eqk else 6):
-            w("    const double a%d = hi ? %s : %s;" % (j, lit(hi[j]), lit(lo[j])))
-        w("    const double cps = a0 + T * a1 + T2 * a2 + T3 * a3 + T4 * a4;")
-        w("    t.cvk[%d] = %s * (cps - 1.0);" % (k, lit(ru_wt[k])))
-        w("    const double hs = a0 + (0.5 * T) * a1 + (T2 * (1.0 / 3.0)) * a2 + (0.25 * T3) * a3 + (0.2 * T4) * a4;")
-        w("    t.h[%d] = t.rut * (hs + a5 * Tinv) * %s;" % (k, lit(wt_inv[k])))
+        w("    const double* c = CHEM_GEN_TAB(nasa)[hi%d][%d];" % (tm.index(m.tmid[k]), k))
+        w("    t.cvk[%d] = c[0] + T * (c[1] + T * (c[2] + T * (c[3] + T * c[4])));" % k)
+        w("    t.u[%d] = c[10] + T * (c[5] + T * (c[6] + T * (c[7] + T * (c[8] + T * c[9]))));" % k)
         if eqk:
+            for j in range(7):
+                w("    const double a%d = hi%d ? %s : %s;" % (j, tm.index(m.tmid[k]), lit(hi[j]), lit(lo[j])))
             w("    const double sv = (alogt - 1.0) * a0 + (0.5 * T) * a1 + (T2 * (1.0 / 6.0)) * a2 +")
             w("                      (T3 * (1.0 / 12.0)) * a3 + (T4 * 0.05) * a4;")
             w("    smh%d = sv + a6 - a5 * Tinv;" % k)
         w("  }")
+    w("#pragma unroll 2")
+    w("  for (int i = 0; i < %d; ++i) {" % n_exp)
+    w("    const double* p = CHEM_GEN_TAB(arr)[i];")
+    w("    t.k[i] = p[0] * fm_exp(p[1] * alogt - p[2] * Tinv);")
+    w("  }")
     for r in R:
         i = r["i"]
-        p = r["par"]
-        w("  t.kf[%d] = %s * exp(%s * alogt - %s * Tinv);" % (i, lit(p[0]), lit(p[1]), lit(p[2])))
         if any(r["lt"]):   # Landau-Teller: the expression of fun_tpart
-            w("  t.kf[%d] = t.kf[%d] * exp(%s / pow(T, %s) + %s / pow(T, %s));"
+            w("  t.k[%d] = t.k[%d] * c_exp(%s / pow(T, %s) + %s / pow(T, %s));"
               % (i, i, lit(r["lt"][0]), lit(LT_P1), lit(r["lt"][1]), lit(LT_P2)))
-        if r["rev"] == 2:
-            q = r["rpar"]
-            w("  t.kr[%d] = %s * exp(%s * alogt - %s * Tinv);" % (kr_slot[i], lit(q[0]), lit(q[1]), lit(q[2])))
-        elif r["rev"] == 1:   # k_f / K_c, K_c from the species' S/R - H/RT
+        if r["rev"] == 1:   # k_f / K_c, K_c from the species' S/R - H/RT
             w("  {")
             w("    double sumsmh = 0.0;")
             for n in range(6):
                 if r["nuk"][n] >= 0:
                     w("    sumsmh = sumsmh + %s * smh%d;" % (lit(float(r["nu"][n])), r["nuk"][n]))
-            w("    double eqk = sumsmh != 0.0 ? exp(fmin(sumsmh, 690.77552789821368)) : 1.0;")
+            w("    double eqk = sumsmh != 0.0 ? c_exp(fmin(sumsmh, 690.77552789821368)) : 1.0;")
             w("    eqk = eqk * powi(%s * Tinv / %s, %d);" % (lit(m.patm), lit(m.ru), sum(r["nu"])))
-            w("    t.kr[%d] = t.kf[%d] / fmax(eqk, 1.0e-300);" % (kr_slot[i], i))
+            w("    t.k[%d] = c_div(t.k[%d], fmax(eqk, 1.0e-300));" % (kr_at[i], i))
             w("  }")
         if any(r["rlt"]):
-            w("  t.kr[%d] = t.kr[%d] * exp(%s / pow(T, %s) + %s / pow(T, %s));"
-              % (kr_slot[i], kr_slot[i], lit(r["rlt"][0]), lit(LT_P1), lit(r["rlt"][1]), lit(LT_P2)))
+            w("  t.k[%d] = t.k[%d] * c_exp(%s / pow(T, %s) + %s / pow(T, %s));"
+              % (kr_at[i], kr_at[i], lit(r["rlt"][0]), lit(LT_P1), lit(r["rlt"][1]), lit(LT_P2)))
         if r["fall"]:
-            q = r["low"]
-            w("  t.klow[%d] = %s * exp(%s * alogt - %s * Tinv);" % (lo_slot[i], lit(q[0]), lit(q[1]), lit(q[2])))
-            if r["fall"] == 2:   # SRI: ln(a exp(-b/T) + exp(-T/c)) in the fclog slot
+            w("  t.k[%d] = c_div(t.k[%d], t.k[%d]);" % (lo_at[i], lo_at[i], i))
+            if r["fall"] == 2:   # SRI: ln(a exp(-b/T) + exp(-T/c)) in the lnfc slot
                 sr = r["sri"]
                 cinv = 1.0 / sr[2] if sr[2] != 0.0 else 0.0
-                w("  t.fclog[%d] = log(%s * exp(-%s * Tinv) + exp(-T * %s));" % (tr_slot[i], lit(sr[0]), lit(sr[1]),
+                w("  t.lnfc[%d] = c_log(%s * c_exp(-%s * Tinv) + c_exp(-T * %s));" % (tr_slot[i], lit(sr[0]), lit(sr[1]),
                                                                                   lit(cinv)))
             elif r["fall"] > 1:
                 ta = r["troe"][0]
@@ -175,30 +225,33 @@ def generate(m, name="h2air9", source="phd_gb300/data/h2_sandiego12.inp"):
                 ti1 = 1.0 / r["troe"][2] if r["troe"][2] != 0.0 else 0.0
                 w("  {")
                 w("    const double ta = %s;" % lit(ta))
-                w("    double fcent = (1.0 - ta) * exp(-T * %s) + ta * exp(-T * %s);" % (lit(ti0), lit(ti1)))
+                w("    double fcent = (1.0 - ta) * c_exp(-T * %s) + ta * c_exp(-T * %s);" % (lit(ti0), lit(ti1)))
                 if r["fall"] == 4:
-                    w("    fcent = fcent + exp(-%s * Tinv);" % lit(r["troe"][3]))
-                w("    t.fclog[%d] = log(fmax(fcent, 1.0e-300)) * 0.4342944819032518277;" % tr_slot[i])
+                    w("    fcent = fcent + c_exp(-%s * Tinv);" % lit(r["troe"][3]))
+                w("    const double lnfc = c_log(fmax(fcent, 1.0e-300));")
+                w("    t.lnfc[%d] = lnfc;" % tr_slot[i])
+                w("    t.trc[%d] = kTroeC + 0.67 * lnfc;" % tr_slot[i])
+                w("    t.trn[%d] = kTroeN - 1.27 * lnfc;" % tr_slot[i])
                 w("  }")
     w("}")
     w("")
     # ---------------------------------------------------------------- cpart
-    w("HD __forceinline__ void cpart(double rho, const double* z, const FunT& t, double* zp) {")
+    w("HD __forceinline__ void cpart(const Cell<%d>& cell, const double* z, const FunT& t, double* zp) {" % kk)
     w("  const double* Y = z + 1;")
     w("  double cv = 0.0, ctot = 0.0;")
     for k in range(kk):
         w("  cv = cv + Y[%d] * t.cvk[%d];" % (k, k))
-        w("  const double C%d = rho * Y[%d] * %s;" % (k, k, lit(wt_inv[k])))
+        w("  const double C%d = Y[%d] * cell.rw[%d];" % (k, k, k))
         w("  ctot = ctot + C%d;" % k)
     for r in R:
         i = r["i"]
         nuk, nu = r["nuk"], r["nu"]
         w("  double rop%d;" % i)
         w("  {   // reaction %d" % i)
-        w("    double rkft = t.kf[%d];" % i)
+        w("    double rkft = t.k[%d];" % i)
         isrev = r["rev"] != 0
         if isrev:
-            w("    double rkrt = t.kr[%d];" % kr_slot[i])
+            w("    double rkrt = t.k[%d];" % kr_at[i])
         ctb = None
         if r["thb"]:
             w("    double ctb = ctot;")
@@ -207,30 +260,21 @@ def generate(m, name="h2air9", source="phd_gb300/data/h2_sandiego12.inp"):
                     w("    ctb = ctb + %s * C%d;" % (lit(r["eff"][k] - 1.0), k))
             ctb = "ctb"
         if r["fall"]:
-            f = lo_slot[i]
             if r["kfal"]:   # one species is the collider; a third-body factor stays
-                w("    const double pr = t.klow[%d] * C%d / rkft;" % (f, r["kfal"] - 1))
+                w("    const double pr = t.k[%d] * C%d;" % (lo_at[i], r["kfal"] - 1))
             else:
-                w("    const double pr = t.klow[%d] * %s / rkft;" % (f, ctb if ctb else "1.0"))
+                w("    const double pr = t.k[%d] * %s;" % (lo_at[i], ctb if ctb else "1.0"))
                 ctb = None
-            w("    double pcor = pr / (1.0 + pr);")
+            w("    double pcor = c_div(pr, 1.0 + pr);")
             if r["fall"] == 2:
                 w("    {")
-                w("      const double prlog = log(fmax(pr, 1.0e-300)) * 0.4342944819032518277;")
-                w("      const double xp = 1.0 / (1.0 + prlog * prlog);")
-                w("      pcor = exp(xp * t.fclog[%d]) * %s * pow(t.T, %s) * pcor;" % (tr_slot[i], lit(r["sri"][3]),
+                w("      const double prlog = c_log(fmax(pr, 1.0e-300)) * kInvLn10;")
+                w("      const double xp = c_rcp(1.0 + prlog * prlog);")
+                w("      pcor = c_exp(xp * t.lnfc[%d]) * %s * pow(t.T, %s) * pcor;" % (tr_slot[i], lit(r["sri"][3]),
                                                                                    lit(r["sri"][4])))
                 w("    }")
             elif r["fall"] > 1:
-                w("    {")
-                w("      const double prlog = log(fmax(pr, 1.0e-300)) * 0.4342944819032518277;")
-                w("      const double fclog = t.fclog[%d];" % tr_slot[i])
-                w("      const double xn = 0.75 - 1.27 * fclog;")
-                w("      const double cprlog = prlog - (0.4 + 0.67 * fclog);")
-                w("      const double q = cprlog / (xn - 0.14 * cprlog);")
-                w("      const double flog = fclog / (1.0 + q * q);")
-                w("      pcor = exp(flog * 2.302585092994045684) * pcor;")
-                w("    }")
+                w("    pcor = troe_factor(pr, t.lnfc[%d], t.trc[%d], t.trn[%d]) * pcor;" % ((tr_slot[i],) * 3))
             w("    rkft = rkft * pcor;")
             if isrev:
                 w("    rkrt = rkrt * pcor;")
@@ -257,18 +301,27 @@ def generate(m, name="h2air9", source="phd_gb300/data/h2_sandiego12.inp"):
         for r in R:
             k = r["nuk"][n]
             if k >= 0:
-                acc[k].append("rop%d * %s" % (r["i"], lit(float(r["nu"][n]))))
+                v = r["nu"][n]
+                acc[k].append("%s rop%d%s" % ("+" if v > 0 else "-", r["i"],
+                                              "" if abs(v) == 1 else " * %s" % lit(float(abs(v)))))
     for k in range(kk):
-        expr = "0.0"
-        for t in acc[k]:
-            expr = "(%s + %s)" % (expr, t)
+        expr = " ".join(acc[k]) if acc[k] else "0.0"
         w("  const double wdot%d = %s;" % (k, expr))
-    w("  const double rho_i = 1.0 / rho;")
     w("  double sum = 0.0;")
     for k in range(kk):
-        w("  zp[%d] = wdot%d * %s * rho_i;" % (k + 1, k, lit(m.wt[k])))
-        w("  sum = sum + t.h[%d] * wdot%d * %s + (-t.rut) * wdot%d;" % (k, k, lit(m.wt[k]), k))
-    w("  zp[0] = -sum / (rho * cv);")
+        if not acc[k]:   # an inert species
+            w("  zp[%d] = 0.0;" % (k + 1))
+            continue
+        w("  zp[%d] = wdot%d * %s * cell.rho_i;" % (k + 1, k, lit(m.wt[k])))
+        w("  sum = sum + t.u[%d] * wdot%d;" % (k, k))
+    w("  zp[0] = -c_div(sum, cell.rho * cv);")
+    w("}")
+    w("")
+    w("// the same from the density alone")
+    w("HD __forceinline__ void cpart(double rho, const double* z, const FunT& t, double* zp) {")
+    w("  Cell<%d> cell;" % kk)
+    w("  cell_set(rho, cell);")
+    w("  cpart(cell, z, t, zp);")
     w("}")
     w("")
     # ------------------------------------------------------- host check
