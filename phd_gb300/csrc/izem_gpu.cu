@@ -314,9 +314,15 @@ int enq_visc(izem_ctx* c) {
   const bool eg = c->cfg.eglib != 0;
   const int nderiv = (eg ? 15 : 12) + 3 * NRV;
   int rc;
-  if ((rc = launch(c, "visc_grad", [&] { k_grad<NRV><<<grid_for(g.nint), kThreads, 0, c->stream>>>(g, mt, c->prim, c->T, c->Xa, c->fd); })))
+  if ((rc = launch(c, "visc_grad", [&] {
+         auto kern = g.ng == 4 ? k_grad<NRV, 4> : k_grad<NRV, 3>;
+         kern<<<grid_for(g.nint), kThreads, 0, c->stream>>>(g, mt, c->prim, c->T, c->Xa, c->fd);
+       })))
     return rc;
-  if (eg && (rc = launch(c, "visc_grad_p", [&] { k_grad_p<NRV><<<grid_for(g.nint), kThreads, 0, c->stream>>>(g, mt, c->prim, c->fd); })))
+  if (eg && (rc = launch(c, "visc_grad_p", [&] {
+               auto kern = g.ng == 4 ? k_grad_p<NRV, 4> : k_grad_p<NRV, 3>;
+               kern<<<grid_for(g.nint), kThreads, 0, c->stream>>>(g, mt, c->prim, c->fd);
+             })))
     return rc;
   const bool les = c->les_on;
   if (les && (rc = launch(c, "les_prep", [&] {
@@ -366,7 +372,10 @@ int enq_visc(izem_ctx* c) {
          k_visc_point<NRV><<<grid_for(slab_count(g), c->tb_visc), c->tb_visc, 0, c->stream>>>(g, c->v, c->T, c->W_i, c->ha, c->Xa, c->fd, c->tau, c->qv);
        })))
     return rc;
-  return launch(c, "visc_div", [&] { k_visc_div<NRV><<<grid_for(g.nint), kThreads, 0, c->stream>>>(g, mt, c->tau, c->qv, c->fd, c->f); });
+  return launch(c, "visc_div", [&] {
+    auto kern = g.ng == 4 ? k_visc_div<NRV, 4> : k_visc_div<NRV, 3>;
+    kern<<<grid_for(g.nint), kThreads, 0, c->stream>>>(g, mt, c->tau, c->qv, c->fd, c->f);
+  });
 }
 
 // NR_boundaries (module_BCs.f90:185-212): bc_noreflectionweno on every

@@ -411,7 +411,7 @@ __device__ __forceinline__ void eg_species_cp(double T, double* cpk) {
 
 // Pressure gradients of the EGLIB flux (fd slots 12 + 3 NRV + d) from the
 // primitive pressure P = rho T W_i.
-template <int NRV>
+template <int NRV, int NG>
 __global__ void k_grad_p(Geo g, Metrics mt, const double* __restrict__ prim, double* __restrict__ fd) {
   long long idx = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   if (idx >= g.nint) return;
@@ -425,9 +425,9 @@ __global__ void k_grad_p(Geo g, Metrics mt, const double* __restrict__ prim, dou
   const long long strides[3] = {1LL, (long long)g.g[0], (long long)g.g[0] * g.g[1]};
 #pragma unroll
   for (int d = 0; d < 3; ++d) {
-    const double di = mt.dxi[d][c[d] - 1 + g.ng];
     fd[(12 + 3 * NRV + d) * nc + p] =
-        deriv_at(prim + PR_P * nc, p, strides[d], c[d], g.n[d], g.bnd[2 * d], g.bnd[2 * d + 1], di, g.ng);
+        deriv_at<NG>(prim + PR_P * nc, p, deriv_row<NG>(strides[d], c[d], g.n[d], g.bnd[2 * d], g.bnd[2 * d + 1],
+                                                        mt.dxi[d][c[d] - 1 + NG]));
   }
 }
 

