@@ -43,6 +43,7 @@ struct izem_ctx {
   std::vector<double> kt_ms;
   std::vector<std::vector<std::pair<cudaEvent_t, cudaEvent_t>>> kt_pending;
   bool have_eg = false;   // EGLIB linking data uploaded (izem_gpu_set_eglib)
+  long long* eg_tab = nullptr;   // its functions of T (eg_table.cuh)
   // threads per block chosen by izem_gpu_autotune (face fluxes, viscous point kernel)
   int tb_euler = 128, tb_visc = 128;
   // sensor x-blocks (izem_gpu_set_sensor_xblocks): block size in x (nx for

@@ -352,7 +352,7 @@ int enq_visc(izem_ctx* c) {
     const long long ns_all = slab_count(g);
     if ((rc = launch(c, "visc_point_eg", [&] {
            k_visc_point_eg<NRV, true><<<grid_for(ns_all, c->tb_visc), c->tb_visc, 0, c->stream>>>(
-               g, c->v, c->T, c->W_i, c->ha, c->Xa, c->prim, c->fd, c->tau, c->qv, sa);
+               g, c->v, c->T, c->W_i, c->ha, c->Xa, c->prim, c->fd, c->tau, c->qv, c->eg_tab, sa);
          })))
       return rc;
   } else if (les) {
@@ -365,7 +365,8 @@ int enq_visc(izem_ctx* c) {
     const long long ns_all = slab_count(g);
     if ((rc = launch(c, "visc_point_eg", [&] {
            k_visc_point_eg<NRV><<<grid_for(ns_all, c->tb_visc), c->tb_visc, 0, c->stream>>>(g, c->v, c->T, c->W_i, c->ha, c->Xa,
-                                                                                         c->prim, c->fd, c->tau, c->qv);
+                                                                                         c->prim, c->fd, c->tau, c->qv,
+                                                                                         c->eg_tab);
          })))
       return rc;
   } else if ((rc = launch(c, "visc_point", [&] {
@@ -661,6 +662,31 @@ int tune_flow(izem_ctx* c, std::string* rep) {
   return e == cudaSuccess ? IZEM_OK : ctx_fail(c, IZEM_ERR_CUDA, "autotune", e);
 }
 
+// The table of EGLIB's functions of T for the linking data just uploaded.
+// Where a coefficient does not fit its word (fits far from those of any gas)
+// the context has no table and every point evaluates the functions directly.
+template <int NRV>
+int eg_build_table(izem_ctx* c) {
+  using I = EgIdx<NRV>;
+  drop_graphs(c);   // captured graphs hold the table's address
+  const size_t words = (size_t)kEgRows * I::NF * 6;
+  if (!c->eg_tab) CK(cudaMalloc(&c->eg_tab, (words + 1) * sizeof(long long)));
+  int* bad = reinterpret_cast<int*>(c->eg_tab + words);
+  int h_bad = 1;
+  cudaError_t e = cudaMemsetAsync(bad, 0, sizeof(int), c->stream);
+  if (e == cudaSuccess) {
+    k_eg_table<NRV><<<kEgRows, kEgBuildThreads, 0, c->stream>>>(c->eg_tab, bad);
+    if ((e = cudaGetLastError()) == cudaSuccess &&
+        (e = cudaMemcpyAsync(&h_bad, bad, sizeof(int), cudaMemcpyDeviceToHost, c->stream)) == cudaSuccess)
+      e = cudaStreamSynchronize(c->stream);
+  }
+  if (e != cudaSuccess || h_bad) {
+    cudaFree(c->eg_tab);
+    c->eg_tab = nullptr;
+  }
+  return e == cudaSuccess ? IZEM_OK : ctx_fail(c, IZEM_ERR_CUDA, "EGLIB table", e);
+}
+
 // ================================================================ C ABI =====
 extern "C" {
 
@@ -828,7 +854,7 @@ void izem_gpu_destroy(izem_ctx* c) {
   if (c->d_chem_stats) cudaFree(c->d_chem_stats);
   if (c->h_chem_stats) cudaFreeHost(c->h_chem_stats);
   cudaFree(c->b_T); cudaFree(c->b_rho); cudaFree(c->b_Y); cudaFree(c->b_dt);
-  cudaFree(c->b_list); cudaFree(c->d_list_count); cudaFree(c->les); cudaFree(c->mu_sgs); cudaFree(c->d_y); cudaFree(c->d_z);
+  cudaFree(c->b_list); cudaFree(c->d_list_count); cudaFree(c->les); cudaFree(c->mu_sgs); cudaFree(c->eg_tab); cudaFree(c->d_y); cudaFree(c->d_z);
   if (c->h_status) cudaFreeHost(c->h_status);
   if (c->h_dt) cudaFreeHost(c->h_dt);
   for (auto& v : c->kt_pending)
@@ -1094,6 +1120,8 @@ int izem_gpu_set_eglib(izem_ctx* c, const izem_eglib* L) {
   DevEg e;
   eg_prepare(*L, c->thd, c->adi, e);
   CK(cudaMemcpyToSymbol(c_eg, &e, sizeof(DevEg)));
+  int rc = IZEM_DISPATCH(c, eg_build_table, c);
+  if (rc) return rc;
   c->have_eg = true;
   return IZEM_OK;
 }

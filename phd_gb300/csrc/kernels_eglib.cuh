@@ -42,8 +42,10 @@ struct DevEg {
   double bdiag[IZEM_NSMAX];       // 5 PATMOS W / (6 RU): D_int,kk = bdiag / (T A*_kk eta_k)
   double lfac[IZEM_NSMAX];        // 5 PATMOS W / (3 RU): FAC of Lambda_[e] = lfac / (T eta_k)
   double wsinv[IZEM_NSMAX][IZEM_NSMAX];                    // 1 / (W_i + W_j)
-  double hoff[IZEM_NSMAX][IZEM_NSMAX];                     // A*(1000) - 5/3
-  double hdi[IZEM_NSMAX][IZEM_NSMAX], hdj[IZEM_NSMAX][IZEM_NSMAX];   // A* W_j/W_i + 5/3, A* W_i/W_j + 5/3
+  // the shear matrix's pair constants over W_i + W_j: A*(1000) - 5/3, A* W_j/W_i + 5/3, A* W_i/W_j + 5/3
+  double hoff[IZEM_NSMAX][IZEM_NSMAX];
+  double hdi[IZEM_NSMAX][IZEM_NSMAX], hdj[IZEM_NSMAX][IZEM_NSMAX];
+  double cr[2][IZEM_NSMAX][5];    // internal heat capacity c_int in powers of the code-unit temperature
   double p1[IZEM_NSMAX][IZEM_NSMAX];                       // wwi wwj
   double tti[IZEM_NSMAX][IZEM_NSMAX], ttj[IZEM_NSMAX][IZEM_NSMAX];   // 4/3 wioj, 4/3 wjoi
   double c1j[IZEM_NSMAX][IZEM_NSMAX], c2j[IZEM_NSMAX][IZEM_NSMAX], c3j[IZEM_NSMAX][IZEM_NSMAX];
@@ -133,9 +135,9 @@ inline void eg_prepare(const izem_eglib& L, const izem_thd& t, const izem_adi& a
       const double wioj = 3.0 * wi / wj - 2.0, wjoi = 3.0 * wj / wi - 2.0;
       const double A = E.ctaij[i][j];
       E.wsinv[i][j] = 1.0 / (wi + wj);
-      E.hoff[i][j] = A - 5.0 / 3.0;
-      E.hdi[i][j] = A * wj / wi + 5.0 / 3.0;
-      E.hdj[i][j] = A * wi / wj + 5.0 / 3.0;
+      E.hoff[i][j] = (A - 5.0 / 3.0) / (wi + wj);
+      E.hdi[i][j] = (A * wj / wi + 5.0 / 3.0) / (wi + wj);
+      E.hdj[i][j] = (A * wi / wj + 5.0 / 3.0) / (wi + wj);
       const double p1 = wwi * wwj;
       E.p1[i][j] = p1;
       E.tti[i][j] = 4.0 / 3.0 * wioj;
@@ -152,238 +154,27 @@ inline void eg_prepare(const izem_eglib& L, const izem_thd& t, const izem_adi& a
   E.eta_adim = 1.0e-1 / t.muinf;
   E.lbda_adim = 1.0e-5 / t.laminf;
   E.rd_adim = 1.0e-1 / (a.rho_ref * t.dinf[0]);
+  for (int k = 0; k < n; ++k)
+    for (int r = 0; r < 2; ++r) {
+      double tp = t.gam2 * t.Wc_i[k] * E.cp_cgs * E.wtru[k];
+      for (int j = 0; j < 5; ++j) {
+        E.cr[r][k][j] = L.lin[k] ? t.heatcap[k][r][j] * tp : 0.0;
+        tp *= t.tinf;
+      }
+      if (L.lin[k]) E.cr[r][k][0] -= 2.5;
+    }
 }
+
+#include "eg_table.cuh"
 
 // packed symmetric index of EGLIB (0-based, i <= j)
 template <int N>
-__device__ __forceinline__ int egs(int i, int j) { return N * i - (i * (i + 1)) / 2 + j; }
-
-template <int N>
-__device__ __forceinline__ double eg_poly6(const double* f, double d1, double d2, double d3, double d4, double d5,
-                                           double d6) {
-  return f[0] + f[1] * d1 + f[2] * d2 + f[3] * d3 + f[4] * d4 + f[5] * d5 + f[6] * d6;
-}
-
-// One point: T [K], mole fractions, species cp [erg/g/K] -> eta [g/cm/s],
-// lambda [erg/cm/s/K], chi (N), rho * D [g/cm/s] as D[l*N+m].  The same
-// EGLIB formulas as the routines named above, with the factors that depend
-// only on the species (molar masses, EGLIB's fixed coefficients, Parker's
-// reference value) folded on the host, reciprocals instead of divisions,
-// 1/eta from exp(-ln eta), and the packed factorisation with its scaling
-// applied in place: the same quantities up to rounding.
-template <int N>
-__device__ void eg_point_dev(double T, const double* X, const double* cpms, double& eta_mix, double& tc,
-                             double* chit, double* D) {
-  constexpr int NP = N * (N + 1) / 2;
-  const double patmos = 1.01325e6, ru = 8.314e7;
-  const double Tinv = 1.0 / T;
-  // ---- LSPAR (IFLAG = 7): pure viscosities, reciprocal binary diffusion
-  // coefficients, internal heat capacities, Parker's rotational relaxation,
-  // internal self-diffusion on the diagonal of BIN
-  const double d1 = log(T);
-  const double d2 = d1 * d1, d3 = d2 * d1, d4 = d3 * d1, d5 = d4 * d1, d6 = d5 * d1;
-  double eta_i[N], bin[NP], cint[N], cxi[N];
-#pragma unroll
-  for (int k = 0; k < N; ++k) {
-    const double* ce = c_eg.cofe[k];
-    eta_i[k] = exp(-(ce[0] + ce[1] * d1 + ce[2] * d2 + ce[3] * d3));   // 1 / eta_k
-  }
-#pragma unroll
-  for (int k = 0; k < N; ++k)
-#pragma unroll
-    for (int l = k + 1; l < N; ++l) {
-      const double* cf = c_eg.cofd[k][l];
-      bin[egs<N>(k, l)] = exp(-(cf[0] + cf[1] * d1 + cf[2] * d2 + cf[3] * d3));
-    }
-  const double pfac = 1.0 + 2.985e3 / (T * sqrt(T));   // polar correction of D_int
-#pragma unroll
-  for (int k = 0; k < N; ++k) {
-    cint[k] = c_eg.lin[k] ? cpms[k] * c_eg.wtru[k] - 2.5 : 0.0;
-    const double dd = c_eg.eps[k] * Tinv, sqdd = sqrt(dd);
-    cxi[k] = c_eg.cx[k] * (1.0 + 2.7842 * sqdd + 4.4674 * dd + 5.5683 * (sqdd * dd));
-    const double aii = eg_poly6<N>(c_eg.fita[k][k], d1, d2, d3, d4, d5, d6);
-    double b = c_eg.bdiag[k] * Tinv * eta_i[k] / aii;
-    if (c_eg.dip[k] != 0.0) b = b * pfac;
-    bin[egs<N>(k, k)] = b;
-  }
-  // ---- EGSPAR: regularised mole and mass fractions
-  double sum = 0.0;
-#pragma unroll
-  for (int i = 0; i < N; ++i) sum = sum + X[i];
-  const double xm = sum * (1.0 / double(N)), sss = 1.0e-16;
-  double xtr[N], ytr[N], aux[N];
-  double wwtr = 0.0;
-#pragma unroll
-  for (int i = 0; i < N; ++i) {
-    xtr[i] = X[i] + sss * (xm - X[i]);
-    wwtr = wwtr + xtr[i] * c_eg.wt[i];
-  }
-  const double wwtr_i = 1.0 / wwtr;
-  double ysum = 0.0;
-#pragma unroll
-  for (int i = 0; i < N; ++i) { ytr[i] = xtr[i] * c_eg.wt[i] * wwtr_i; ysum = ysum + ytr[i]; }
-#pragma unroll
-  for (int i = 0; i < N; ++i) aux[i] = ysum - ytr[i];
-  double g[NP], an[N];
-  // ---- EGSE2: matrix H with the 1000 K A*, one conjugate-gradient step
-  {
-    const double fac = (6.0 * ru / (5.0 * patmos)) * T;
-#pragma unroll
-    for (int i = 0; i < N; ++i) g[egs<N>(i, i)] = xtr[i] * xtr[i] * eta_i[i];
-#pragma unroll
-    for (int i = 0; i < N; ++i)
-#pragma unroll
-      for (int j = i + 1; j < N; ++j) {
-        const double a = xtr[i] * xtr[j] * fac * bin[egs<N>(i, j)] * c_eg.wsinv[i][j];
-        g[egs<N>(i, j)] = a * c_eg.hoff[i][j];
-        g[egs<N>(i, i)] = g[egs<N>(i, i)] + a * c_eg.hdi[i][j];
-        g[egs<N>(j, j)] = g[egs<N>(j, j)] + a * c_eg.hdj[i][j];
-      }
-    double zn[N], tmp[N], aaa = 0.0;
-#pragma unroll
-    for (int i = 0; i < N; ++i) {
-      zn[i] = xtr[i] / g[egs<N>(i, i)];
-      aaa = aaa + zn[i] * xtr[i];
-      tmp[i] = g[egs<N>(i, i)] * zn[i];
-    }
-#pragma unroll
-    for (int i = 0; i < N; ++i)
-#pragma unroll
-      for (int j = i + 1; j < N; ++j) {
-        tmp[i] = tmp[i] + g[egs<N>(i, j)] * zn[j];
-        tmp[j] = tmp[j] + g[egs<N>(i, j)] * zn[i];
-      }
-    double bbb = 0.0, dot = 0.0;
-#pragma unroll
-    for (int i = 0; i < N; ++i) { bbb = bbb + zn[i] * tmp[i]; dot = dot + zn[i] * xtr[i]; }
-    eta_mix = aaa / bbb * dot;
-  }
-  // ---- EGSLCT2: matrix Lambda_[e], factorisation, solve
-  {
-    double beta[N];
-#pragma unroll
-    for (int i = 0; i < N; ++i) {
-      beta[i] = (2.5 + cint[i]) * xtr[i];
-      const double xx = xtr[i] * xtr[i];
-      g[egs<N>(i, i)] = c_eg.lfac[i] * Tinv * eta_i[i] * xx * (1.0 + (8.0 / 15.0) * cxi[i]) + xx * cint[i] * bin[egs<N>(i, i)];
-    }
-#pragma unroll
-    for (int i = 0; i < N; ++i)
-#pragma unroll
-      for (int j = i + 1; j < N; ++j) {
-        const double A = eg_poly6<N>(c_eg.fita[i][j], d1, d2, d3, d4, d5, d6);
-        const double B = eg_poly6<N>(c_eg.fitb[i][j], d1, d2, d3, d4, d5, d6);
-        const double a = xtr[i] * xtr[j] * bin[egs<N>(i, j)];
-        const double b3 = 6.25 - 3.0 * B;
-        const double bbb = c_eg.p1[i][j] * (13.75 - 3.0 * B - 4.0 * A + A * (c_eg.tti[i][j] * cxi[i] + c_eg.ttj[i][j] * cxi[j]));
-        const double a4 = 4.0 * A * c_eg.p1[i][j];
-        const double bbj = c_eg.c1j[i][j] + b3 * c_eg.c2j[i][j] + a4 + A * (c_eg.c3j[i][j] * cxi[i] + c_eg.c4[i][j] * cxi[j]);
-        const double bbi = c_eg.c1i[i][j] + b3 * c_eg.c2i[i][j] + a4 + A * (c_eg.c3i[i][j] * cxi[j] + c_eg.c4[i][j] * cxi[i]);
-        g[egs<N>(i, j)] = -bbb * a;
-        g[egs<N>(i, i)] = g[egs<N>(i, i)] + a * (bbj + cint[i]);
-        g[egs<N>(j, j)] = g[egs<N>(j, j)] + a * (bbi + cint[j]);
-      }
-    // EGSDEC (packed LDL^T) and EGSSOL
-#pragma unroll 1
-    for (int k = 0; k < N; ++k) {
-      double w[N];
-      for (int j = 0; j < k; ++j) w[j] = g[egs<N>(j, j)] * g[egs<N>(j, k)];
-      const int kk = egs<N>(k, k);
-      double gkk = g[kk];
-      for (int j = 0; j < k; ++j) gkk = gkk - w[j] * g[egs<N>(j, k)];
-      g[kk] = gkk;
-      const double rk = 1.0 / gkk;
-      for (int i = k + 1; i < N; ++i) {
-        double gki = g[egs<N>(k, i)];
-        for (int j = 0; j < k; ++j) gki = gki - g[egs<N>(j, i)] * w[j];
-        g[egs<N>(k, i)] = gki * rk;
-      }
-    }
-#pragma unroll
-    for (int i = 0; i < N; ++i) an[i] = beta[i];
-#pragma unroll
-    for (int j = 0; j < N - 1; ++j)
-#pragma unroll
-      for (int k = j + 1; k < N; ++k) an[k] = an[k] - g[egs<N>(j, k)] * an[j];
-#pragma unroll
-    for (int j = 0; j < N; ++j) an[j] = an[j] / g[egs<N>(j, j)];
-#pragma unroll
-    for (int j = N - 1; j >= 1; --j)
-#pragma unroll
-      for (int k = 0; k < j; ++k) an[k] = an[k] - g[egs<N>(k, j)] * an[j];
-    double s = 0.0;
-#pragma unroll
-    for (int i = 0; i < N; ++i) s = s + an[i] * beta[i];
-    tc = s * patmos * Tinv;
-#pragma unroll
-    for (int i = 0; i < N; ++i) chit[i] = 0.0;
-#pragma unroll
-    for (int i = 0; i < N; ++i)
-#pragma unroll
-      for (int j = i + 1; j < N; ++j) {
-        const double C = eg_poly6<N>(c_eg.fitc[i][j], d1, d2, d3, d4, d5, d6);
-        const double term = 0.5 * bin[egs<N>(i, j)] * (6.0 * C - 5.0) *
-                            (c_eg.wt[i] * an[j] - c_eg.wt[j] * an[i]) * c_eg.wsinv[i][j];
-        chit[i] = chit[i] + xtr[j] * term;
-        chit[j] = chit[j] - xtr[i] * term;
-      }
-  }
-  // ---- EGSDR1: matrix L_[00], two stationary steps, mass-conservation projection
-  {
-    double gd[N], dmi[N], tmp[N];
-#pragma unroll
-    for (int i = 0; i < N; ++i) gd[i] = 0.0;
-#pragma unroll
-    for (int i = 0; i < N; ++i)
-#pragma unroll
-      for (int j = i + 1; j < N; ++j) {
-        const double a = xtr[i] * xtr[j] * bin[egs<N>(i, j)];
-        g[egs<N>(i, j)] = a;   // holds -L_ij
-        gd[i] = gd[i] + a;
-        gd[j] = gd[j] + a;
-      }
-#pragma unroll
-    for (int i = 0; i < N; ++i) dmi[i] = aux[i] / gd[i];
-#pragma unroll
-    for (int i = 0; i < N; ++i) {
-      D[i * N + i] = ytr[i] * (dmi[i] * (1.0 + ytr[i]));
-#pragma unroll
-      for (int j = i + 1; j < N; ++j) {
-        const double dij = dmi[i] * dmi[j] * g[egs<N>(i, j)];
-        D[i * N + j] = ytr[i] * dij;
-        D[j * N + i] = ytr[j] * dij;
-      }
-    }
-    const double rsumy = 1.0 / sum;
-#pragma unroll
-    for (int i = 0; i < N; ++i) {
-      double t = 0.0;
-#pragma unroll
-      for (int j = 0; j < N; ++j) t = t + D[i * N + j] * ytr[j];
-      const double a = t * rsumy;
-#pragma unroll
-      for (int j = 0; j < N; ++j) D[i * N + j] = D[i * N + j] - a;
-    }
-#pragma unroll
-    for (int i = 0; i < N; ++i) tmp[i] = 0.0;
-#pragma unroll
-    for (int j = 0; j < N; ++j)
-#pragma unroll
-      for (int i = 0; i < N; ++i) tmp[i] = tmp[i] + D[j * N + i];
-    const double aa = (patmos / ru) * wwtr * Tinv;
-#pragma unroll
-    for (int i = 0; i < N; ++i) {
-      const double yr = ytr[i] * rsumy;
-#pragma unroll
-      for (int j = 0; j < N; ++j) D[i * N + j] = aa * (D[i * N + j] - yr * tmp[j]);
-    }
-  }
-}
+__host__ __device__ constexpr int egs(int i, int j) { return N * i - (i * (i + 1)) / 2 + j; }
 
 // Species cp of egvars (module_eg_lib.f90:170-240): NASA-7 with the linear
 // extrapolation outside [Tpolymin, Tpolymax], in erg/g/K.
 template <int N>
-__device__ __forceinline__ void eg_species_cp(double T, double* cpk) {
+__device__ __noinline__ void eg_species_cp(double T, double* cpk) {
 #pragma unroll
   for (int is = 0; is < N; ++is) {
     double t1 = T * c_thd.tinf, t2 = t1 * t1, t3 = t2 * t1, t4 = t3 * t1;
@@ -406,6 +197,232 @@ __device__ __forceinline__ void eg_species_cp(double T, double* cpk) {
       cpv = c_thd.gam2 * c_thd.Wc_i[is] * (dcp0 * (T * c_thd.tinf - c_thd.tpolymax[is]) + cp0);
     }
     cpk[is] = cpv * c_eg.cp_cgs;
+  }
+}
+
+// c_int of every species: c_p / R - 5/2 (0 for an atom)
+template <int N>
+__device__ __forceinline__ void eg_cint(double T, double* cint) {
+  const int r = th_range(T);
+  if (r >= 0) {
+#pragma unroll
+    for (int k = 0; k < N; ++k) {
+      const double* a = c_eg.cr[r][k];
+      cint[k] = fma(T, fma(T, fma(T, fma(T, a[4], a[3]), a[2]), a[1]), a[0]);
+    }
+    return;
+  }
+  double cpk[N];
+  eg_species_cp<N>(T, cpk);
+#pragma unroll
+  for (int k = 0; k < N; ++k) cint[k] = c_eg.lin[k] ? cpk[k] * c_eg.wtru[k] - 2.5 : 0.0;
+}
+
+// What the fluxes of one point take from EGLIB: the viscosity, the
+// conductivity, the thermal diffusion ratios, and the flux diffusion matrix
+// rho D as an operator.  EGSDR1 forms D = P2 (y_i (dmi_i a_ij dmi_j + (1 +
+// y_i) dmi_i delta_ij) - a_i) with the row averages a_i and the column
+// projection P2; its product with a vector needs the symmetric a_ij and
+// rank-one terms only, 99 FP64 operations a vector plus 43 for the
+// projections, against 400 to build the projected 9 x 9 matrix and 81 a
+// product.
+template <int N>
+struct EgPoint {
+  double eta, tc;                         // [g/cm/s], [erg/cm/s/K]
+  double chi[N];
+  double a[N * (N - 1) / 2];              // x_i x_j / D_ij
+  double dmi[N], yd[N], oney[N], sa[N], yr[N];
+  double scale;                           // PATM / RU times W / T
+
+  // rho D u over `scale`
+  __device__ __forceinline__ void apply(const double* u, double* out) const {
+    double e[N], U = 0.0, Q = 0.0;
+#pragma unroll
+    for (int i = 0; i < N; ++i) {
+      e[i] = dmi[i] * u[i];
+      out[i] = oney[i] * u[i];
+      U = U + u[i];
+    }
+#pragma unroll
+    for (int i = 0; i < N; ++i)
+#pragma unroll
+      for (int j = i + 1; j < N; ++j) {
+        const double aij = a[egp<N>(i, j)];
+        out[i] = fma(aij, e[j], out[i]);
+        out[j] = fma(aij, e[i], out[j]);
+      }
+#pragma unroll
+    for (int i = 0; i < N; ++i) {
+      out[i] = fma(yd[i], out[i], -(sa[i] * U));
+      Q = Q + out[i];
+    }
+#pragma unroll
+    for (int i = 0; i < N; ++i) out[i] = fma(-yr[i], Q, out[i]);
+  }
+};
+
+// One point: T [K], mole fractions X, c_int -> EgPoint.  The EGLIB formulas
+// of the routines named above on the tabulated functions of T, in another
+// order of operations: the same quantities up to rounding (against 80-bit
+// arithmetic on random states: eta 8e-16 -> 2e-16, rho D 1.0e-15 -> 2.9e-16,
+// the conductivity and the thermal diffusion ratios, which an ill-conditioned
+// solve dominates, unchanged).
+template <int N>
+__device__ __forceinline__ void eg_point(double T, const double* X, const double* cint,
+                                         const long long* __restrict__ tab, EgPoint<N>& o) {
+  using I = EgIdx<N>;
+  const double patmos = 1.01325e6, ru = 8.314e7;
+  const EgRow row = eg_row<N>(tab, T);
+  double tv[I::NF];   // functions of T of a point outside the table (local memory)
+  if (!row.row) eg_direct<N>(T, tv);
+  auto f = [&](int k) -> double { return row.row ? eg_eval<true>(row, k) : tv[k]; };
+  auto fs = [&](int k) -> double { return row.row ? eg_eval<false>(row, k) : tv[k]; };   // of either sign
+  // ---- EGSPAR: regularised mole and mass fractions
+  double sum = 0.0;
+#pragma unroll
+  for (int i = 0; i < N; ++i) sum = sum + X[i];
+  const double xm = sum * (1.0 / double(N)), sss = 1.0e-16;
+  double xtr[N], ytr[N], wwtr = 0.0;
+#pragma unroll
+  for (int i = 0; i < N; ++i) {
+    xtr[i] = fma(sss, xm - X[i], X[i]);
+    wwtr = fma(xtr[i], c_eg.wt[i], wwtr);
+  }
+  const double wwtr_i = fm_rcp(wwtr);
+  double ysum = 0.0;
+#pragma unroll
+  for (int i = 0; i < N; ++i) {
+    ytr[i] = xtr[i] * c_eg.wt[i] * wwtr_i;
+    ysum = ysum + ytr[i];
+  }
+  double gd[N];
+#pragma unroll
+  for (int i = 0; i < N; ++i) gd[i] = 0.0;
+  double g[I::NP], gdiag[N];
+  // ---- EGSE2: matrix H over its common factor 6 RU T / (5 PATM), with the
+  // 1000 K A*; one conjugate-gradient step.  The pairs' x_i x_j / D_ij and
+  // their row sums serve the other routines too.
+  {
+#pragma unroll
+    for (int i = 0; i < N; ++i) gdiag[i] = xtr[i] * xtr[i] * f(I::shear + i);
+#pragma unroll
+    for (int i = 0; i < N; ++i)
+#pragma unroll
+      for (int j = i + 1; j < N; ++j) {
+        const double a = (xtr[i] * xtr[j]) * f(I::bin + egp<N>(i, j));
+        o.a[egp<N>(i, j)] = a;
+        gd[i] = gd[i] + a;
+        gd[j] = gd[j] + a;
+        g[egp<N>(i, j)] = a * c_eg.hoff[i][j];
+        gdiag[i] = fma(a, c_eg.hdi[i][j], gdiag[i]);
+        gdiag[j] = fma(a, c_eg.hdj[i][j], gdiag[j]);
+      }
+    // z = x / diag(H), (z.x)^2 / (z.H z); H z holds x from the diagonal
+    double zn[N], zx = 0.0, zo = 0.0;
+#pragma unroll
+    for (int i = 0; i < N; ++i) {
+      zn[i] = fm_div(xtr[i], gdiag[i]);
+      zx = fma(zn[i], xtr[i], zx);
+    }
+#pragma unroll
+    for (int i = 0; i < N; ++i) {
+      double t = 0.0;
+#pragma unroll
+      for (int j = i + 1; j < N; ++j) t = fma(g[egp<N>(i, j)], zn[j], t);
+      zo = fma(zn[i], t, zo);
+    }
+    o.eta = fm_div(zx * zx, fma(2.0, zo, zx) * ((6.0 * ru / (5.0 * patmos)) * T));
+  }
+  // ---- EGSLCT2: matrix Lambda_[e], factorisation (EGSDEC: L D L^T), solve
+  {
+    double an[N], beta[N], ri[N];
+#pragma unroll
+    for (int i = 0; i < N; ++i) {
+      beta[i] = (2.5 + cint[i]) * xtr[i];
+      an[i] = beta[i];
+      const double d = fma(cint[i], f(I::spec + 2 * i + 1), f(I::spec + 2 * i));
+      gdiag[i] = fma(xtr[i] * xtr[i], d, cint[i] * gd[i]);
+    }
+#pragma unroll
+    for (int i = 0; i < N; ++i)
+#pragma unroll
+      for (int j = i + 1; j < N; ++j) {
+        const int q = I::lam + 3 * egp<N>(i, j);
+        const double xx = xtr[i] * xtr[j];
+        g[egp<N>(i, j)] = -xx * f(q);
+        gdiag[i] = fma(xx, f(q + 1), gdiag[i]);
+        gdiag[j] = fma(xx, f(q + 2), gdiag[j]);
+      }
+    // row by row: the multipliers of column k replace its entries
+#pragma unroll
+    for (int k = 0; k < N; ++k) {
+      double w[N];
+#pragma unroll
+      for (int j = 0; j < k; ++j) w[j] = gdiag[j] * g[egp<N>(j, k)];
+#pragma unroll
+      for (int j = 0; j < k; ++j) gdiag[k] = fma(-w[j], g[egp<N>(j, k)], gdiag[k]);
+      ri[k] = fm_rcp(gdiag[k]);
+#pragma unroll
+      for (int i = k + 1; i < N; ++i) {
+        double t = g[egp<N>(k, i)];
+#pragma unroll
+        for (int j = 0; j < k; ++j) t = fma(-g[egp<N>(j, i)], w[j], t);
+        g[egp<N>(k, i)] = t * ri[k];
+      }
+    }
+#pragma unroll
+    for (int j = 0; j < N - 1; ++j)
+#pragma unroll
+      for (int k = j + 1; k < N; ++k) an[k] = fma(-g[egp<N>(j, k)], an[j], an[k]);
+#pragma unroll
+    for (int j = 0; j < N; ++j) an[j] = an[j] * ri[j];
+#pragma unroll
+    for (int j = N - 1; j >= 1; --j)
+#pragma unroll
+      for (int k = 0; k < j; ++k) an[k] = fma(-g[egp<N>(k, j)], an[j], an[k]);
+    double s = 0.0;
+#pragma unroll
+    for (int i = 0; i < N; ++i) s = fma(an[i], beta[i], s);
+    const double Tinv = fm_rcp(T);
+    o.tc = s * patmos * Tinv;
+    o.scale = (patmos / ru) * wwtr * Tinv;
+#pragma unroll
+    for (int i = 0; i < N; ++i) o.chi[i] = 0.0;
+#pragma unroll
+    for (int i = 0; i < N; ++i)
+#pragma unroll
+      for (int j = i + 1; j < N; ++j) {
+        const double term = fs(I::chi + egp<N>(i, j)) * (c_eg.wt[i] * an[j] - c_eg.wt[j] * an[i]);
+        o.chi[i] = fma(xtr[j], term, o.chi[i]);
+        o.chi[j] = fma(-xtr[i], term, o.chi[j]);
+      }
+  }
+  // ---- EGSDR1: the operator's vectors (L_[00], two stationary steps, projection)
+  {
+    const double rsumy = fm_rcp(sum);
+#pragma unroll
+    for (int i = 0; i < N; ++i) {
+      o.dmi[i] = fm_div(ysum - ytr[i], gd[i]);
+      o.yd[i] = ytr[i] * o.dmi[i];
+      o.oney[i] = 1.0 + ytr[i];
+      o.yr[i] = ytr[i] * rsumy;
+    }
+    double t[N], e[N];
+#pragma unroll
+    for (int i = 0; i < N; ++i) {
+      e[i] = o.dmi[i] * ytr[i];
+      t[i] = o.oney[i] * ytr[i];
+    }
+#pragma unroll
+    for (int i = 0; i < N; ++i)
+#pragma unroll
+      for (int j = i + 1; j < N; ++j) {
+        const double aij = o.a[egp<N>(i, j)];
+        t[i] = fma(aij, e[j], t[i]);
+        t[j] = fma(aij, e[i], t[j]);
+      }
+#pragma unroll
+    for (int i = 0; i < N; ++i) o.sa[i] = o.yd[i] * t[i] * rsumy;
   }
 }
 
@@ -506,13 +523,18 @@ __global__ void k_les_prep(Geo g, Metrics mt, const double* __restrict__ v, cons
 // stresses.  The reference reuses its temperature-gradient scalar wrk1 for
 // the SGS factor of each species, so the x thermal-diffusion term of species
 // l >= 2 uses the SGS factor of species l - 1; that is reproduced.
+// Bound by the FP64 pipe: 5154 -> 1893 instructions a point with nine species,
+// 91.2 -> 35.7 ms on 256 x 256 x 128 (73 % of the pipe busy), 0.75 -> 0.25 ms
+// on 33 x 40 x 21.  Two blocks of 256 threads an SM, i.e. 128 registers: the
+// spills hit L1, and 16 warps hide the integer chains of the table better than
+// 8 with 255 registers do (41.5 ms; 168: 39.5, 96: 38.4, 80: 40.2).
 template <int NRV, bool LES = false>
-__global__ void __launch_bounds__(256) k_visc_point_eg(Geo g, const double* __restrict__ v,
+__global__ void __launch_bounds__(256, 2) k_visc_point_eg(Geo g, const double* __restrict__ v,
                                                        const double* __restrict__ T, const double* __restrict__ W_i,
                                                        const double* __restrict__ ha, const double* __restrict__ Xa,
                                                        const double* __restrict__ prim, double* __restrict__ fd,
                                                        double* __restrict__ tau, double* __restrict__ qv,
-                                                       SgsArgs sa = SgsArgs{}) {
+                                                       const long long* __restrict__ tab, SgsArgs sa = SgsArgs{}) {
   long long idx = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   int i, j, k, dom;
   if (!slab_point(g, idx, i, j, k, dom)) return;
@@ -520,35 +542,33 @@ __global__ void __launch_bounds__(256) k_visc_point_eg(Geo g, const double* __re
   const long long nc = g.ncell;
   const long long p = gid(g, i, j, k);
   const double rho = v[p], Tp = T[p], Wi = W_i[p];
-  const double rho_i = 1.0 / rho;
+  const double rho_i = fm_rcp(rho);
   // ---- egvars
-  double Xe[NRV], cpk[NRV];
+  EgPoint<NRV> eg;
   {
-    const double wrk = rho_i * (1.0 / Wi);
+    double Xe[NRV], cint[NRV];
+    const double wrk = rho_i * fm_rcp(Wi);
 #pragma unroll
     for (int l = 0; l < NRV; ++l) Xe[l] = v[(IZEM_NIV + l) * nc + p] * wrk * c_thd.Wc_i[l];
-    eg_species_cp<NRV>(Tp, cpk);
+    eg_cint<NRV>(Tp, cint);
+    eg_point<NRV>(Tp * c_thd.tinf, Xe, cint, tab, eg);
   }
-  double eta_eg, ct_eg, tdr[NRV], rd[NRV * NRV];
-  eg_point_dev<NRV>(Tp * c_thd.tinf, Xe, cpk, eta_eg, ct_eg, tdr, rd);
-  const double mu = eta_eg * c_eg.eta_adim;
-  const double ct = ct_eg * c_eg.lbda_adim;
+  const double mu = eg.eta * c_eg.eta_adim;
+  const double ct = eg.tc * c_eg.lbda_adim;
   // ---- fluxes
   auto F = [&](int q1) -> double { return fd[(long long)(q1 - 1) * nc + p]; };
-  const double rmu = -c_thd.sqgmr * mu;
-  const double rmk = -c_thd.sqgmr * 0.0;
-  const double bulk = rmk * (F(1) + F(5) + F(9));
+  const double rmu = -c_thd.sqgmr * mu;   // the volume viscosity is 0 (module_eg_lib.f90:288)
   const double twothirds = 2.0 / 3.0;
-  const double sxx = bulk + twothirds * rmu * (F(1) + F(1) - (F(5) + F(9)));
+  const double sxx = twothirds * rmu * (F(1) + F(1) - (F(5) + F(9)));
   const double sxy = rmu * (F(4) + F(2));
   const double sxz = rmu * (F(7) + F(3));
-  const double syy = bulk + twothirds * rmu * (F(5) + F(5) - (F(1) + F(9)));
+  const double syy = twothirds * rmu * (F(5) + F(5) - (F(1) + F(9)));
   const double syz = rmu * (F(8) + F(6));
-  const double szz = bulk + twothirds * rmu * (F(9) + F(9) - (F(1) + F(5)));
+  const double szz = twothirds * rmu * (F(9) + F(9) - (F(1) + F(5)));
   double mu_sgs = 0.0;
   if constexpr (LES) {
     const double dxv = sa.dxi[0][i - 1 + g.ng], dyv = sa.dxi[1][j - 1 + g.ng], dzv = sa.dxi[2][k - 1 + g.ng];
-    const double delta = 1.0 / pow(dxv * dyv * dzv, 1.0 / 3.0);
+    const double delta = fm_rcp(fm_root(dxv * dyv * dzv, 1.0 / 3.0));
     const double s11 = F(1), s12 = 0.5 * (F(2) + F(4)), s13 = 0.5 * (F(3) + F(7));
     const double s22 = F(5), s23 = 0.5 * (F(6) + F(8)), s33 = F(9);
     double sb = s11 * s11 + s12 * s12 + s13 * s13 + s12 * s12 + s22 * s22 + s23 * s23 + s13 * s13 + s23 * s23 +
@@ -556,72 +576,68 @@ __global__ void __launch_bounds__(256) k_visc_point_eg(Geo g, const double* __re
     sb = sqrt(sb + sb);
     mu_sgs = rho * sa.cs2 * (delta * delta) * sb * sa.les[3 * nc + p];
   }
-  const double Ps = 1.0 / prim[PR_P * nc + p];
-  const double Ts = 1.0 / Tp;
-  const double w1 = F(10) * Ts, w2 = F(11) * Ts, w3 = F(12) * Ts;
-  const double w4 = fd[(12 + 3 * NRV) * nc + p] * Ps;
-  const double w5 = fd[(13 + 3 * NRV) * nc + p] * Ps;
-  const double w6 = fd[(14 + 3 * NRV) * nc + p] * Ps;
-  double dx[NRV], dy[NRV], dz[NRV], xt[NRV], xa[NRV];
+  const double Ps = fm_rcp(prim[PR_P * nc + p]);
+  const double Ts = fm_rcp(Tp);
+  // the diffusion driving forces of the three directions, one by one
+  double xt[NRV], hk[NRV];
 #pragma unroll
   for (int l = 0; l < NRV; ++l) {
-    const double X = Xa[l * nc + p];
-    xa[l] = X;
-    const double xy = X - v[(IZEM_NIV + l) * nc + p] * rho_i;
-    dx[l] = F(13 + 3 * l) + xy * w4;
-    dy[l] = F(14 + 3 * l) + xy * w5;
-    dz[l] = F(15 + 3 * l) + xy * w6;
-    xt[l] = X * tdr[l];
+    xt[l] = Xa[l * nc + p] * eg.chi[l];
+    hk[l] = fma(Tp * c_thd.Wc_i[l], eg.chi[l], ha[l * nc + p]);
   }
-  const double rvd0 = c_thd.rvd0;
-  const double uxs = v[nc + p] * rho_i, vys = v[2 * nc + p] * rho_i, wzs = v[3 * nc + p] * rho_i;
-  double sx = 0.0, sy = 0.0, sz = 0.0;
+  const double jsc = -c_thd.rvd0 * eg.scale * c_eg.rd_adim;
+  double sh[3];
+  // LES: rho D of the thermal diffusion ratios on its own, since the x term
+  // of species l takes the reference's reused scalar (wrk1)
+  double jt[LES ? NRV : 1];
+  if constexpr (LES) eg.apply(xt, jt);
   const double dm_sgs = mu_sgs * rho_i * sa.sc_sgs_i;
-  double w1c = w1;   // the reference's wrk1
 #pragma unroll
-  for (int l = 0; l < NRV; ++l) {
-    double jx = 0.0, jy = 0.0, jz = 0.0;
+  for (int d = 0; d < 3; ++d) {
+    const double wT = F(10 + d) * Ts, wP = fd[(12 + 3 * NRV + d) * nc + p] * Ps;
+    double u[NRV], jd[NRV];
 #pragma unroll
-    for (int m = 0; m < NRV; ++m) {
-      const double r = rd[l * NRV + m] * c_eg.rd_adim;
-      jx = jx + r * (dx[m] + xt[m] * (LES ? w1c : w1));
-      jy = jy + r * (dy[m] + xt[m] * w2);
-      jz = jz + r * (dz[m] + xt[m] * w3);
+    for (int l = 0; l < NRV; ++l) {
+      const double xy = fma(-v[(IZEM_NIV + l) * nc + p], rho_i, Xa[l * nc + p]);
+      u[l] = fma(xy, wP, F(13 + 3 * l + d));
+      if constexpr (!LES) u[l] = fma(xt[l], wT, u[l]);
     }
-    if constexpr (LES) {
-      const double wk = rho * dm_sgs * sa.sc * c_thd.Wc[l];
-      const double fw = 1.0 + wk * Wi;
-      const double wx = wk * xa[l];
-      jx = -rvd0 * (jx * fw + wx * sa.les[p]);
-      jy = -rvd0 * (jy * fw + wx * sa.les[nc + p]);
-      jz = -rvd0 * (jz * fw + wx * sa.les[2 * nc + p]);
-      w1c = wk;
-    } else {
-      jx = -rvd0 * jx;
-      jy = -rvd0 * jy;
-      jz = -rvd0 * jz;
+    eg.apply(u, jd);
+    double s = 0.0;
+#pragma unroll
+    for (int l = 0; l < NRV; ++l) {
+      double jl;
+      if constexpr (LES) {
+        const double wk = rho * dm_sgs * sa.sc * c_thd.Wc[l];
+        const double fw = 1.0 + wk * Wi;
+        const double wx = wk * Xa[l * nc + p];
+        // wrk1 at species l: the temperature factor for the first, then the
+        // SGS factor of the species before
+        const double w1 = (d == 0 && l > 0) ? rho * dm_sgs * sa.sc * c_thd.Wc[l > 0 ? l - 1 : 0] : wT;
+        const double jm = fma(w1, jt[LES ? l : 0], jd[l]) * (eg.scale * c_eg.rd_adim);
+        jl = -c_thd.rvd0 * (jm * fw + wx * sa.les[d * nc + p]);
+      } else {
+        jl = jsc * jd[l];
+      }
+      fd[(long long)(12 + 3 * l + d) * nc + p] = jl;
+      s = fma(jl, hk[l], s);
     }
-    fd[(long long)(12 + 3 * l) * nc + p] = jx;
-    fd[(long long)(13 + 3 * l) * nc + p] = jy;
-    fd[(long long)(14 + 3 * l) * nc + p] = jz;
-    const double h = ha[l * nc + p] + Tp * c_thd.Wc_i[l] * tdr[l];
-    sx = sx + jx * h;
-    sy = sy + jy * h;
-    sz = sz + jz * h;
+    sh[d] = s;
   }
+  const double uxs = v[nc + p] * rho_i, vys = v[2 * nc + p] * rho_i, wzs = v[3 * nc + p] * rho_i;
   double wl;
   if constexpr (LES) {
     const double ct_sgs = mu_sgs * sa.cp[p] * sa.pr_sgs_i;
     wl = -c_thd.rlam0 * (ct + ct_sgs);
-    const double fs = 1.0 + -c_thd.sqgmr * mu_sgs / rmu;
-    tau[0 * nc + p] = bulk + (sxx - bulk) * fs; tau[1 * nc + p] = sxy * fs; tau[2 * nc + p] = sxz * fs;
-    tau[3 * nc + p] = bulk + (syy - bulk) * fs; tau[4 * nc + p] = syz * fs; tau[5 * nc + p] = bulk + (szz - bulk) * fs;
+    const double fs = 1.0 + fm_div(-c_thd.sqgmr * mu_sgs, rmu);
+    tau[0 * nc + p] = sxx * fs; tau[1 * nc + p] = sxy * fs; tau[2 * nc + p] = sxz * fs;
+    tau[3 * nc + p] = syy * fs; tau[4 * nc + p] = syz * fs; tau[5 * nc + p] = szz * fs;
   } else {
     wl = -c_thd.rlam0 * ct;
     tau[0 * nc + p] = sxx; tau[1 * nc + p] = sxy; tau[2 * nc + p] = sxz;
     tau[3 * nc + p] = syy; tau[4 * nc + p] = syz; tau[5 * nc + p] = szz;
   }
-  qv[0 * nc + p] = sx + wl * F(10) + uxs * sxx + vys * sxy + wzs * sxz;
-  qv[1 * nc + p] = sy + wl * F(11) + uxs * sxy + vys * syy + wzs * syz;
-  qv[2 * nc + p] = sz + wl * F(12) + uxs * sxz + vys * syz + wzs * szz;
+  qv[0 * nc + p] = sh[0] + wl * F(10) + uxs * sxx + vys * sxy + wzs * sxz;
+  qv[1 * nc + p] = sh[1] + wl * F(11) + uxs * sxy + vys * syy + wzs * syz;
+  qv[2 * nc + p] = sh[2] + wl * F(12) + uxs * sxz + vys * syz + wzs * szz;
 }
