@@ -44,8 +44,8 @@ struct izem_ctx {
   std::vector<std::vector<std::pair<cudaEvent_t, cudaEvent_t>>> kt_pending;
   bool have_eg = false;   // EGLIB linking data uploaded (izem_gpu_set_eglib)
   long long* eg_tab = nullptr;   // its functions of T (eg_table.cuh)
-  // threads per block chosen by izem_gpu_autotune (face fluxes, viscous point kernel)
-  int tb_euler = 128, tb_visc = 128;
+  // threads per block chosen by izem_gpu_autotune (face fluxes, viscous point kernel); 0: by the grid's size
+  int tb_euler = 0, tb_visc = 0;
   // sensor x-blocks (izem_gpu_set_sensor_xblocks): block size in x (nx for
   // one block) and the block-edge faces as seen by the right block
   int sensor_bx = 0;

@@ -28,7 +28,21 @@ namespace {
 constexpr int kThreads = 128;
 constexpr int kNewtonChunk = 4;    // direct-launch Newton: iterations between two host reads of the stop flags
 
-unsigned grid_for(long long n, int threads = kThreads) { return (unsigned)((n + threads - 1) / threads); }
+unsigned grid_for(long long n, int threads) { return (unsigned)((n + threads - 1) / threads); }
+
+// Threads per block of a point kernel over n points.  The point kernels are
+// bound by the FP64 pipe of the SM that they run on, which a few warps fill,
+// so a grid of few warps is cut into smaller blocks that reach more SMs and
+// leave a fuller last wave: below 32 warps an SM blocks of 64, below 8 of 32.
+// A step of 33 x 40 x 21 points (6 warps an SM) takes 7.75 ms with blocks of
+// 128, 7.35 of 64 and 7.39 of 32; the fluxes of 61 x 50 x 38 (24 warps an SM)
+// 2.17, 2.07 and 2.06; above the line (160 x 128 x 64, 270 warps an SM) 82.9,
+// 83.5 and 84.4, the smaller blocks paying for their launch.
+int tb(const izem_ctx* c, long long n) {
+  const long long warps = (n + 31) / 32;
+  return warps >= 32LL * c->nsm ? kThreads : (warps >= 8LL * c->nsm ? 64 : 32);
+}
+int tb_or(const izem_ctx* c, int tuned, long long n) { return tuned ? tuned : tb(c, n); }
 
 }  // namespace
 
@@ -202,8 +216,8 @@ int enq_newton(izem_ctx* c, int ghost, double eps, int itmax, int check_negT) {
     return rc;
   auto iterate = [&](cudaGraphConditionalHandle cond, int use_cond) -> int {
     int r = launch(c, iname, [&] {
-      k_newton_iter<NRV><<<grid_for(n), kThreads, 0, c->stream>>>(g, ghost, c->v, c->T, c->cp, c->ha, c->d_status, check_negT,
-                                                                  bx);
+      k_newton_iter<NRV><<<grid_for(n, tb(c, n)), tb(c, n), 0, c->stream>>>(g, ghost, c->v, c->T, c->cp, c->ha, c->d_status,
+                                                                            check_negT, bx);
     });
     if (r) return r;
     return launch(c, "newton_check", [&] {
@@ -259,7 +273,7 @@ int enq_prim(izem_ctx* c) {
   const Geo& g = c->g;
   long long n = slab_count(g);
   return launch(c, "prim", [&] {
-    k_prim<NRV><<<grid_for(n), kThreads, 0, c->stream>>>(g, c->v, c->T, c->W_i, c->cp, c->ha, c->prim,
+    k_prim<NRV><<<grid_for(n, tb(c, n)), tb(c, n), 0, c->stream>>>(g, c->v, c->T, c->W_i, c->cp, c->ha, c->prim,
                                                           c->cfg.vis ? c->Xa : nullptr, c->d_status);
   });
 }
@@ -272,7 +286,7 @@ int enq_euler(izem_ctx* c, int d) {
   int rc;
   const char* names[3] = {"euler_face_x", "euler_face_y", "euler_face_z"};
 #define IZEM_FACE(DD, NGV)                                                                                         \
-  k_euler_face<NRV, DD, NGV><<<grid_for(nf, c->tb_euler), c->tb_euler, 0, c->stream>>>(                                \
+  k_euler_face<NRV, DD, NGV><<<grid_for(nf, tb_or(c, c->tb_euler, nf)), tb_or(c, c->tb_euler, nf), 0, c->stream>>>(                                \
       g, c->cfg.weno_avg, c->cfg.weno5_linear_fix, c->v, c->prim, c->sensor, c->fhat, nf, c->sensor_bx, 0)
   rc = launch(c, names[d], [&] {
     if (g.ng == 4) {   // WENO7
@@ -290,7 +304,7 @@ int enq_euler(izem_ctx* c, int d) {
   if (d == 0 && c->sensor_bx < g.n[0]) {   // block-edge faces as seen by the right block
     rc = launch(c, "euler_face_edge", [&] {
 #define IZEM_EDGE(NGV)                                                                                            \
-  k_euler_face<NRV, 0, NGV><<<grid_for(c->nedge, c->tb_euler), c->tb_euler, 0, c->stream>>>(                      \
+  k_euler_face<NRV, 0, NGV><<<grid_for(c->nedge, tb(c, c->nedge)), tb(c, c->nedge), 0, c->stream>>>(                      \
       g, c->cfg.weno_avg, c->cfg.weno5_linear_fix, c->v, c->prim, c->sensor, c->fhat_edge, c->nedge, c->sensor_bx, 1)
       if (g.ng == 4) IZEM_EDGE(4);
       else IZEM_EDGE(3);
@@ -300,9 +314,9 @@ int enq_euler(izem_ctx* c, int d) {
   if (rc) return rc;
   return launch(c, "flux_diff", [&] {
     const int bx = c->sensor_bx;
-    if (d == 0) k_flux_diff<0><<<grid_for(g.nint), kThreads, 0, c->stream>>>(g, NV, c->fhat, nf, c->dxi[0], c->f, 0, bx, c->fhat_edge, c->nedge);
-    if (d == 1) k_flux_diff<1><<<grid_for(g.nint), kThreads, 0, c->stream>>>(g, NV, c->fhat, nf, c->dxi[1], c->f, 1, bx, c->fhat_edge, c->nedge);
-    if (d == 2) k_flux_diff<2><<<grid_for(g.nint), kThreads, 0, c->stream>>>(g, NV, c->fhat, nf, c->dxi[2], c->f, 1, bx, c->fhat_edge, c->nedge);
+    if (d == 0) k_flux_diff<0><<<grid_for(g.nint, tb(c, g.nint)), tb(c, g.nint), 0, c->stream>>>(g, NV, c->fhat, nf, c->dxi[0], c->f, 0, bx, c->fhat_edge, c->nedge);
+    if (d == 1) k_flux_diff<1><<<grid_for(g.nint, tb(c, g.nint)), tb(c, g.nint), 0, c->stream>>>(g, NV, c->fhat, nf, c->dxi[1], c->f, 1, bx, c->fhat_edge, c->nedge);
+    if (d == 2) k_flux_diff<2><<<grid_for(g.nint, tb(c, g.nint)), tb(c, g.nint), 0, c->stream>>>(g, NV, c->fhat, nf, c->dxi[2], c->f, 1, bx, c->fhat_edge, c->nedge);
   });
 }
 
@@ -316,26 +330,28 @@ int enq_visc(izem_ctx* c) {
   int rc;
   if ((rc = launch(c, "visc_grad", [&] {
          auto kern = g.ng == 4 ? k_grad<NRV, 4> : k_grad<NRV, 3>;
-         kern<<<grid_for(g.nint), kThreads, 0, c->stream>>>(g, mt, c->prim, c->T, c->Xa, c->fd);
+         kern<<<grid_for(g.nint, tb(c, g.nint)), tb(c, g.nint), 0, c->stream>>>(g, mt, c->prim, c->T, c->Xa, c->fd);
        })))
     return rc;
   if (eg && (rc = launch(c, "visc_grad_p", [&] {
                auto kern = g.ng == 4 ? k_grad_p<NRV, 4> : k_grad_p<NRV, 3>;
-               kern<<<grid_for(g.nint), kThreads, 0, c->stream>>>(g, mt, c->prim, c->fd);
+               kern<<<grid_for(g.nint, tb(c, g.nint)), tb(c, g.nint), 0, c->stream>>>(g, mt, c->prim, c->fd);
              })))
     return rc;
   const bool les = c->les_on;
   if (les && (rc = launch(c, "les_prep", [&] {
                 // the criterion of shock_det_slv under EGLIB, of shock_det_ducros_slv with the fitted transport
-                k_les_prep<<<grid_for(g.nint), kThreads, 0, c->stream>>>(g, mt, c->v, c->T, c->W_i, c->les_pw, c->les,
+                k_les_prep<<<grid_for(g.nint, tb(c, g.nint)), tb(c, g.nint), 0, c->stream>>>(g, mt, c->v, c->T, c->W_i, c->les_pw, c->les,
                                                                          c->prim, eg ? 0 : 1);
               })))
     return rc;
   long long ns = slab_count(g) - g.nint;
-  if ((rc = launch(c, "visc_wrap", [&] { k_wrap_periodic<<<grid_for(ns), kThreads, 0, c->stream>>>(g, nderiv, c->fd); })))
+  if ((rc = launch(c, "visc_wrap", [&] { k_wrap_periodic<<<grid_for(ns, tb(c, ns)), tb(c, ns), 0, c->stream>>>(g, nderiv, c->fd); })))
     return rc;
-  if (les && (rc = launch(c, "les_wrap", [&] { k_wrap_periodic<<<grid_for(ns), kThreads, 0, c->stream>>>(g, 4, c->les); })))
+  if (les && (rc = launch(c, "les_wrap", [&] { k_wrap_periodic<<<grid_for(ns, tb(c, ns)), tb(c, ns), 0, c->stream>>>(g, 4, c->les); })))
     return rc;
+  const long long ns_all = slab_count(g);
+  const int tv = tb_or(c, c->tb_visc, ns_all);
   SgsArgs sa{};
   if (les) {
     sa.les = c->les;
@@ -349,33 +365,31 @@ int enq_visc(izem_ctx* c) {
     sa.mu_sgs = c->mu_sgs;
   }
   if (les && eg) {
-    const long long ns_all = slab_count(g);
     if ((rc = launch(c, "visc_point_eg", [&] {
-           k_visc_point_eg<NRV, true><<<grid_for(ns_all, c->tb_visc), c->tb_visc, 0, c->stream>>>(
+           k_visc_point_eg<NRV, true><<<grid_for(ns_all, tv), tv, 0, c->stream>>>(
                g, c->v, c->T, c->W_i, c->ha, c->Xa, c->prim, c->fd, c->tau, c->qv, c->eg_tab, sa);
          })))
       return rc;
   } else if (les) {
     if ((rc = launch(c, "visc_point", [&] {
-           k_visc_point<NRV, true><<<grid_for(slab_count(g), c->tb_visc), c->tb_visc, 0, c->stream>>>(
+           k_visc_point<NRV, true><<<grid_for(ns_all, tv), tv, 0, c->stream>>>(
                g, c->v, c->T, c->W_i, c->ha, c->Xa, c->fd, c->tau, c->qv, sa);
          })))
       return rc;
   } else if (eg) {
-    const long long ns_all = slab_count(g);
     if ((rc = launch(c, "visc_point_eg", [&] {
-           k_visc_point_eg<NRV><<<grid_for(ns_all, c->tb_visc), c->tb_visc, 0, c->stream>>>(g, c->v, c->T, c->W_i, c->ha, c->Xa,
+           k_visc_point_eg<NRV><<<grid_for(ns_all, tv), tv, 0, c->stream>>>(g, c->v, c->T, c->W_i, c->ha, c->Xa,
                                                                                          c->prim, c->fd, c->tau, c->qv,
                                                                                          c->eg_tab);
          })))
       return rc;
   } else if ((rc = launch(c, "visc_point", [&] {
-         k_visc_point<NRV><<<grid_for(slab_count(g), c->tb_visc), c->tb_visc, 0, c->stream>>>(g, c->v, c->T, c->W_i, c->ha, c->Xa, c->fd, c->tau, c->qv);
+         k_visc_point<NRV><<<grid_for(ns_all, tv), tv, 0, c->stream>>>(g, c->v, c->T, c->W_i, c->ha, c->Xa, c->fd, c->tau, c->qv);
        })))
     return rc;
   return launch(c, "visc_div", [&] {
     auto kern = g.ng == 4 ? k_visc_div<NRV, 4> : k_visc_div<NRV, 3>;
-    kern<<<grid_for(g.nint), kThreads, 0, c->stream>>>(g, mt, c->tau, c->qv, c->fd, c->f);
+    kern<<<grid_for(g.nint, tb(c, g.nint)), tb(c, g.nint), 0, c->stream>>>(g, mt, c->tau, c->qv, c->fd, c->f);
   });
 }
 
@@ -391,7 +405,7 @@ int enq_nr(izem_ctx* c) {
     const long long np = (long long)(d == 0 ? g.n[1] : g.n[0]) * (d == 2 ? g.n[1] : g.n[2]);
     rc = launch(c, "bc_nr", [&] {
 #define IZEM_NR(DD, NGV)                                                                                           \
-  k_bc_nr<NRV, DD, NGV><<<grid_for(np), kThreads, 0, c->stream>>>(g, hi, c->v, c->T, c->W_i, c->cp, c->ha, c->dxi[DD], c->f)
+  k_bc_nr<NRV, DD, NGV><<<grid_for(np, tb(c, np)), tb(c, np), 0, c->stream>>>(g, hi, c->v, c->T, c->W_i, c->cp, c->ha, c->dxi[DD], c->f)
       if (g.ng == 4) {
         if (d == 0) IZEM_NR(0, 4);
         if (d == 1) IZEM_NR(1, 4);
@@ -420,7 +434,7 @@ int enq_boundaries(izem_ctx* c, const double* tdt, double tk) {
   long long ns = slab_count(g) - g.nint;
   const bool jet = jet_face(g.bc[0]) || jet_face(g.bc[1]);
   if (!jet) {
-    if ((rc = launch(c, "halo", [&] { k_halo<NRV><<<grid_for(ns), kThreads, 0, c->stream>>>(g, 0, c->cfg.forcesum, c->v, c->W_i); })))
+    if ((rc = launch(c, "halo", [&] { k_halo<NRV><<<grid_for(ns, tb(c, ns)), tb(c, ns), 0, c->stream>>>(g, 0, c->cfg.forcesum, c->v, c->W_i); })))
       return rc;
     return enq_newton<NRV>(c, 1, 1.0e-5, 200, 1);
   }
@@ -437,23 +451,23 @@ int enq_boundaries(izem_ctx* c, const double* tdt, double tk) {
   ja.tdt = tdt;
   ja.tk = tk;
   const long long np = (long long)g.n[1] * g.n[2];
-  if (per && (rc = launch(c, "halo", [&] { k_halo<NRV><<<grid_for(ns), kThreads, 0, c->stream>>>(g, 0, c->cfg.forcesum, c->v, c->W_i, per); })))
+  if (per && (rc = launch(c, "halo", [&] { k_halo<NRV><<<grid_for(ns, tb(c, ns)), tb(c, ns), 0, c->stream>>>(g, 0, c->cfg.forcesum, c->v, c->W_i, per); })))
     return rc;
   if (g.bc[0] == IZEM_BC_INFLOWJET &&
-      (rc = launch(c, "bc_inflowjet", [&] { k_bc_inflowjet<NRV><<<grid_for(np), kThreads, 0, c->stream>>>(g, ja, c->v); })))
+      (rc = launch(c, "bc_inflowjet", [&] { k_bc_inflowjet<NRV><<<grid_for(np, tb(c, np)), tb(c, np), 0, c->stream>>>(g, ja, c->v); })))
     return rc;
   if (g.bc[1] == IZEM_BC_NSCBC_OUT && (rc = launch(c, "bc_nscbc_out", [&] {
-                                         k_bc_nscbc_out<NRV><<<grid_for(np), kThreads, 0, c->stream>>>(g, ja, c->T, c->W_i, c->cp, c->v);
+                                         k_bc_nscbc_out<NRV><<<grid_for(np, tb(c, np)), tb(c, np), 0, c->stream>>>(g, ja, c->T, c->W_i, c->cp, c->v);
                                        })))
     return rc;
   if ((rc = launch(c, "dirichlet_prep", [&] {
-         k_dirichlet_prep<NRV><<<grid_for(2 * np), kThreads, 0, c->stream>>>(g, c->cfg.forcesum, c->v, c->W_i);
+         k_dirichlet_prep<NRV><<<grid_for(2 * np, tb(c, 2 * np)), tb(c, 2 * np), 0, c->stream>>>(g, c->cfg.forcesum, c->v, c->W_i);
        })))
     return rc;
   if ((rc = enq_newton<NRV>(c, 2, 1.0e-5, 200, 1))) return rc;
-  if (ext && (rc = launch(c, "halo", [&] { k_halo<NRV><<<grid_for(ns), kThreads, 0, c->stream>>>(g, 0, c->cfg.forcesum, c->v, c->W_i, ext); })))
+  if (ext && (rc = launch(c, "halo", [&] { k_halo<NRV><<<grid_for(ns, tb(c, ns)), tb(c, ns), 0, c->stream>>>(g, 0, c->cfg.forcesum, c->v, c->W_i, ext); })))
     return rc;
-  if ((rc = launch(c, "halo", [&] { k_halo<NRV><<<grid_for(ns), kThreads, 0, c->stream>>>(g, 2, c->cfg.forcesum, c->v, c->W_i, dir); })))
+  if ((rc = launch(c, "halo", [&] { k_halo<NRV><<<grid_for(ns, tb(c, ns)), tb(c, ns), 0, c->stream>>>(g, 2, c->cfg.forcesum, c->v, c->W_i, dir); })))
     return rc;
   return enq_newton<NRV>(c, 1, 1.0e-5, 200, 1);
 }
@@ -481,10 +495,10 @@ int enq_sensor_prim(izem_ctx* c) {
     Metrics mt;
     for (int d = 0; d < 3; ++d) mt.dxi[d] = c->dxi[d];
     return launch(c, "sensor", [&] {
-      k_sensor_ducros<<<grid_for(g.nint), kThreads, 0, c->stream>>>(g, mt, c->prim, c->ducros_treduc, c->sensor);
+      k_sensor_ducros<<<grid_for(g.nint, tb(c, g.nint)), tb(c, g.nint), 0, c->stream>>>(g, mt, c->prim, c->ducros_treduc, c->sensor);
     });
   }
-  if ((rc = launch(c, "sensor", [&] { k_sensor<<<grid_for(g.nint), kThreads, 0, c->stream>>>(g, c->cfg.max_rel_weight, c->v, c->T, c->W_i, c->sensor, c->sensor_bx); })))
+  if ((rc = launch(c, "sensor", [&] { k_sensor<<<grid_for(g.nint, tb(c, g.nint)), tb(c, g.nint), 0, c->stream>>>(g, c->cfg.max_rel_weight, c->v, c->T, c->W_i, c->sensor, c->sensor_bx); })))
     return rc;
   return enq_prim<NRV>(c);
 }
@@ -500,7 +514,7 @@ int enq_stage(izem_ctx* c, int stage) {
     if ((rc = enq_visc<NRV>(c))) return rc;
   if ((rc = enq_nr<NRV>(c))) return rc;
   if ((rc = launch(c, "rk_update", [&] {
-         k_rk_update<NRV><<<grid_for(g.nint), kThreads, 0, c->stream>>>(g, stage, c->cfg.forcesum, c->d_dt, c->v, c->v0, c->f, c->W_i);
+         k_rk_update<NRV><<<grid_for(g.nint, tb(c, g.nint)), tb(c, g.nint), 0, c->stream>>>(g, stage, c->cfg.forcesum, c->d_dt, c->v, c->v0, c->f, c->W_i);
        })))
     return rc;
   return enq_update_primitives_after<NRV>(c, stage);
@@ -525,11 +539,11 @@ template <int NRV>
 int do_finalize_ic(izem_ctx* c) {
   const Geo& g = c->g;
   int rc;
-  if ((rc = launch(c, "wmix", [&] { k_wmix_interior<NRV><<<grid_for(g.nint), kThreads, 0, c->stream>>>(g, c->v, c->W_i); })))
+  if ((rc = launch(c, "wmix", [&] { k_wmix_interior<NRV><<<grid_for(g.nint, tb(c, g.nint)), tb(c, g.nint), 0, c->stream>>>(g, c->v, c->W_i); })))
     return rc;
   if ((rc = enq_newton<NRV>(c, 0, 1.0e-10, 100, 0))) return rc;
   long long ns = slab_count(g) - g.nint;
-  if ((rc = launch(c, "halo", [&] { k_halo<NRV><<<grid_for(ns), kThreads, 0, c->stream>>>(g, 1, 0, c->v, c->W_i); }))) return rc;
+  if ((rc = launch(c, "halo", [&] { k_halo<NRV><<<grid_for(ns, tb(c, ns)), tb(c, ns), 0, c->stream>>>(g, 1, 0, c->v, c->W_i); }))) return rc;
   return enq_newton<NRV>(c, 1, 1.0e-10, 100, 0);
 }
 
@@ -539,7 +553,7 @@ int do_update_primitives(izem_ctx* c) {
   int rc;
   // upd_prim_var_domain on the current interior state (force_sumY + W_i)
   if ((rc = launch(c, "prep_interior", [&] {
-         k_prep_interior<NRV><<<grid_for(g.nint), kThreads, 0, c->stream>>>(g, c->cfg.forcesum, c->v, c->W_i);
+         k_prep_interior<NRV><<<grid_for(g.nint, tb(c, g.nint)), tb(c, g.nint), 0, c->stream>>>(g, c->cfg.forcesum, c->v, c->W_i);
        })))
     return rc;
   return enq_update_primitives_after<NRV>(c);
@@ -552,7 +566,7 @@ int do_chem_after(izem_ctx* c) {
   const Geo& g = c->g;
   int rc;
   if ((rc = launch(c, "prim_woT", [&] {
-         k_prim_woT<NRV><<<grid_for(g.nint), kThreads, 0, c->stream>>>(g, c->v, c->T, c->W_i, c->cp, c->ha);
+         k_prim_woT<NRV><<<grid_for(g.nint, tb(c, g.nint)), tb(c, g.nint), 0, c->stream>>>(g, c->v, c->T, c->W_i, c->cp, c->ha);
        })))
     return rc;
   return enq_boundaries<NRV>(c, c->d_dt + 4, 0.0);
@@ -564,13 +578,13 @@ int do_timestep(izem_ctx* c) {
   Metrics mt;
   for (int d = 0; d < 3; ++d) mt.dxi[d] = c->dxi[d];
   int rc = launch(c, "timestep", [&] {
-    k_dtc<NRV><<<grid_for(g.nint), kThreads, 0, c->stream>>>(g, mt, c->v, c->T, c->W_i, c->cp, c->d_status);
+    k_dtc<NRV><<<grid_for(g.nint, tb(c, g.nint)), tb(c, g.nint), 0, c->stream>>>(g, mt, c->v, c->T, c->W_i, c->cp, c->d_status);
   });
   if (rc || !(c->cfg.vis && c->cfg.vis_dt)) return rc;
   return launch(c, "timestep_fourier", [&] {
     // with the fitted-transport LES, mu_SGS of the last flux evaluation
     const bool msgs = c->les_on && !c->cfg.eglib && c->mu_sgs;
-    k_dtv<NRV><<<grid_for(g.nint), kThreads, 0, c->stream>>>(g, mt, c->v, c->T, c->W_i, c->cp, c->d_status,
+    k_dtv<NRV><<<grid_for(g.nint, tb(c, g.nint)), tb(c, g.nint), 0, c->stream>>>(g, mt, c->v, c->T, c->W_i, c->cp, c->d_status,
                                                             msgs ? c->mu_sgs : nullptr, c->adi.sc, c->les_sc_sgs,
                                                             c->adi.pr, c->les_pr_sgs_i);
   });
@@ -581,7 +595,7 @@ template <int NRV>
 int do_sensor(izem_ctx* c) {
   if (c->sensor_type == IZEM_SENSOR_DUCROS) return enq_sensor_prim<NRV>(c);
   const Geo& g = c->g;
-  return launch(c, "sensor", [&] { k_sensor<<<grid_for(g.nint), kThreads, 0, c->stream>>>(g, c->cfg.max_rel_weight, c->v, c->T, c->W_i, c->sensor, c->sensor_bx); });
+  return launch(c, "sensor", [&] { k_sensor<<<grid_for(g.nint, tb(c, g.nint)), tb(c, g.nint), 0, c->stream>>>(g, c->cfg.max_rel_weight, c->v, c->T, c->W_i, c->sensor, c->sensor_bx); });
 }
 
 template <int NRV>
