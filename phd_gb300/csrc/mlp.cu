@@ -78,12 +78,11 @@ struct izem_mlp {
   uint8_t *xa = nullptr, *xt = nullptr;          // inputs: cap x 16; transposed 128 x cap
   uint8_t *acta[NL - 1] = {}, *actt[NL - 1] = {};   // hidden activations: cap x 256; 256 x cap
   float* z[NL - 1] = {};                         // hidden pre-activations (FP32, cap x 256)
-  float* out = nullptr;                          // network output (FP32, cap x 16)
   float* gout = nullptr;                         // output gradient (FP32, cap x 16) ...
   uint8_t *goa = nullptr, *got = nullptr;        // ... as K-slabs: cap x 16; 16 x cap
-  float* dzf = nullptr;                          // hidden gradient (FP32, cap x 256) ...
-  uint8_t *dza[2] = {}, *dzt = nullptr;          // ... as K-slabs: cap x 256 (two); 256 x cap
-  float* part = nullptr;                         // split-K partial weight gradients
+  float* dzf[NL - 1] = {};                       // hidden gradients (FP32, cap x 256) ...
+  uint8_t *dza[2] = {}, *dzt[NL - 1] = {};       // ... as K-slabs: cap x 256 (two); 256 x cap
+  float* part = nullptr;                         // split-K partial weight gradients, layer after layer
   int splits = 0, split_chunks = 0;              // K split of the weight-gradient GEMMs
   uint8_t *wt[NL] = {}, *wn[NL] = {};            // BF16 weights as K-slabs: W^T (forward), W (backward)
   double* d_loss = nullptr;
@@ -115,13 +114,21 @@ struct izem_mlp {
 
 namespace {
 
+// rows of layer l's weight-gradient tiles (the 16 inputs are padded to one tile) and one split's partials of all layers
+constexpr int part_rows(int l) { return l == 0 ? 128 : LIN[l]; }
+constexpr int part_floats(int layers) { return layers == 0 ? 0 : part_floats(layers - 1) + part_rows(layers - 1) * LOUT[layers - 1]; }
+constexpr int kPartFloats = part_floats(NL);
+static_assert(NL == mlptt::WG_LAYERS, "layers of the batched weight-gradient launch");
+
 // Training buffers for batches of up to `rows` rows (rounded up to 128).
 cudaError_t mlp_ensure(izem_mlp* m, int rows) {
   rows = (rows + 127) / 128 * 128;
   if (rows <= m->cap) return cudaSuccess;
-  cudaFree(m->xa); cudaFree(m->xt); cudaFree(m->out); cudaFree(m->gout); cudaFree(m->goa); cudaFree(m->got);
-  cudaFree(m->dzf); cudaFree(m->dza[0]); cudaFree(m->dza[1]); cudaFree(m->dzt); cudaFree(m->part);
-  for (int l = 0; l < NL - 1; ++l) { cudaFree(m->acta[l]); cudaFree(m->actt[l]); cudaFree(m->z[l]); }
+  cudaFree(m->xa); cudaFree(m->xt); cudaFree(m->gout); cudaFree(m->goa); cudaFree(m->got);
+  cudaFree(m->dza[0]); cudaFree(m->dza[1]); cudaFree(m->part);
+  for (int l = 0; l < NL - 1; ++l) {
+    cudaFree(m->acta[l]); cudaFree(m->actt[l]); cudaFree(m->z[l]); cudaFree(m->dzf[l]); cudaFree(m->dzt[l]);
+  }
   m->cap = 0;
   const size_t M = rows;
   // the weight-gradient GEMMs split the batch (K = rows, chunks of 64) over
@@ -131,18 +138,36 @@ cudaError_t mlp_ensure(izem_mlp* m, int rows) {
   m->splits = (nchunks + m->split_chunks - 1) / m->split_chunks;
   cudaError_t e;
   if ((e = cudaMalloc(&m->xa, M * 16 * 2)) || (e = cudaMalloc(&m->xt, 128 * M * 2)) ||
-      (e = cudaMemset(m->xt, 0, 128 * M * 2)) || (e = cudaMalloc(&m->out, M * 16 * 4)) ||
+      (e = cudaMemset(m->xt, 0, 128 * M * 2)) ||
       (e = cudaMalloc(&m->gout, M * 16 * 4)) || (e = cudaMalloc(&m->goa, M * 16 * 2)) ||
-      (e = cudaMalloc(&m->got, M * 16 * 2)) || (e = cudaMalloc(&m->dzf, M * H * 4)) ||
+      (e = cudaMalloc(&m->got, M * 16 * 2)) ||
       (e = cudaMalloc(&m->dza[0], M * H * 2)) || (e = cudaMalloc(&m->dza[1], M * H * 2)) ||
-      (e = cudaMalloc(&m->dzt, M * H * 2)) || (e = cudaMalloc(&m->part, (size_t)m->splits * H * H * 4)))
+      (e = cudaMalloc(&m->part, (size_t)m->splits * kPartFloats * 4)))
     return e;
   for (int l = 0; l < NL - 1; ++l)
     if ((e = cudaMalloc(&m->acta[l], M * H * 2)) || (e = cudaMalloc(&m->actt[l], M * H * 2)) ||
-        (e = cudaMalloc(&m->z[l], M * H * 4)))
+        (e = cudaMalloc(&m->z[l], M * H * 4)) || (e = cudaMalloc(&m->dzf[l], M * H * 4)) ||
+        (e = cudaMalloc(&m->dzt[l], M * H * 2)))
       return e;
   m->cap = rows;
   return cudaSuccess;
+}
+
+// A launch of a training step, dependent on the one before it in the stream
+// (after_previous_launch)
+template <class Args>
+cudaError_t step_launch(void (*kern)(Args), dim3 grid, int threads, uint32_t smem, cudaStream_t s, const Args& a) {
+  cudaLaunchAttribute at{};
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cfg.attrs = &at;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kern, a);
 }
 
 template <int NT, int MODE>
@@ -155,15 +180,24 @@ cudaError_t tg_launch(const mlptt::TgArgs& a, int mt, int nt, int splits, cudaSt
       return e;
     attr = true;
   }
-  mlptt::k_tgemm<NT, MODE><<<dim3(mt, nt, splits), mlptt::GT_THREADS, mlptt::tg_smem_bytes(NT), s>>>(a);
-  return cudaGetLastError();
+  return step_launch(mlptt::k_tgemm<NT, MODE>, dim3(mt, nt, splits), mlptt::GT_THREADS, mlptt::tg_smem_bytes(NT), s, a);
 }
 
-// Forward pass of M rows (a multiple of 128) whose inputs are in m->xa:
-// hidden pre-activations and activations of every layer kept for the
-// backward pass, FP32 outputs in m->out.
-cudaError_t mlp_forward(izem_mlp* m, int M) {
+constexpr float kBeta1 = 0.9f, kBeta2 = 0.999f;   // Adam
+constexpr int kTileN = 32;   // columns a tile of the forward and input-gradient GEMMs (k_tgemm)
+
+// CTAs over which the weight gradients split a batch of M rows
+int mlp_splits(const izem_mlp* m, int M) { return (M / mlptt::KCMAX + m->split_chunks - 1) / m->split_chunks; }
+
+// Forward pass of M rows (a multiple of 128), the first `valid` of them x
+// (12 columns) and targets t (10): hidden pre-activations and activations of
+// every layer kept for the backward pass, the loss sum added to m->d_loss, the
+// output gradient in m->gout / m->goa / m->got.
+cudaError_t mlp_forward(izem_mlp* m, const float* x, const float* t, int M, int valid) {
   cudaError_t e;
+  if ((e = step_launch(mlptt::k_tg_pack_input, dim3((M * 16 + 255) / 256), 256, 0, m->s,
+                       mlptt::PackArgs{x, M, valid, m->xa, m->xt})) != cudaSuccess)
+    return e;
   for (int l = 0; l < NL; ++l) {
     mlptt::TgArgs a{};
     a.A = l == 0 ? m->xa : m->acta[l - 1];
@@ -181,10 +215,17 @@ cudaError_t mlp_forward(izem_mlp* m, int M) {
       a.ot = m->actt[l];
       a.oaR = M;
       a.otK = M;
-      e = tg_launch<128, mlptt::TG_FWD_GELU>(a, M / 128, H / 128, 1, m->s);
+      e = tg_launch<kTileN, mlptt::TG_FWD_GELU>(a, M / 128, H / kTileN, 1, m->s);
     } else {
-      a.outf = m->out;
-      e = tg_launch<OUTP, mlptt::TG_FWD_OUT>(a, M / 128, 1, 1, m->s);
+      a.outf = m->gout;
+      a.oa = m->goa;
+      a.ot = m->got;
+      a.oaR = M;
+      a.otK = M;
+      a.target = t;
+      a.M_valid = valid;
+      a.loss = m->d_loss;
+      e = tg_launch<OUTP, mlptt::TG_FWD_LOSS>(a, M / 128, 1, 1, m->s);
     }
     if (e != cudaSuccess) return e;
   }
@@ -192,31 +233,13 @@ cudaError_t mlp_forward(izem_mlp* m, int M) {
 }
 
 // Backward pass of M rows from the output gradient in m->gout / m->goa /
-// m->got to the parameter gradients gW, gb.
+// m->got to the split partials of the weight gradients and the output
+// gradient of every layer.
 cudaError_t mlp_backward(izem_mlp* m, int M) {
   cudaError_t e;
   const uint8_t* gA = m->goa;   // this layer's output gradient as an A operand
   int nxt = 0;
-  for (int l = NL - 1; l >= 0; --l) {
-    // gW_l = act_l^T dZ_l: K = the batch, split over CTAs, partials added in order
-    mlptt::TgArgs w{};
-    w.A = l == 0 ? m->xt : m->actt[l - 1];
-    w.RA = l == 0 ? 128 : H;
-    w.B = l == NL - 1 ? m->got : m->dzt;
-    w.RB = LOUT[l];
-    w.K = M;
-    w.chunks = m->split_chunks;
-    w.N = LOUT[l];
-    w.outf = m->part;
-    w.err = m->d_err;
-    const int splits = (M / mlptt::KCMAX + w.chunks - 1) / w.chunks;
-    if (l == NL - 1) e = tg_launch<OUTP, mlptt::TG_WGRAD>(w, w.RA / 128, 1, splits, m->s);
-    else e = tg_launch<H, mlptt::TG_WGRAD>(w, w.RA / 128, 1, splits, m->s);
-    if (e != cudaSuccess) return e;
-    const int nw = LIN[l] * LOUT[l];
-    mlptt::k_tg_reduce<<<(nw + 255) / 256, 256, 0, m->s>>>(m->part, splits, w.RA, LIN[l], LOUT[l], m->gW[l]);
-    mlptt::k_tg_colsum<<<LOUT[l], 256, 0, m->s>>>(l == NL - 1 ? m->gout : m->dzf, M, LOUT[l], m->gb[l]);
-    if (l == 0) break;
+  for (int l = NL - 1; l > 0; --l) {
     // dZ_{l-1} = (dZ_l W_l^T) gelu'(z_{l-1})
     mlptt::TgArgs d{};
     d.A = gA;
@@ -227,42 +250,68 @@ cudaError_t mlp_backward(izem_mlp* m, int M) {
     d.chunks = LOUT[l] / mlptt::kslab_kc(LOUT[l]);
     d.N = H;
     d.zin = m->z[l - 1];
-    d.outf = m->dzf;
+    d.outf = m->dzf[l - 1];
     d.oa = m->dza[nxt];
-    d.ot = m->dzt;
+    d.ot = m->dzt[l - 1];
     d.oaR = M;
     d.otK = M;
     d.err = m->d_err;
-    if ((e = tg_launch<128, mlptt::TG_BWD_GELU>(d, M / 128, H / 128, 1, m->s)) != cudaSuccess) return e;
+    if ((e = tg_launch<kTileN, mlptt::TG_BWD_GELU>(d, M / 128, H / kTileN, 1, m->s)) != cudaSuccess) return e;
     gA = m->dza[nxt];
     nxt ^= 1;
   }
-  return cudaGetLastError();
-}
-
-// Adam on one parameter array; for weights (lin x lout, wt != nullptr) it
-// also writes the BF16 copies the GEMMs read (row-major, W^T and W K-slabs).
-__global__ void k_adam(float* w, const float* gw, float* mw, float* vw, int n, float lr, float b1, float b2, float eps,
-                       float c1, float c2, int lout, int lin, __nv_bfloat16* wb, uint8_t* wt, uint8_t* wn) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  const float gr = gw[i];
-  const float m = b1 * mw[i] + (1.f - b1) * gr;
-  const float v = b2 * vw[i] + (1.f - b2) * gr * gr;
-  mw[i] = m;
-  vw[i] = v;
-  const float wv = w[i] - lr * (m / c1) / (sqrtf(v / c2) + eps);
-  w[i] = wv;
-  if (wt) {
-    const int r = i / lout, c = i % lout;
-    const __nv_bfloat16 b = __float2bfloat16(wv);
-    wb[i] = b;
-    *reinterpret_cast<__nv_bfloat16*>(wt + mlptt::kslab_off(c, r, lout, lin)) = b;
-    *reinterpret_cast<__nv_bfloat16*>(wn + mlptt::kslab_off(r, c, lin, lout)) = b;
+  // gW_l = act_l^T dZ_l: K = the batch, split over CTAs, partials added in order
+  mlptt::TgLayers b{};
+  const int splits = mlp_splits(m, M);
+  for (int l = 0; l < NL; ++l) {
+    mlptt::TgArgs& w = b.l[l];
+    w.A = l == 0 ? m->xt : m->actt[l - 1];
+    w.RA = part_rows(l);
+    w.B = l == NL - 1 ? m->got : m->dzt[l];
+    w.RB = LOUT[l];
+    w.K = M;
+    w.chunks = m->split_chunks;
+    w.N = LOUT[l];
+    w.outf = m->part + (size_t)splits * part_floats(l);
+    w.err = m->d_err;
+    b.first[l + 1] = b.first[l] + w.RA / 128 * ((LOUT[l] + mlptt::WG_NT - 1) / mlptt::WG_NT);
   }
+  static bool attr = false;
+  if (!attr) {
+    if ((e = cudaFuncSetAttribute(mlptt::k_tg_wgrad, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  (int)mlptt::tg_smem_bytes(mlptt::WG_NT))) != cudaSuccess)
+      return e;
+    attr = true;
+  }
+  return step_launch(mlptt::k_tg_wgrad, dim3(b.first[NL], splits), mlptt::GT_THREADS, mlptt::tg_smem_bytes(mlptt::WG_NT),
+                     m->s, b);
 }
 
-// The BF16 copies of every weight array after W changed outside Adam.
+// The parameter gradients of the backward pass's M rows, applied as one Adam
+// step (adam) or written to gW, gb.
+cudaError_t mlp_update(izem_mlp* m, int M, bool adam, float lr, float c1, float c2) {
+  mlptt::UpdArgs u{};
+  u.splits = mlp_splits(m, M);
+  u.M = M;
+  u.adam = adam;
+  u.lr = lr; u.b1 = kBeta1; u.b2 = kBeta2; u.eps = 1e-8f; u.c1 = c1; u.c2 = c2;
+  int nw = 0;
+  for (int l = 0; l < NL; ++l) {
+    mlptt::UpdLayer& p = u.l[l];
+    p.part = m->part + (size_t)u.splits * part_floats(l);
+    p.dz = l == NL - 1 ? m->gout : m->dzf[l];
+    p.w = m->W[l]; p.mw = m->mW[l]; p.vw = m->vW[l]; p.gw = m->gW[l];
+    p.b = m->b[l]; p.mb = m->mb[l]; p.vb = m->vb[l]; p.gb = m->gb[l];
+    p.wb = m->Wb[l]; p.wt = m->wt[l]; p.wn = m->wn[l];
+    p.rows = part_rows(l); p.lin = LIN[l]; p.lout = LOUT[l];
+    p.first_b = u.nblk_b;
+    u.nblk_b += LOUT[l] / 8;
+    p.first_w = nw;
+    nw += (LIN[l] * LOUT[l] + mlptt::UPD_THREADS - 1) / mlptt::UPD_THREADS;
+  }
+  return step_launch(mlptt::k_tg_update, dim3(u.nblk_b + nw), mlptt::UPD_THREADS, 0, m->s, u);
+}
+
 cudaError_t mlp_weight_copies(izem_mlp* m) {
   for (int l = 0; l < NL; ++l) {
     const int nw = LIN[l] * LOUT[l];
@@ -368,9 +417,11 @@ void izem_mlp_destroy(izem_mlp* m) {
     cudaFree(m->mb[l]); cudaFree(m->vb[l]); cudaFree(m->gW[l]); cudaFree(m->gb[l]);
     cudaFree(m->wt[l]); cudaFree(m->wn[l]);
   }
-  for (int l = 0; l < NL - 1; ++l) { cudaFree(m->acta[l]); cudaFree(m->actt[l]); cudaFree(m->z[l]); }
-  cudaFree(m->xa); cudaFree(m->xt); cudaFree(m->out); cudaFree(m->gout); cudaFree(m->goa); cudaFree(m->got);
-  cudaFree(m->dzf); cudaFree(m->dza[0]); cudaFree(m->dza[1]); cudaFree(m->dzt); cudaFree(m->part);
+  for (int l = 0; l < NL - 1; ++l) {
+    cudaFree(m->acta[l]); cudaFree(m->actt[l]); cudaFree(m->z[l]); cudaFree(m->dzf[l]); cudaFree(m->dzt[l]);
+  }
+  cudaFree(m->xa); cudaFree(m->xt); cudaFree(m->gout); cudaFree(m->goa); cudaFree(m->got);
+  cudaFree(m->dza[0]); cudaFree(m->dza[1]); cudaFree(m->part);
   cudaFree(m->d_loss);
   cudaFree(m->ib[0]); cudaFree(m->ib[1]); cudaFree(m->iout); cudaFree(m->d_norm);
   for (int l = 0; l < NL; ++l) cudaFree(m->blob[l]);
@@ -486,13 +537,10 @@ int izem_mlp_grads(izem_mlp* m, int M, const float* x, const float* t, double* l
       cudaMemcpy(dt, t, (size_t)M * OUT * 4, cudaMemcpyHostToDevice) != cudaSuccess)
     rc = IZEM_ERR_CUDA;
   if (rc == IZEM_OK) {
-    mlptt::k_tg_pack_input<<<(Mp * 16 + 255) / 256, 256, 0, m->s>>>(dx, Mp, M, m->xa, m->xt);
-    if (cudaGetLastError() != cudaSuccess || mlp_forward(m, Mp) != cudaSuccess) rc = IZEM_ERR_CUDA;
-  }
-  if (rc == IZEM_OK) {
-    cudaMemsetAsync(m->d_loss, 0, sizeof(double), m->s);
-    mlptt::k_tg_mse<<<(Mp * 16 + 255) / 256, 256, 0, m->s>>>(m->out, dt, Mp, M, m->gout, m->goa, m->got, m->d_loss);
-    if (cudaGetLastError() != cudaSuccess || mlp_backward(m, Mp) != cudaSuccess) rc = IZEM_ERR_CUDA;
+    if (cudaMemsetAsync(m->d_loss, 0, sizeof(double), m->s) != cudaSuccess ||
+        mlp_forward(m, dx, dt, Mp, M) != cudaSuccess || mlp_backward(m, Mp) != cudaSuccess ||
+        mlp_update(m, Mp, false, 0.f, 1.f, 1.f) != cudaSuccess)
+      rc = IZEM_ERR_CUDA;
   }
   if (rc == IZEM_OK) {
     if (cudaMemcpyAsync(loss, m->d_loss, sizeof(double), cudaMemcpyDeviceToHost, m->s) != cudaSuccess) rc = IZEM_ERR_CUDA;
@@ -546,21 +594,14 @@ int izem_mlp_train(izem_mlp* m, long long n, const float* x, const float* t, int
     cudaMemsetAsync(m->d_loss, 0, sizeof(double), m->s);
     for (long long q = 0; q < nb; ++q) {
       const long long r0 = perm[q] * batch;
-      mlptt::k_tg_pack_input<<<(Mp * 16 + 255) / 256, 256, 0, m->s>>>(dx + r0 * IN, Mp, batch, m->xa, m->xt);
-      if (mlp_forward(m, Mp) != cudaSuccess) { rc = IZEM_ERR_CUDA; break; }
-      mlptt::k_tg_mse<<<(Mp * 16 + 255) / 256, 256, 0, m->s>>>(m->out, dt + r0 * OUT, Mp, batch, m->gout, m->goa,
-                                                                 m->got, m->d_loss);
-      if (mlp_backward(m, Mp) != cudaSuccess) { rc = IZEM_ERR_CUDA; break; }
-      m->step += 1;
-      const float b1 = 0.9f, b2 = 0.999f;
-      const float c1 = 1.f - powf(b1, (float)m->step), c2 = 1.f - powf(b2, (float)m->step);
-      for (int l = 0; l < NL; ++l) {
-        const int nw = LIN[l] * LOUT[l];
-        k_adam<<<(nw + 255) / 256, 256, 0, m->s>>>(m->W[l], m->gW[l], m->mW[l], m->vW[l], nw, lr, b1, b2, 1e-8f, c1, c2,
-                                                   LOUT[l], LIN[l], m->Wb[l], m->wt[l], m->wn[l]);
-        k_adam<<<(LOUT[l] + 255) / 256, 256, 0, m->s>>>(m->b[l], m->gb[l], m->mb[l], m->vb[l], LOUT[l], lr, b1, b2,
-                                                        1e-8f, c1, c2, 0, 0, nullptr, nullptr, nullptr);
+      if (mlp_forward(m, dx + r0 * IN, dt + r0 * OUT, Mp, batch) != cudaSuccess ||
+          mlp_backward(m, Mp) != cudaSuccess) {
+        rc = IZEM_ERR_CUDA;
+        break;
       }
+      m->step += 1;
+      const float c1 = 1.f - powf(kBeta1, (float)m->step), c2 = 1.f - powf(kBeta2, (float)m->step);
+      if (mlp_update(m, Mp, true, lr, c1, c2) != cudaSuccess) { rc = IZEM_ERR_CUDA; break; }
       m->blob_dirty = true;
     }
     if (rc != IZEM_OK) break;
