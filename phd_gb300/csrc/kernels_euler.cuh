@@ -207,6 +207,124 @@ __device__ __forceinline__ double weno_nl(const double* vp, const double* vm) {
   else return weno5_nl(vp, vm);
 }
 
+// The face-constant data of a sensed face, held by the thread that owns it.
+template <int NRV>
+struct FaceState {
+  double uc[3], Yc[NRV], psi[NRV];
+  double un, cs, cs_i, b2, xi, q, ht;
+  double lm0, lm1, lm2;
+  long long p0;   // first stencil point
+};
+
+// Nonlinear reconstruction (wenorec) of the sensed faces of one warp, GL lanes
+// to a face: lane m holds variable m while the characteristic projections are
+// formed (their species products are sums over the lanes), then reconstructs
+// field m, and writes component m of R ghat.  A face a thread
+// instead serialises 2 NG projections and NV reconstructions, some 1900 FP64
+// operations with nine species, for the few lanes that need them while the
+// rest of the warp waits.  The sweeps of the 400 x 11 shock tube (WENO7, two
+// species), all latency, took 98 us in x and in y and take 80 and 43; a sweep
+// of 61 x 50 x 38 with nine species and 1 % of the points flagged 0.61 ms and
+// 0.28.
+template <int NRV, int D, int NG>
+__device__ __forceinline__ void weno_face_lanes(unsigned sensed, const FaceState<NRV>& own, long long own_idx,
+                                                long long nc, long long stride, const double* __restrict__ v,
+                                                const double* __restrict__ prim, double* __restrict__ fhat,
+                                                long long nfaces) {
+  constexpr int NV = IZEM_NIV + NRV;
+  constexpr int GL = NV <= 8 ? 8 : 16, PER = 32 / GL;
+  constexpr int T1 = D == 0 ? 1 : 0;
+  constexpr int T2 = D == 2 ? 1 : 2;
+  static_assert(NV <= 16, "a variable a lane");
+  constexpr unsigned full = 0xffffffffu;
+  const int lane = threadIdx.x & 31, grp = lane / GL, m = lane % GL;
+  while (sensed) {
+    // the faces of this round: group g takes the g-th set bit (the first
+    // again when there are fewer; it does not store then)
+    unsigned rest = sensed;
+    for (int g = 0; g < grp && rest; ++g) rest &= rest - 1;
+    const bool store = rest != 0;
+    const int src = __ffs(store ? rest : sensed) - 1;
+    for (int g = 0; g < PER; ++g) sensed &= sensed - 1;
+    auto from = [&](double x) { return __shfl_sync(full, x, src); };
+    const double uT1 = from(own.uc[T1]), uT2 = from(own.uc[T2]), un = from(own.un);
+    const double u0 = D == 0 ? un : uT1, u1 = D == 1 ? un : (D == 0 ? uT1 : uT2), u2 = D == 2 ? un : uT2;
+    const double cs = from(own.cs), cs_i = from(own.cs_i), b2 = from(own.b2), xi = from(own.xi), q = from(own.q);
+    const double ht = from(own.ht), lm0 = from(own.lm0), lm1 = from(own.lm1), lm2 = from(own.lm2);
+    const long long p0 = __shfl_sync(full, own.p0, src), idx = __shfl_sync(full, own_idx, src);
+    double psi_v = 0.0, psi_r = 0.0, Y_v = 0.0, Y_r = 0.0, psi_n = 0.0;   // of variable m, of field m (species m - 6)
+#pragma unroll
+    for (int l = 0; l < NRV; ++l) {
+      const double ps = from(own.psi[l]), y = from(own.Yc[l]);
+      if (m == IZEM_NIV + l) { psi_v = ps; Y_v = y; }
+      if (m == IZEM_NIV + 1 + l && l < NRV - 1) { psi_r = ps; Y_r = y; }
+      if (l == NRV - 1) psi_n = ps;
+    }
+    // row m of L as coefficients of x_0, x_n, x_t1, x_t2, kappa, psi.x_s and x_{m-1}
+    const double h = 0.5 * cs_i;
+    double k0 = 0.0, kn = 0.0, kt1 = 0.0, kt2 = 0.0, kk = 0.0, ks = 0.0, kx = 0.0;
+    if (m == 0) { k0 = un * h; kn = -h; kk = 0.5 * b2; }
+    else if (m == 1) { k0 = 1.0; kk = -b2; }
+    else if (m == 2) { k0 = -un * h; kn = h; kk = 0.5 * b2; }
+    else if (m == 3) { k0 = -uT1; kt1 = 1.0; }
+    else if (m == 4) { k0 = -uT2; kt2 = 1.0; }
+    else if (m == 5) { kk = 1.0 + xi; ks = -1.0; }
+    else { kk = -Y_r * b2; kx = 1.0; }
+    const double lam = m == 0 ? lm0 : (m == 2 ? lm2 : lm1);
+    auto project = [&](double x) {
+      const double x0 = __shfl_sync(full, x, 0, GL), x1 = __shfl_sync(full, x, 1, GL);
+      const double x2 = __shfl_sync(full, x, 2, GL), x3 = __shfl_sync(full, x, 3, GL);
+      const double x4 = __shfl_sync(full, x, 4, GL), xp = __shfl_up_sync(full, x, 1, GL);
+      double sw = psi_v * x;   // psi_v is 0 outside the species
+#pragma unroll
+      for (int o = GL / 2; o > 0; o >>= 1) sw = sw + __shfl_xor_sync(full, sw, o, GL);
+      const double kappa = fma(q, x0, x4) - (u0 * x1 + u1 * x2 + u2 * x3) + sw;
+      const double xn = D == 0 ? x1 : (D == 1 ? x2 : x3);
+      const double xt1 = T1 == 0 ? x1 : x2, xt2 = T2 == 1 ? x2 : x3;
+      double r = fma(kk, kappa, ks * sw);
+      r = fma(k0, x0, r);
+      r = fma(kn, xn, r);
+      r = fma(kt1, xt1, r);
+      r = fma(kt2, xt2, r);
+      return fma(kx, xp, r);
+    };
+    double gpl[2 * NG], gmi[2 * NG];
+#pragma unroll
+    for (int st = 0; st < 2 * NG; ++st) {
+      const long long ps = p0 + st * stride;
+      const double w = m < NV ? v[m * nc + ps] : 0.0;
+      const double u_s = prim[(PR_U + D) * nc + ps], P_s = prim[PR_P * nc + ps];
+      const double wn = __shfl_sync(full, w, 1 + D, GL);
+      double f = u_s * w;
+      if (m == 0) f = wn;
+      if (m == 1 + D) f = f + P_s;
+      if (m == 4) f = u_s * (w + P_s);
+      const double pw = project(w), pf = project(f);
+      gpl[st] = 0.5 * (pf + lam * pw);
+      gmi[st] = pf - gpl[st];
+    }
+    const double gh = weno_nl<NG>(gpl, gmi);
+    // component m of R ghat (module_weno.f90:881-989)
+    const double g0 = __shfl_sync(full, gh, 0, GL), g1 = __shfl_sync(full, gh, 1, GL);
+    const double g2 = __shfl_sync(full, gh, 2, GL), g3 = __shfl_sync(full, gh, 3, GL);
+    const double g4 = __shfl_sync(full, gh, 4, GL), g5 = __shfl_sync(full, gh, 5, GL);
+    const double gd = __shfl_down_sync(full, gh, 1, GL);
+    double sg = psi_r * gh;   // sum_s psi_s ghat_{6+s}
+#pragma unroll
+    for (int o = GL / 2; o > 0; o >>= 1) sg = sg + __shfl_xor_sync(full, sg, o, GL);
+    const double s3 = g0 + g1 + g2, s2 = g0 + g2;
+    double fh;
+    if (m == 0) fh = s3;
+    else if (m == 1 + D) fh = un * s3 + cs * (g2 - g0);
+    else if (m == 1 + T1) fh = uT1 * s3 + g3;
+    else if (m == 1 + T2) fh = uT2 * s3 + g4;
+    else if (m == 4) fh = ht * s2 + un * cs * (g2 - g0) + q * g1 + uT1 * g3 + uT2 * g4 + g5;
+    else if (m < NV - 1) fh = Y_v * s2 + gd;
+    else fh = Y_v * s2 - fm_div(g5 + sg, psi_n);
+    if (store && m < NV) fhat[m * nfaces + idx] = fh;
+  }
+}
+
 // K2: one thread per cell face along axis D.  Linear (sensor-off) faces take
 // the reconstruction of wenorec_nw without forming the characteristic
 // variables.  The LLF speeds of a face are one number per field and L, R and
@@ -226,7 +344,9 @@ __device__ __forceinline__ double weno_nl(const double* vp, const double* vm) {
 // 18.1 -> 7.5 ms a sweep of 256 x 256 x 128; 0.300 -> 0.144 ms a sweep of 64^3
 // with two.  The result equals the reference's dense nv x nv products up to
 // rounding (relative error against dense 64-bit products 7.6e-15 -> 6.2e-15).
-// Sensed faces keep the 2NG projected values for the nonlinear weights.
+// Sensed faces keep the 2NG projected values for the nonlinear weights: a warp
+// with few of them takes them together (weno_face_lanes), one with many a face
+// a thread.
 // NG = 3 is WENO5, NG = 4 WENO7 (module_weno.f90, ng branches).
 //
 // Sensor blocks (x sweep only): with bx < n[0] the x direction is read as
@@ -247,7 +367,9 @@ __global__ void __launch_bounds__(256) k_euler_face(Geo g, int weno_avg, int lin
   constexpr int T1 = D == 0 ? 1 : 0;
   constexpr int T2 = D == 2 ? 1 : 2;
   long long idx = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  if (idx >= nfaces) return;
+  // lanes past the end repeat the last face: sensed faces are a warp's work
+  const bool valid = idx < nfaces;
+  if (!valid) idx = nfaces - 1;
   int c[3];
   if (D == 0 && edge) {
     const int ne = g.n[0] / bx - 1;
@@ -338,7 +460,13 @@ __global__ void __launch_bounds__(256) k_euler_face(Geo g, int weno_avg, int lin
     shk = shk || (counts && sensor[ps] != 0);
   }
   const double lm0 = __longlong_as_double(m0), lm1 = __longlong_as_double(m1), lm2 = __longlong_as_double(m2);
-  shk = shk && (weno_avg != 0);
+  shk = shk && (weno_avg != 0) && valid;
+  // about where the two forms meet: 300 FP64 operations a round of 2 (4 with
+  // two species) faces against some 1900 (800) for the whole warp.  The sweeps
+  // of 61 x 50 x 38 with 1 % of the points flagged take 1.17 ms with a line of
+  // 6, 1.09 of 12 and 1.13 with lanes always.
+  constexpr int kLanesMost = 12;
+  const unsigned sensed = __ballot_sync(0xffffffffu, shk);
 
   double fh[NV];
   if (!shk) {
@@ -412,7 +540,7 @@ __global__ void __launch_bounds__(256) k_euler_face(Geo g, int weno_avg, int lin
     for (int l = 0; l < NRV; ++l)
       fh[IZEM_NIV + l] = fma(Yc[l], S, fh[IZEM_NIV + l]);
     fh[NV - 1] = fma(delta, fma(lm1, kW, kF), fh[NV - 1]);
-  } else {
+  } else if (__popc(sensed) > kLanesMost) {
     // nonlinear reconstruction (wenorec): keep the 2NG stencil values of every
     // field.  The three acoustic/entropy rows of L are dense over (rho, m, rho
     // e_t) plus a rank-one species term psi.w, the shear rows have two
@@ -486,8 +614,21 @@ __global__ void __launch_bounds__(256) k_euler_face(Geo g, int weno_avg, int lin
     for (int s = 0; s < NRV - 1; ++s) acc = acc + (wrk * psi[s]) * gh[6 + s];
     fh[NV - 1] = acc;
   }
+  if (valid && (!shk || __popc(sensed) > kLanesMost)) {
 #pragma unroll
-  for (int m = 0; m < NV; ++m) fhat[m * nfaces + idx] = fh[m];
+    for (int m = 0; m < NV; ++m) fhat[m * nfaces + idx] = fh[m];
+  }
+  if (sensed && __popc(sensed) <= kLanesMost) {
+    FaceState<NRV> own;
+#pragma unroll
+    for (int d = 0; d < 3; ++d) own.uc[d] = uc[d];
+#pragma unroll
+    for (int l = 0; l < NRV; ++l) { own.Yc[l] = Yc[l]; own.psi[l] = psi[l]; }
+    own.un = un; own.cs = cs_c; own.cs_i = cs_c_i; own.b2 = b2; own.xi = xi; own.q = q; own.ht = ht_c;
+    own.lm0 = lm0; own.lm1 = lm1; own.lm2 = lm2;
+    own.p0 = p0;
+    weno_face_lanes<NRV, D, NG>(sensed, own, idx, nc, stride, v, prim, fhat, nfaces);
+  }
 }
 
 // fl(i) = (fhat(i) - fhat(i-1)) * dx_i(i); the x sweep overwrites, y and z
