@@ -65,11 +65,14 @@ static __constant__ DevThd c_thd;
 constexpr int kNewtonXBlocksMax = 8;
 constexpr int kNewtonSlots = 10 * kNewtonXBlocksMax;
 
+// Shared state of one Newton solve (k_newton_solve); all zero between solves.
+struct NewtonShared {
+  unsigned long long max[3][kNewtonSlots];   // per slot max dT^2 (bit pattern of a non-negative double), iteration mod 3
+  unsigned arrived, left;                    // blocks at the iterations' barriers, blocks through
+};
+
 struct DevStatus {
-  // per slot max dT^2 (bit pattern of a non-negative double), iterations, stop flag
-  unsigned long long maxdf_bits[kNewtonSlots];
-  int it[kNewtonSlots];
-  int done[kNewtonSlots];
+  NewtonShared newton;
   int neg_pressure;
   int neg_temperature;
   int newton_nan;

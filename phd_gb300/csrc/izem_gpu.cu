@@ -26,7 +26,6 @@
 namespace {
 
 constexpr int kThreads = 128;
-constexpr int kNewtonChunk = 4;    // direct-launch Newton: iterations between two host reads of the stop flags
 
 unsigned grid_for(long long n, int threads) { return (unsigned)((n + threads - 1) / threads); }
 
@@ -195,77 +194,30 @@ void drop_graphs(izem_ctx* c) {
 // prim_inv_var's Newton loop (module_thermodynamics.f90:79-186) on one kind
 // of sub-domain; every sub-domain stops on its own test, after at most itmax
 // iterations.  ghost: 0 the interior (sub-domain 0), 1 the ghost slabs (1-6),
-// 2 the Dirichlet planes of jet faces (7-8).
-//
-// Captured into a graph, the loop is a conditional WHILE node whose body is
-// one iteration and the stopping test; the test launch clears the condition
-// when every sub-domain has stopped, so the graph runs exactly the
-// iterations the reference runs.  Launched directly (kernel timing), the
-// host runs the iterations in chunks and reads the stop flags between them;
-// iterations after a sub-domain has stopped leave it untouched, so both
-// forms give the same bits.
+// 2 the Dirichlet planes of jet faces (7-8).  One cooperative launch of as many
+// blocks as the points need or the GPU holds at once; the same inside a
+// captured graph and launched directly.
 template <int NRV>
 int enq_newton(izem_ctx* c, int ghost, double eps, int itmax, int check_negT) {
   const Geo& g = c->g;
   const int d0 = ghost == 2 ? 7 : (ghost ? 1 : 0), d1 = ghost == 2 ? 8 : (ghost ? 6 : 0);
   const long long n = ghost == 2 ? 2LL * g.n[1] * g.n[2] : (ghost ? slab_count(g) - g.nint : g.nint);
-  const char* iname = ghost == 2 ? "newton_iter_plane" : (ghost ? "newton_iter_ghost" : "newton_iter");
-  int rc;
-  const int nxb = g.n[0] / c->newton_bx, bx = c->newton_bx;
-  if ((rc = launch(c, "newton_reset", [&] { k_newton_reset<<<1, 16 * kNewtonXBlocksMax, 0, c->stream>>>(c->d_status, d0, d1, nxb); })))
-    return rc;
-  auto iterate = [&](cudaGraphConditionalHandle cond, int use_cond) -> int {
-    int r = launch(c, iname, [&] {
-      k_newton_iter<NRV><<<grid_for(n, tb(c, n)), tb(c, n), 0, c->stream>>>(g, ghost, c->v, c->T, c->cp, c->ha, c->d_status,
-                                                                            check_negT, bx);
-    });
-    if (r) return r;
-    return launch(c, "newton_check", [&] {
-      k_newton_check<<<1, 32, 0, c->stream>>>(c->d_status, d0, d1, nxb, eps, itmax, cond, use_cond);
-    });
-  };
-  if (c->capturing) {
-    cudaStreamCaptureStatus cs;
-    cudaGraph_t graph = nullptr;
-    const cudaGraphNode_t* deps = nullptr;
-    size_t ndeps = 0;
-    CK(cudaStreamGetCaptureInfo(c->stream, &cs, nullptr, &graph, &deps, nullptr, &ndeps));
-    cudaGraphConditionalHandle cond;
-    // the condition is 1 at every launch of the graph: the loop body runs at
-    // least once, as the reference's first iteration always does
-    CK(cudaGraphConditionalHandleCreate(&cond, graph, 1, cudaGraphCondAssignDefault));
-    cudaGraphNodeParams np{};
-    np.type = cudaGraphNodeTypeConditional;
-    np.conditional.handle = cond;
-    np.conditional.type = cudaGraphCondTypeWhile;
-    np.conditional.size = 1;
-    cudaGraphNode_t node;
-    CK(cudaGraphAddNode(&node, graph, deps, nullptr, ndeps, &np));
-    CK(cudaStreamUpdateCaptureDependencies(c->stream, &node, nullptr, 1, cudaStreamSetCaptureDependencies));
-    cudaStream_t main = c->stream;
-    cudaError_t e = cudaStreamBeginCaptureToGraph(c->side, np.conditional.phGraph_out[0], nullptr, nullptr, 0,
-                                                  cudaStreamCaptureModeThreadLocal);
-    if (e != cudaSuccess) return ctx_fail(c, IZEM_ERR_CUDA, "cudaStreamBeginCaptureToGraph", e);
-    c->stream = c->side;   // the body's launches go to the side stream
-    rc = iterate(cond, 1);
-    c->stream = main;
-    cudaGraph_t body = nullptr;
-    e = cudaStreamEndCapture(c->side, &body);
-    if (rc) return rc;
-    if (e != cudaSuccess) return ctx_fail(c, IZEM_ERR_CUDA, "cudaStreamEndCapture (Newton loop body)", e);
-    return IZEM_OK;
-  }
-  for (int it = 0; it < itmax; it += kNewtonChunk) {
-    for (int q = 0; q < kNewtonChunk && it + q < itmax; ++q)
-      if ((rc = iterate(0, 0))) return rc;
-    CK(cudaMemcpyAsync(c->h_done, c->d_status->done, kNewtonSlots * sizeof(int), cudaMemcpyDeviceToHost, c->stream));
-    CK(cudaStreamSynchronize(c->stream));
-    bool all = true;
-    for (int b = 0; b < nxb; ++b)
-      for (int d = d0; d <= d1; ++d) all = all && c->h_done[d + 10 * b] != 0;
-    if (all) break;
-  }
-  return IZEM_OK;
+  const int nxb = g.n[0] / c->newton_bx, threads = tb(c, n);
+  int per_sm = 0;
+  CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_newton_solve<NRV>, threads, 0));
+  cudaLaunchAttribute at{};
+  at.id = cudaLaunchAttributeCooperative;
+  at.val.cooperative = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3((unsigned)std::min<long long>((long long)per_sm * c->nsm, grid_for(n, threads)));
+  cfg.blockDim = dim3(threads);
+  cfg.stream = c->stream;
+  cfg.attrs = &at;
+  cfg.numAttrs = 1;
+  return launch(c, ghost == 2 ? "newton_plane" : (ghost ? "newton_ghost" : "newton"), [&] {
+    cudaLaunchKernelEx(&cfg, k_newton_solve<NRV>, g, ghost, n, (const double*)c->v, c->T, c->cp, c->ha, c->d_status,
+                       check_negT, c->newton_bx, d0, d1, nxb, eps, itmax);
+  });
 }
 
 template <int NRV>
@@ -806,13 +758,11 @@ int ctx_alloc(izem_ctx* c) {
   const Geo& g = c->g;
   const int nv = c->nv, nrv = c->cfg.nrv;
   CK(cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking));
-  CK(cudaStreamCreateWithFlags(&c->side, cudaStreamNonBlocking));
   {
     int dev = 0;
     CK(cudaGetDevice(&dev));
     CK(cudaDeviceGetAttribute(&c->nsm, cudaDevAttrMultiProcessorCount, dev));
   }
-  CK(cudaMallocHost(&c->h_done, kNewtonSlots * sizeof(int)));
   CK(cudaMemcpyToSymbol(c_thd, &c->devthd, sizeof(DevThd)));
   auto alloc = [&](double** p, size_t n) -> cudaError_t {
     cudaError_t e = cudaMalloc(p, n * sizeof(double));
@@ -875,8 +825,6 @@ void izem_gpu_destroy(izem_ctx* c) {
     for (auto& pr : v) { cudaEventDestroy(pr.first); cudaEventDestroy(pr.second); }
   if (c->t0) cudaEventDestroy(c->t0);
   if (c->t1) cudaEventDestroy(c->t1);
-  if (c->h_done) cudaFreeHost(c->h_done);
-  if (c->side) cudaStreamDestroy(c->side);
   if (c->stream) cudaStreamDestroy(c->stream);
   delete c;
 }

@@ -219,10 +219,10 @@ struct FaceState {
 // Nonlinear reconstruction (wenorec) of the sensed faces of one warp, GL lanes
 // to a face: lane m holds variable m while the characteristic projections are
 // formed (their species products are sums over the lanes), then reconstructs
-// field m, and writes component m of R ghat.  A face a thread
-// instead serialises 2 NG projections and NV reconstructions, some 1900 FP64
-// operations with nine species, for the few lanes that need them while the
-// rest of the warp waits.  The sweeps of the 400 x 11 shock tube (WENO7, two
+// field m, and writes component m of R ghat.  A face a thread instead
+// serialises 2 NG projections and NV reconstructions, some 1900 FP64 operations
+// with nine species, for the few lanes that need them while the rest of the
+// warp waits.  The sweeps of the 400 x 11 shock tube (WENO7, two
 // species), all latency, took 98 us in x and in y and take 80 and 43; a sweep
 // of 61 x 50 x 38 with nine species and 1 % of the points flagged 0.61 ms and
 // 0.28.

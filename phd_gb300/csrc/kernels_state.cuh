@@ -35,7 +35,7 @@ __device__ __forceinline__ void force_sumY_cell(double* v, long long nc, long lo
 // file are bound by the FP64 pipe, not by memory, and the quotients were most
 // of their operations: k_rk_update 236 -> 56 FP64 instructions a point with
 // nine species (3.08 -> 1.18 ms on 256 x 256 x 128), k_prim_woT 370 -> 108 (5.31
-// -> 1.55 ms), k_newton_iter 267 -> 140 (2.44 -> 1.00 ms).
+// -> 1.55 ms), a Newton iteration 267 -> 140 (2.44 -> 1.00 ms).
 template <int NRV>
 __device__ __forceinline__ double wmix_cell(const double* v, long long nc, long long p) {
   double w = 0.0;
@@ -160,19 +160,18 @@ __global__ void k_halo(Geo g, int mode, int forcesum, double* __restrict__ v, do
   W_i[p] = wmix_cell<NRV>(v, nc, p);
 }
 
-// One Newton iteration (newton + the T update of prim_inv_var) on the
-// interior (ghost = 0) or on all six ghost slabs (ghost = 1); each
-// sub-domain stops on its own maximum correction.
+// One Newton iteration (newton + the T update of prim_inv_var) of point idx of
+// the interior (ghost = 0), the six ghost slabs (1) or the Dirichlet planes of
+// jet faces (2), unless its sub-domain has stopped.
 template <int NRV>
-__global__ void k_newton_iter(Geo g, int ghost, const double* __restrict__ v, double* __restrict__ T,
-                              double* __restrict__ cp, double* __restrict__ ha, DevStatus* st, int check_negT,
-                              int bx) {
-  long long idx = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+__device__ __forceinline__ void newton_point(const Geo& g, int ghost, long long idx, const double* __restrict__ v,
+                                             double* __restrict__ T, double* __restrict__ cp, double* __restrict__ ha,
+                                             DevStatus* st, int check_negT, int bx, const int* done,
+                                             unsigned long long* maxdf) {
   int i, j, k, dom;
   if (ghost == 2) {
     // the Dirichlet planes i = 1 (sub-domain 7) and i = nx (8) of jet faces
     const long long np = (long long)g.n[1] * g.n[2];
-    if (idx >= 2 * np) return;
     const int face = (int)(idx / np);
     if (g.bc[face] != IZEM_BC_INFLOWJET && g.bc[face] != IZEM_BC_NSCBC_OUT) return;
     const long long r = idx - face * np;
@@ -181,11 +180,8 @@ __global__ void k_newton_iter(Geo g, int ghost, const double* __restrict__ v, do
     k = (int)(r / g.n[1]) + 1;
     dom = 7 + face;
   } else if (ghost) {
-    const long long ntot = slab_count(g) - g.nint;
-    if (idx >= ntot) return;
     if (!slab_point(g, idx + g.nint, i, j, k, dom)) return;
   } else {
-    if (idx >= g.nint) return;
     i = (int)(idx % g.n[0]) + 1;
     long long r = idx / g.n[0];
     j = (int)(r % g.n[1]) + 1;
@@ -195,7 +191,7 @@ __global__ void k_newton_iter(Geo g, int ghost, const double* __restrict__ v, do
   // the interior and the y / z ghost slabs span x: with an emulated
   // x-decomposition (bx < nx) each x-block of them stops on its own test
   if (bx < g.n[0] && (dom == 0 || (dom >= 3 && dom <= 6))) dom += 10 * ((i - 1) / bx);
-  if (st->done[dom]) return;
+  if (done[dom]) return;
   const long long nc = g.ncell;
   const long long p = gid(g, i, j, k);
   // F = e(T) - e of the conserved state, with the sums over rho Y_k
@@ -225,46 +221,90 @@ __global__ void k_newton_iter(Geo g, int ghost, const double* __restrict__ v, do
   if (nan) atomicExch(&st->newton_nan, 1);
   // the sub-domain's largest correction, combined over the warp's lanes of
   // the same sub-domain (a NaN counts as 0 here; the flag records it)
-  atomic_max_nonneg_warp(&st->maxdf_bits[dom], nan ? 0.0 : df2);
+  atomic_max_nonneg_warp(&maxdf[dom], nan ? 0.0 : df2);
 }
 
-// Stopping test of prim_inv_var (module_thermodynamics.f90:110-115,161-162)
-// for sub-domains [d0, d1]: a sub-domain stops when its largest correction
-// is below eps, or after itmax iterations with a convergence warning, as the
-// reference's `it > itmax` exit.  Inside a captured graph (use_cond) the
-// launch also sets the condition of the enclosing WHILE node: the loop runs
-// while any sub-domain is still iterating.  Every iteration moves each live
-// sub-domain one step closer to itmax, so the loop ends after at most itmax
-// passes.
-__global__ void k_newton_check(DevStatus* st, int d0, int d1, int nxb, double eps, int itmax,
-                               cudaGraphConditionalHandle cond, int use_cond) {
-  if (threadIdx.x != 0 || blockIdx.x != 0) return;
-  unsigned live = 0;
-  for (int b = 0; b < nxb; ++b)
-    for (int d = d0 + 10 * b; d <= d1 + 10 * b; ++d) {
-      if (st->done[d]) continue;
-      st->it[d] += 1;
-      const double err = sqrt(__longlong_as_double((long long)st->maxdf_bits[d]));
-      st->maxdf_bits[d] = 0ULL;
-      if (err < eps) st->done[d] = 1;
-      else if (st->it[d] >= itmax) { st->done[d] = 1; st->newton_unconverged += 1; }
-      if (st->done[d]) st->newton_it_max = max(st->newton_it_max, st->it[d]);
-      else live = 1;
-    }
-  if (use_cond) cudaGraphSetConditional(cond, live);
-}
-
-// Slots of sub-domains [d0, d1] of every x-block start iterating; the slots
-// of x-blocks b > 0 of a sub-domain that does not span x receive no points
-// and stop on their first test.
-__global__ void k_newton_reset(DevStatus* st, int d0, int d1, int nxb) {
-  const int b = threadIdx.x / 16, d = d0 + threadIdx.x % 16;
-  if (b < nxb && d <= d1) {
-    const int q = d + 10 * b;
-    st->done[q] = 0;
-    st->it[q] = 0;
-    st->maxdf_bits[q] = 0ULL;
+// Barrier of a cooperative launch: thread 0 waits, a bounded number of polls,
+// until `target` blocks have arrived.  Returns false when it gave up.
+__device__ inline bool grid_barrier(unsigned* arrived, unsigned target) {
+  __shared__ int through;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    __threadfence();
+    atomicAdd(arrived, 1u);
+    int polls = 1 << 26;
+    while (*(volatile unsigned*)arrived < target && --polls) {}
+    __threadfence();
+    through = polls != 0;
   }
+  __syncthreads();
+  return through;
+}
+
+// A whole Newton solve (prim_inv_var, module_thermodynamics.f90:79-186; its test
+// :110-115, 161-162), at most itmax iterations, as one cooperative launch:
+// between two iterations the blocks meet at a barrier and each makes the
+// stopping test for itself, so every point takes exactly the iterations that
+// the reference gives its sub-domain (d0 .. d1 of each of nxb x-blocks, each
+// stopping when its largest correction is below eps, or after itmax iterations
+// with a convergence warning).  Slots of x-blocks of a sub-domain that does
+// not span x receive no points and stop on their first test.
+// Four iterations are the rule, of 1.0 ms each at 256 x 256 x 128 and of a few
+// microseconds on small blocks, where the launches of a loop of an iteration
+// and a test were most of the time: a step of the 400 x 11 shock tube took
+// 0.96 ms so and takes 0.85, of 64^3 2.94 and 2.83, of 256 x 256 x 128 the same.
+template <int NRV>
+__global__ void __launch_bounds__(128) k_newton_solve(Geo g, int ghost, long long n, const double* __restrict__ v,
+                                                      double* __restrict__ T, double* __restrict__ cp,
+                                                      double* __restrict__ ha, DevStatus* st, int check_negT, int bx,
+                                                      int d0, int d1, int nxb, double eps, int itmax) {
+  __shared__ int done[kNewtonSlots], last;
+  NewtonShared& sh = st->newton;
+  for (int q = threadIdx.x; q < kNewtonSlots; q += blockDim.x) done[q] = 0;
+  __syncthreads();
+  const int nd = d1 - d0 + 1, nslots = nd * nxb;
+  const long long step = (long long)gridDim.x * blockDim.x;
+  int live = 1;
+  for (int it = 1; live; ++it) {
+    unsigned long long* mx = sh.max[it % 3];
+    for (long long idx = blockIdx.x * (long long)blockDim.x + threadIdx.x; idx < n; idx += step)
+      newton_point<NRV>(g, ghost, idx, v, T, cp, ha, st, check_negT, bx, done, mx);
+    if (!grid_barrier(&sh.arrived, (unsigned)it * gridDim.x)) {
+      if (threadIdx.x == 0) atomicExch(&st->timeout, 1);
+      break;
+    }
+    int l = 0;
+    for (int q = threadIdx.x; q < nslots; q += blockDim.x) {
+      const int d = d0 + q % nd + 10 * (q / nd);
+      if (!done[d]) {
+        const double err = sqrt(__longlong_as_double((long long)__ldcg(mx + d)));
+        const bool ok = err < eps;
+        if (ok || it >= itmax) {
+          done[d] = 1;
+          if (blockIdx.x == 0) {
+            if (!ok) atomicAdd(&st->newton_unconverged, 1);
+            atomicMax(&st->newton_it_max, it);
+          }
+        } else {
+          l = 1;
+        }
+      }
+      // read by every block before it came to this barrier, used again after the next
+      if (blockIdx.x == 0) sh.max[(it + 2) % 3][d] = 0ULL;
+    }
+    live = __syncthreads_or(l);
+  }
+  // the last block out clears the shared state for the next solve
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    __threadfence();
+    last = atomicInc(&sh.left, gridDim.x - 1) == gridDim.x - 1;
+    __threadfence();
+  }
+  __syncthreads();
+  if (!last) return;
+  for (int q = threadIdx.x; q < 3 * kNewtonSlots; q += blockDim.x) sh.max[q / kNewtonSlots][q % kNewtonSlots] = 0ULL;
+  if (threadIdx.x == 0) sh.arrived = 0;
 }
 
 // Convective time-step criterion: max over the interior of (|u_d|+c) dx_i.
