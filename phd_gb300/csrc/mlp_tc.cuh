@@ -150,8 +150,8 @@ __device__ __forceinline__ void tmem_wait_ld() { asm volatile("tcgen05.wait::ld.
 
 struct TcArgs {
   const __nv_bfloat16* x;          // M x 16 input features (BF16, normalised)
-  float* out;                      // M x 16 network output (FP32)
-  int M;
+  float* out;                      // M x ldo network output (FP32): 16 columns, or the 10 real ones
+  int M, ldo;
   const __nv_bfloat16* blob[5];    // B_l = W_l^T (N x K) in core-matrix layout
   const float* bias[5];
   int* err;                        // set to 1 when a wait gave up
@@ -304,12 +304,13 @@ __global__ void __launch_bounds__(THREADS, 1) k_mlp_tc(TcArgs a) {
       tmem_wait_ld();
       const int gr = row0 + warp * 32 + lane;
       if (gr < a.M) {
-        float4* dst = reinterpret_cast<float4*>(a.out + (size_t)gr * NOUT);
+        // ldo is even: rows of 16 (all columns) or of 10 (the real ones)
+        float2* dst = reinterpret_cast<float2*>(a.out + (size_t)gr * a.ldo);
 #pragma unroll
-        for (int q = 0; q < 4; ++q)
-          dst[q] = make_float4(__uint_as_float(v[4 * q]) + a.bias[4][4 * q], __uint_as_float(v[4 * q + 1]) + a.bias[4][4 * q + 1],
-                               __uint_as_float(v[4 * q + 2]) + a.bias[4][4 * q + 2],
-                               __uint_as_float(v[4 * q + 3]) + a.bias[4][4 * q + 3]);
+        for (int q = 0; q < NOUT / 2; ++q)
+          if (2 * q < a.ldo)
+            dst[q] = make_float2(__uint_as_float(v[2 * q]) + a.bias[4][2 * q],
+                                 __uint_as_float(v[2 * q + 1]) + a.bias[4][2 * q + 1]);
       }
     }
     tc_before_sync();

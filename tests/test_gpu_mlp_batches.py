@@ -43,3 +43,19 @@ def test_gradients_and_adam_steps(M):
             v[k] = float(b2) * v[k] + (1.0 - float(b2)) * g * g
             ref = P[k] - lr * (m[k] / c1) / (np.sqrt(v[k] / c2) + eps)
             assert np.all(np.abs(new - ref) <= 2.0 ** -23 * np.abs(ref) + (16 * 2.0 ** -24 + 6e-5) * 2.0 * lr)
+
+
+# rows around one tile of 128, several tiles and a ragged end, more tiles than SMs
+@pytest.mark.parametrize("M", [1, 127, 129, 1000, 152 * 128 + 37])
+def test_forward_rows(M):
+    rng = np.random.Generator(np.random.PCG64(100 + M))
+    x = rng.standard_normal((M, 12)).astype(np.float32)
+    s = Surrogate(seed=22)
+    W, b = s.get_params()
+    b = [rng.standard_normal(a.shape).astype(np.float32) * 0.1 for a in b]
+    s.set_params(W, b)
+    y = s.forward(x)
+    assert y.shape == (M, 10)
+    ref, _ = mo.forward(W, b, x)
+    # BF16 operands on both sides: 1e-2 of the largest output, as in test_gpu_mlp.py
+    assert np.abs(y - ref).max() <= 1e-2 * np.abs(ref).max()
