@@ -41,6 +41,18 @@ int tb(const izem_ctx* c, long long n) {
   const long long warps = (n + 31) / 32;
   return warps >= 32LL * c->nsm ? kThreads : (warps >= 8LL * c->nsm ? 64 : 32);
 }
+
+// log2 of the lanes to a face in the flux kernel: with four, a warp holds eight
+// faces, and a grid of up to a warp an SM reaches four times the warps, which
+// share the rounds of the sensed faces.  Every face costs a lane's work four
+// times then, in lanes and SMs that had none: two or four lanes as long as that
+// leaves no SM more than four warps.  The x sweep of the 400 x 11 shock tube
+// (138 warps) 80 -> 64 us; two lanes (276 warps) gave nothing there, eight no
+// more than four.
+int face_share(const izem_ctx* c, long long faces) {
+  const long long warps = (faces + 31) / 32;
+  return 4 * warps <= 4LL * c->nsm ? 2 : (2 * warps <= 4LL * c->nsm ? 1 : 0);
+}
 int tb_or(const izem_ctx* c, int tuned, long long n) { return tuned ? tuned : tb(c, n); }
 
 }  // namespace
@@ -237,9 +249,10 @@ int enq_euler(izem_ctx* c, int d) {
   long long nf = (long long)(g.n[0] + (d == 0)) * (g.n[1] + (d == 1)) * (g.n[2] + (d == 2));
   int rc;
   const char* names[3] = {"euler_face_x", "euler_face_y", "euler_face_z"};
-#define IZEM_FACE(DD, NGV)                                                                                         \
-  k_euler_face<NRV, DD, NGV><<<grid_for(nf, tb_or(c, c->tb_euler, nf)), tb_or(c, c->tb_euler, nf), 0, c->stream>>>(                                \
-      g, c->cfg.weno_avg, c->cfg.weno5_linear_fix, c->v, c->prim, c->sensor, c->fhat, nf, c->sensor_bx, 0)
+  const int share = face_share(c, nf), tf = tb_or(c, c->tb_euler, nf << share);
+#define IZEM_FACE(DD, NGV)                                                                                \
+  k_euler_face<NRV, DD, NGV><<<grid_for(nf << share, tf), tf, 0, c->stream>>>(                              \
+      g, c->cfg.weno_avg, c->cfg.weno5_linear_fix, c->v, c->prim, c->sensor, c->fhat, nf, c->sensor_bx, 0, share)
   rc = launch(c, names[d], [&] {
     if (g.ng == 4) {   // WENO7
       if (d == 0) IZEM_FACE(0, 4);
@@ -255,9 +268,10 @@ int enq_euler(izem_ctx* c, int d) {
   if (rc) return rc;
   if (d == 0 && c->sensor_bx < g.n[0]) {   // block-edge faces as seen by the right block
     rc = launch(c, "euler_face_edge", [&] {
-#define IZEM_EDGE(NGV)                                                                                            \
-  k_euler_face<NRV, 0, NGV><<<grid_for(c->nedge, tb(c, c->nedge)), tb(c, c->nedge), 0, c->stream>>>(                      \
-      g, c->cfg.weno_avg, c->cfg.weno5_linear_fix, c->v, c->prim, c->sensor, c->fhat_edge, c->nedge, c->sensor_bx, 1)
+      const int se = face_share(c, c->nedge), te = tb(c, c->nedge << se);
+#define IZEM_EDGE(NGV)                                                                                    \
+  k_euler_face<NRV, 0, NGV><<<grid_for(c->nedge << se, te), te, 0, c->stream>>>(                            \
+      g, c->cfg.weno_avg, c->cfg.weno5_linear_fix, c->v, c->prim, c->sensor, c->fhat_edge, c->nedge, c->sensor_bx, 1, se)
       if (g.ng == 4) IZEM_EDGE(4);
       else IZEM_EDGE(3);
 #undef IZEM_EDGE

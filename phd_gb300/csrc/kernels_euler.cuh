@@ -362,14 +362,15 @@ __global__ void __launch_bounds__(256) k_euler_face(Geo g, int weno_avg, int lin
                                                     const double* __restrict__ v,
                                                     const double* __restrict__ prim,
                                                     const uint8_t* __restrict__ sensor,
-                                                    double* __restrict__ fhat, long long nfaces, int bx, int edge) {
+                                                    double* __restrict__ fhat, long long nfaces, int bx, int edge, int share) {
   constexpr int NV = IZEM_NIV + NRV;
   constexpr int T1 = D == 0 ? 1 : 0;
   constexpr int T2 = D == 2 ? 1 : 2;
-  long long idx = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  // lanes past the end repeat the last face: sensed faces are a warp's work
-  const bool valid = idx < nfaces;
-  if (!valid) idx = nfaces - 1;
+  // 2^share lanes to a face, the first of which stores it; lanes past the end
+  // repeat the last face: sensed faces are a warp's work
+  long long idx = (blockIdx.x * (long long)blockDim.x + threadIdx.x) >> share;
+  const bool valid = idx < nfaces && (threadIdx.x & ((1 << share) - 1)) == 0;
+  if (idx >= nfaces) idx = nfaces - 1;
   int c[3];
   if (D == 0 && edge) {
     const int ne = g.n[0] / bx - 1;
