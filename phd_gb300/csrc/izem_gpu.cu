@@ -53,6 +53,18 @@ int face_share(const izem_ctx* c, long long faces) {
   const long long warps = (faces + 31) / 32;
   return 4 * warps <= 4LL * c->nsm ? 2 : (2 * warps <= 4LL * c->nsm ? 1 : 0);
 }
+// Block rows that share the `parts` independent pieces of a point's work
+// (components, axes): as many as keep a grid of n points within 32 warps an SM.
+// Below that a point kernel waits on its own chain of loads and FP64
+// operations, and the index arithmetic done again in each row is free; above it
+// the FP64 pipe is full.  Limits of 8, 16 and 32 warps are alike.  Gradients and
+// divergence of the 400 x 11 shock tube 22.3 -> 9.9 and 22.4 -> 9.2 us, of 33 x
+// 40 x 21 35 -> 29 and 37 -> 27; a pass of the former 15.95 -> 14.23 ms, a step
+// of the latter 6.8 -> 6.6.
+int rows_for(const izem_ctx* c, long long n, int parts) {
+  const long long warps = (n + 31) / 32, fit = 32LL * c->nsm / warps;
+  return fit >= parts ? parts : (fit < 2 ? 1 : (int)fit);
+}
 int tb_or(const izem_ctx* c, int tuned, long long n) { return tuned ? tuned : tb(c, n); }
 
 }  // namespace
@@ -295,8 +307,11 @@ int enq_visc(izem_ctx* c) {
   const int nderiv = (eg ? 15 : 12) + 3 * NRV;
   int rc;
   if ((rc = launch(c, "visc_grad", [&] {
-         auto kern = g.ng == 4 ? k_grad<NRV, 4> : k_grad<NRV, 3>;
-         kern<<<grid_for(g.nint, tb(c, g.nint)), tb(c, g.nint), 0, c->stream>>>(g, mt, c->prim, c->T, c->Xa, c->fd);
+         const int rows = rows_for(c, g.nint, 3 * (4 + NRV));
+         auto kern = rows >= 3 ? (g.ng == 4 ? k_grad<NRV, 4, true> : k_grad<NRV, 3, true>)
+                           : (g.ng == 4 ? k_grad<NRV, 4, false> : k_grad<NRV, 3, false>);
+         const dim3 grid(grid_for(g.nint, tb(c, g.nint)), rows >= 3 ? 3 : 1, rows >= 3 ? rows / 3 : 1);
+         kern<<<grid, tb(c, g.nint), 0, c->stream>>>(g, mt, c->prim, c->T, c->Xa, c->fd);
        })))
     return rc;
   if (eg && (rc = launch(c, "visc_grad_p", [&] {
@@ -312,9 +327,9 @@ int enq_visc(izem_ctx* c) {
               })))
     return rc;
   long long ns = slab_count(g) - g.nint;
-  if ((rc = launch(c, "visc_wrap", [&] { k_wrap_periodic<<<grid_for(ns, tb(c, ns)), tb(c, ns), 0, c->stream>>>(g, nderiv, c->fd); })))
+  if ((rc = launch(c, "visc_wrap", [&] { k_wrap_periodic<<<dim3(grid_for(ns, tb(c, ns)), 8), tb(c, ns), 0, c->stream>>>(g, nderiv, c->fd); })))
     return rc;
-  if (les && (rc = launch(c, "les_wrap", [&] { k_wrap_periodic<<<grid_for(ns, tb(c, ns)), tb(c, ns), 0, c->stream>>>(g, 4, c->les); })))
+  if (les && (rc = launch(c, "les_wrap", [&] { k_wrap_periodic<<<dim3(grid_for(ns, tb(c, ns)), 4), tb(c, ns), 0, c->stream>>>(g, 4, c->les); })))
     return rc;
   const long long ns_all = slab_count(g);
   const int tv = tb_or(c, c->tb_visc, ns_all);
@@ -354,8 +369,10 @@ int enq_visc(izem_ctx* c) {
        })))
     return rc;
   return launch(c, "visc_div", [&] {
-    auto kern = g.ng == 4 ? k_visc_div<NRV, 4> : k_visc_div<NRV, 3>;
-    kern<<<grid_for(g.nint, tb(c, g.nint)), tb(c, g.nint), 0, c->stream>>>(g, mt, c->tau, c->qv, c->fd, c->f);
+    const int rows = rows_for(c, g.nint, 4 + NRV);
+    auto kern = rows > 1 ? (g.ng == 4 ? k_visc_div<NRV, 4, true> : k_visc_div<NRV, 3, true>)
+                         : (g.ng == 4 ? k_visc_div<NRV, 4, false> : k_visc_div<NRV, 3, false>);
+    kern<<<dim3(grid_for(g.nint, tb(c, g.nint)), rows), tb(c, g.nint), 0, c->stream>>>(g, mt, c->tau, c->qv, c->fd, c->f);
   });
 }
 

@@ -196,7 +196,9 @@ __global__ void k_sensor_ducros(Geo g, Metrics mt, const double* __restrict__ pr
 
 // First derivatives of u, v, w, T (fd 1..12) and of the mole fractions
 // (fd 13.. : 3 per species) at interior points (module_viscflux.f90:1764-1804).
-template <int NRV, int NG>
+// SPLIT, for small grids: an axis to each of three block rows, the variables
+// shared by the grid's z.
+template <int NRV, int NG, bool SPLIT>
 __global__ void k_grad(Geo g, Metrics mt, const double* __restrict__ prim, const double* __restrict__ T,
                        const double* __restrict__ Xa, double* __restrict__ fd) {
   long long idx = blockIdx.x * (long long)blockDim.x + threadIdx.x;
@@ -208,21 +210,36 @@ __global__ void k_grad(Geo g, Metrics mt, const double* __restrict__ prim, const
   c[2] = (int)(r / g.n[1]) + 1;
   const long long nc = g.ncell;
   const long long p = gid(g, c[0], c[1], c[2]);
-  const long long strides[3] = {1LL, (long long)g.g[0], (long long)g.g[0] * g.g[1]};
   const double* src[4] = {prim + PR_U * nc, prim + PR_V * nc, prim + PR_W * nc, T};
-#pragma unroll
-  for (int d = 0; d < 3; ++d) {
-    const DerivRow<NG> row = deriv_row<NG>(strides[d], c[d], g.n[d], g.bnd[2 * d], g.bnd[2 * d + 1],
-                                           mt.dxi[d][c[d] - 1 + NG]);
+  auto axis = [&](int d) {
+    const long long stride = d == 0 ? 1LL : (d == 1 ? (long long)g.g[0] : (long long)g.g[0] * g.g[1]);
+    const int cd = d == 0 ? c[0] : (d == 1 ? c[1] : c[2]);
+    const DerivRow<NG> row = deriv_row<NG>(stride, cd, g.n[d], g.bnd[2 * d], g.bnd[2 * d + 1],
+                                           mt.dxi[d][cd - 1 + NG]);
     const bool none = d == 2 && g.ndim == 2;   // a 2-D run has no z derivative
+    if constexpr (SPLIT) {
+      for (int s = blockIdx.z; s < 4 + NRV; s += gridDim.z) {
+        const double* a = s >= 4 ? Xa + (s - 4) * nc : (s == 3 ? T : prim + (PR_U + s) * nc);
+        fd[(3 * s + d) * nc + p] = none ? 0.0 : deriv_at<NG>(a, p, row);
+      }
+      return;
+    }
 #pragma unroll
     for (int s = 0; s < 4; ++s) fd[(3 * s + d) * nc + p] = none ? 0.0 : deriv_at<NG>(src[s], p, row);
 #pragma unroll
     for (int l = 0; l < NRV; ++l) fd[(12 + 3 * l + d) * nc + p] = none ? 0.0 : deriv_at<NG>(Xa + l * nc, p, row);
+  };
+  if constexpr (SPLIT) {
+    axis(blockIdx.y);
+  } else {
+    axis(0);
+    axis(1);
+    axis(2);
   }
 }
 
-// Periodic wrap of the face-ghost slabs of an ncomp-component ghosted array.
+// Periodic wrap of the face-ghost slabs of an ncomp-component ghosted array,
+// the components shared by the block rows.
 __global__ void k_wrap_periodic(Geo g, int ncomp, double* __restrict__ a) {
   long long idx = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   const long long ntot = slab_count(g) - g.nint;
@@ -234,7 +251,7 @@ __global__ void k_wrap_periodic(Geo g, int ncomp, double* __restrict__ a) {
   int c[3] = {i, j, k};
   c[d] = (f & 1) ? c[d] - g.n[d] : c[d] + g.n[d];
   const long long p = gid(g, i, j, k), q = gid(g, c[0], c[1], c[2]);
-  for (int m = 0; m < ncomp; ++m) a[(long long)m * g.ncell + p] = a[(long long)m * g.ncell + q];
+  for (int m = blockIdx.y; m < ncomp; m += gridDim.y) a[(long long)m * g.ncell + p] = a[(long long)m * g.ncell + q];
 }
 
 // Transport properties, stresses, diffusion velocities with correction
@@ -409,7 +426,8 @@ __global__ void k_visc_point(Geo g, const double* __restrict__ v, const double* 
 }
 
 // Divergence of the viscous fluxes added to f (module_viscflux.f90:2098-2183).
-template <int NRV, int NG>
+// SPLIT: the components are shared by the block rows, for small grids.
+template <int NRV, int NG, bool SPLIT>
 __global__ void k_visc_div(Geo g, Metrics mt, const double* __restrict__ tau, const double* __restrict__ qv,
                            const double* __restrict__ fd, double* __restrict__ fl) {
   long long idx = blockIdx.x * (long long)blockDim.x + threadIdx.x;
@@ -432,6 +450,22 @@ __global__ void k_visc_div(Geo g, Metrics mt, const double* __restrict__ tau, co
     return g.ndim == 2 ? w : deriv_add<NG>(w, az, p, row[2]);
   };
   const long long ni = g.nint;
+  if constexpr (SPLIT) {
+    for (int m = blockIdx.y; m < 4 + NRV; m += gridDim.y) {
+      const double *ax, *ay, *az;
+      if (m < 3) {   // rows of the stress tensor, kept as xx, xy, xz, yy, yz, zz
+        ax = tau + m * nc;
+        ay = tau + (m == 0 ? 1 : m + 2) * nc;
+        az = tau + (m == 0 ? 2 : m + 3) * nc;
+      } else {
+        ax = m == 3 ? qv : fd + (12 + 3 * (m - 4)) * nc;
+        ay = ax + nc;
+        az = ay + nc;
+      }
+      fl[(1 + m) * ni + idx] = fl[(1 + m) * ni + idx] + div3(ax, ay, az);
+    }
+    return;
+  }
   fl[1 * ni + idx] = fl[1 * ni + idx] + div3(tau + 0 * nc, tau + 1 * nc, tau + 2 * nc);
   fl[2 * ni + idx] = fl[2 * ni + idx] + div3(tau + 1 * nc, tau + 3 * nc, tau + 4 * nc);
   fl[3 * ni + idx] = fl[3 * ni + idx] + div3(tau + 2 * nc, tau + 4 * nc, tau + 5 * nc);
