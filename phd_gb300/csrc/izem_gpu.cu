@@ -322,8 +322,9 @@ int enq_visc(izem_ctx* c) {
   const bool les = c->les_on;
   if (les && (rc = launch(c, "les_prep", [&] {
                 // the criterion of shock_det_slv under EGLIB, of shock_det_ducros_slv with the fitted transport
-                k_les_prep<<<grid_for(g.nint, tb(c, g.nint)), tb(c, g.nint), 0, c->stream>>>(g, mt, c->v, c->T, c->W_i, c->les_pw, c->les,
-                                                                         c->prim, eg ? 0 : 1);
+                auto kern = g.ng == 4 ? k_les_prep<4> : k_les_prep<3>;
+                kern<<<grid_for(g.nint, tb(c, g.nint)), tb(c, g.nint), 0, c->stream>>>(g, mt, c->v, c->T, c->W_i, c->les_pw,
+                                                                                     c->les, c->prim, eg ? 0 : 1);
               })))
     return rc;
   long long ns = slab_count(g) - g.nint;
