@@ -144,15 +144,15 @@ CHEM_BYTES_PER_REACTOR = 11 * 8 + 10 * 8
 # generated right-hand side (2 DFMA + DADD + DMUL per thread, summed by ncu
 # over one launch on the 64x64x32 mixing-layer window, 81,225 reactors and
 # 243,675 BDF steps, / those steps)
-CHEM_FLOP_PER_BDF_STEP = 6712
+CHEM_FLOP_PER_BDF_STEP = 3209
 # DRAM bytes (read + write) per reactor of that launch, scaled by reactors to
 # other windows: the per-thread BDF state in local memory that the L2 does
 # not hold
-CHEM_TRAFFIC_PER_REACTOR = 11071
+CHEM_TRAFFIC_PER_REACTOR = 13121
 
 # FP64 flops per face of k_euler_face (2 DFMA + DADD + DMUL per thread, summed
 # by ncu over one launch of the 9-species mixing layer, / faces)
-EULER_FLOP_PER_FACE = {9: 1869}
+EULER_FLOP_PER_FACE = {9: 902}
 
 
 def make_stepper(g, chem, mode=0):
