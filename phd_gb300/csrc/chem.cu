@@ -1834,6 +1834,21 @@ int chem_grid(int* blocks) {
   return 0;
 }
 
+// The launch for n cells.  Fewer cells than the full grid has threads are a
+// cell a thread: one-warp blocks then, as many as the cells fill, which the
+// hardware deals out evenly over the SMs; of the full grid's warps the first to
+// come would take them all, on part of the SMs.  Half step of the 33 x 40 x 21
+// layer's window 0.96 -> 0.45 ms, 4000 reactors 0.49 -> 0.39 (one: 0.35).
+int chem_shape(long long n, int* blocks, int* threads) {
+  if (chem_grid(blocks)) return -1;
+  *threads = kChemThreads;
+  if (n < (long long)*blocks * kChemThreads) {
+    *threads = 32;
+    *blocks = n > 0 ? (int)((n + 31) / 32) : 1;
+  }
+  return 0;
+}
+
 }  // namespace
 
 // ---------------------------------------------------------- host side -------
@@ -1878,23 +1893,23 @@ cudaError_t chem_upload_mech(const izem_mech* m) {
 }
 
 cudaError_t chem_launch_field(const ChemField& f, unsigned* d_counter, ChemStats* d_stats, cudaStream_t s, int kk) {
-  int blocks = 0;
-  if (chem_grid(&blocks)) return cudaErrorUnknown;
+  int blocks = 0, threads = 0;
+  if (chem_shape((long long)f.wx * f.wy * f.wz, &blocks, &threads)) return cudaErrorUnknown;
   cudaError_t e = cudaMemsetAsync(d_counter, 0, sizeof(unsigned), s);
   if (e != cudaSuccess) return e;
   if (kk != 9) return cudaErrorInvalidValue;
-  chem_kernels(g_chem_variant).field<<<blocks, kChemThreads, 0, s>>>(f, d_counter, d_stats);
+  chem_kernels(g_chem_variant).field<<<blocks, threads, 0, s>>>(f, d_counter, d_stats);
   return cudaGetLastError();
 }
 
 cudaError_t chem_launch_batch(int n, double* T, const double* rho, double* Y, const double* dt, int* istate, int* nsteps,
                               unsigned* d_counter, ChemStats* d_stats, cudaStream_t s, int kk) {
-  int blocks = 0;
-  if (chem_grid(&blocks)) return cudaErrorUnknown;
+  int blocks = 0, threads = 0;
+  if (chem_shape(n, &blocks, &threads)) return cudaErrorUnknown;
   cudaError_t e = cudaMemsetAsync(d_counter, 0, sizeof(unsigned), s);
   if (e != cudaSuccess) return e;
   if (kk != 9) return cudaErrorInvalidValue;
-  chem_kernels(g_chem_variant).batch<<<blocks, kChemThreads, 0, s>>>(n, T, rho, Y, dt, istate, nsteps, d_counter,
+  chem_kernels(g_chem_variant).batch<<<blocks, threads, 0, s>>>(n, T, rho, Y, dt, istate, nsteps, d_counter,
                                                                       d_stats);
   return cudaGetLastError();
 }
