@@ -245,7 +245,7 @@ __device__ __forceinline__ void weno_face_lanes(unsigned sensed, const FaceState
   constexpr unsigned full = 0xffffffffu;
   const int lane = threadIdx.x & 31, grp = lane / GL, m = lane % GL;
   while (sensed) {
-    // the faces of this round: group g takes the g-th set bit (the first
+    // the faces of this pass: group g takes the g-th set bit (the first
     // again when there are fewer; it does not store then)
     unsigned rest = sensed;
     for (int g = 0; g < grp && rest; ++g) rest &= rest - 1;
