@@ -1881,15 +1881,16 @@ bool chem_mech_valid(const izem_mech* m) {
   return true;
 }
 
-cudaError_t chem_upload_mech(const izem_mech* m) {
-  cudaError_t e = cudaMemcpyToSymbol(c_mech_dev, m, sizeof(izem_mech));
+cudaError_t chem_upload_mech(const izem_mech* m, cudaStream_t s) {
+  cudaError_t e = cudaMemcpyToSymbolAsync(c_mech_dev, m, sizeof(izem_mech), 0, cudaMemcpyHostToDevice, s);
   if (e != cudaSuccess) return e;
   ChemFast f = chem_fast_constants(*m);
-  if ((e = cudaMemcpyToSymbol(c_fast_dev, &f, sizeof(ChemFast))) != cudaSuccess) return e;
+  if ((e = cudaMemcpyToSymbolAsync(c_fast_dev, &f, sizeof(ChemFast), 0, cudaMemcpyHostToDevice, s)) != cudaSuccess)
+    return e;
   int need = 0;
   for (int i = 0; i < m->ii; ++i) need |= (m->rev[i] == 1);
   g_chem_gen = (g_chem_gen_allowed && chem_gen::matches(*m)) ? 1 : 0;
-  return cudaMemcpyToSymbol(c_need_eqk_dev, &need, sizeof(int));
+  return cudaMemcpyToSymbolAsync(c_need_eqk_dev, &need, sizeof(int), 0, cudaMemcpyHostToDevice, s);
 }
 
 cudaError_t chem_launch_field(const ChemField& f, unsigned* d_counter, ChemStats* d_stats, cudaStream_t s, int kk) {

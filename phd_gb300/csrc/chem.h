@@ -22,7 +22,9 @@ struct ChemStats {
   unsigned long long dtmax_bits;   // max |dT| [K] as a double bit pattern
 };
 
-cudaError_t chem_upload_mech(const izem_mech* m);
+// copies m to the device's constants in the order of stream s, on which the
+// kernels that read them follow
+cudaError_t chem_upload_mech(const izem_mech* m, cudaStream_t s);
 // true when the kernels can evaluate m: 9 species, at most IZEM_MAXREAC
 // reactions, species indices in range, known reverse and fall-off kinds, a
 // collider in range, and nonzero Troe and SRI temperatures where the rate

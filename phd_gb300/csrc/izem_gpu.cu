@@ -795,7 +795,10 @@ int ctx_alloc(izem_ctx* c) {
     CK(cudaGetDevice(&dev));
     CK(cudaDeviceGetAttribute(&c->nsm, cudaDevAttrMultiProcessorCount, dev));
   }
-  CK(cudaMemcpyToSymbol(c_thd, &c->devthd, sizeof(DevThd)));
+  // All set-up work goes to the context's stream, here and in the setters below:
+  // the stream is non-blocking, so that nothing orders its kernels after a copy or
+  // a fill on the default stream, and both may return before they are done.
+  CK(cudaMemcpyToSymbolAsync(c_thd, &c->devthd, sizeof(DevThd), 0, cudaMemcpyHostToDevice, c->stream));
   auto alloc = [&](double** p, size_t n) -> cudaError_t {
     cudaError_t e = cudaMalloc(p, n * sizeof(double));
     if (e == cudaSuccess) c->allocs.push_back(*p);
@@ -817,22 +820,23 @@ int ctx_alloc(izem_ctx* c) {
   for (int d = 0; d < 3; ++d)
     if ((e = alloc(&c->dxi[d], g.g[d]))) return ctx_fail(c, IZEM_ERR_CUDA, "device allocation", e);
   CK(cudaMalloc(&c->sensor, nc));
-  CK(cudaMemset(c->sensor, 0, nc));
+  CK(cudaMemsetAsync(c->sensor, 0, nc, c->stream));
   CK(cudaMalloc(&c->d_status, sizeof(DevStatus)));
-  CK(cudaMemset(c->d_status, 0, sizeof(DevStatus)));
+  CK(cudaMemsetAsync(c->d_status, 0, sizeof(DevStatus), c->stream));
   CK(cudaMallocHost(&c->h_status, sizeof(DevStatus)));
   CK(cudaMallocHost(&c->h_dt, 4 * sizeof(double)));
   // dt, time0 of the RK3 step; zeros for calls outside rk3; the half step
   // and time of the last chemistry step
-  CK(cudaMemset(c->d_dt, 0, 6 * sizeof(double)));
+  CK(cudaMemsetAsync(c->d_dt, 0, 6 * sizeof(double), c->stream));
   // zero the arrays whose ghost corners are never written
-  CK(cudaMemset(c->v, 0, nv * nc * sizeof(double)));
-  CK(cudaMemset(c->fd, 0, (15 + 3 * nrv) * nc * sizeof(double)));
-  CK(cudaMemset(c->tau, 0, 6 * nc * sizeof(double)));
-  CK(cudaMemset(c->qv, 0, 3 * nc * sizeof(double)));
-  CK(cudaMemset(c->f, 0, nv * ni * sizeof(double)));
+  CK(cudaMemsetAsync(c->v, 0, nv * nc * sizeof(double), c->stream));
+  CK(cudaMemsetAsync(c->fd, 0, (15 + 3 * nrv) * nc * sizeof(double), c->stream));
+  CK(cudaMemsetAsync(c->tau, 0, 6 * nc * sizeof(double), c->stream));
+  CK(cudaMemsetAsync(c->qv, 0, 3 * nc * sizeof(double), c->stream));
+  CK(cudaMemsetAsync(c->f, 0, nv * ni * sizeof(double), c->stream));
   CK(cudaEventCreate(&c->t0));
   CK(cudaEventCreate(&c->t1));
+  CK(cudaStreamSynchronize(c->stream));
   return IZEM_OK;
 }
 
@@ -898,7 +902,9 @@ int izem_gpu_last_error(izem_ctx* c, char* buf, int n) {
 int izem_gpu_set_grid(izem_ctx* c, const double* dx_i, const double* dy_i, const double* dz_i) {
   if (!c || !dx_i || !dy_i || !dz_i) return IZEM_ERR_ARG;
   const double* s[3] = {dx_i, dy_i, dz_i};
-  for (int d = 0; d < 3; ++d) CK(cudaMemcpy(c->dxi[d], s[d], c->g.g[d] * sizeof(double), cudaMemcpyHostToDevice));
+  for (int d = 0; d < 3; ++d)
+    CK(cudaMemcpyAsync(c->dxi[d], s[d], c->g.g[d] * sizeof(double), cudaMemcpyHostToDevice, c->stream));
+  CK(cudaStreamSynchronize(c->stream));
   c->grid_set = true;
   return IZEM_OK;
 }
@@ -1113,7 +1119,8 @@ int izem_gpu_set_eglib(izem_ctx* c, const izem_eglib* L) {
     return ctx_fail(c, IZEM_ERR_ARG, "EGLIB linking data must have nrv species", cudaSuccess);
   DevEg e;
   eg_prepare(*L, c->thd, c->adi, e);
-  CK(cudaMemcpyToSymbol(c_eg, &e, sizeof(DevEg)));
+  // ahead of the table's kernel, which reads it and whose result stays with the context
+  CK(cudaMemcpyToSymbolAsync(c_eg, &e, sizeof(DevEg), 0, cudaMemcpyHostToDevice, c->stream));
   int rc = IZEM_DISPATCH(c, eg_build_table, c);
   if (rc) return rc;
   c->have_eg = true;
@@ -1128,7 +1135,8 @@ int izem_gpu_set_mechanism(izem_ctx* c, const izem_mech* mech) {
     return ctx_fail(c, IZEM_ERR_ARG, "mechanism tables out of range (species index, reverse or fall-off kind, "
                     "collider, or a zero Troe/SRI temperature)", cudaSuccess);
   c->mech = *mech;
-  CK(chem_upload_mech(mech));
+  CK(chem_upload_mech(mech, c->stream));
+  CK(cudaStreamSynchronize(c->stream));
   if (!c->d_counter) {
     CK(cudaMalloc(&c->d_counter, sizeof(unsigned)));
     CK(cudaMalloc(&c->d_chem_stats, sizeof(ChemStats)));
@@ -1307,7 +1315,7 @@ int izem_gpu_psr_batch(const izem_mech* mech, int n, double* T, const double* rh
   int rc = IZEM_OK;
   auto fail = [&](int code) { rc = code; };
   do {
-    if (chem_upload_mech(mech) != cudaSuccess) { fail(IZEM_ERR_CUDA); break; }
+    if (chem_upload_mech(mech, s) != cudaSuccess) { fail(IZEM_ERR_CUDA); break; }
     if (cudaMalloc(&mem, small + (device_ptrs ? 0 : (3 + kk) * n8 + 2 * n4)) != cudaSuccess) {
       fail(IZEM_ERR_NOMEM); break;
     }
@@ -1440,8 +1448,9 @@ int izem_gpu_set_coords(izem_ctx* c, const double* x, const double* y, const dou
     CK(cudaMalloc(&c->d_y, c->g.n[1] * sizeof(double)));
     CK(cudaMalloc(&c->d_z, c->g.n[2] * sizeof(double)));
   }
-  CK(cudaMemcpy(c->d_y, y, c->g.n[1] * sizeof(double), cudaMemcpyHostToDevice));
-  CK(cudaMemcpy(c->d_z, z, c->g.n[2] * sizeof(double), cudaMemcpyHostToDevice));
+  CK(cudaMemcpyAsync(c->d_y, y, c->g.n[1] * sizeof(double), cudaMemcpyHostToDevice, c->stream));
+  CK(cudaMemcpyAsync(c->d_z, z, c->g.n[2] * sizeof(double), cudaMemcpyHostToDevice, c->stream));
+  CK(cudaStreamSynchronize(c->stream));
   JetArgs& j = c->jet;
   j.y = c->d_y;
   j.z = c->d_z;
@@ -1487,7 +1496,7 @@ int izem_gpu_set_les(izem_ctx* c, int enable, double mu_sgs_factor, double sc_sg
   drop_graphs(c);
   if (!enable) {
     c->les_on = false;
-    if (c->mu_sgs) CK(cudaMemset(c->mu_sgs, 0, (size_t)c->g.ncell * sizeof(double)));
+    if (c->mu_sgs) CK(cudaMemsetAsync(c->mu_sgs, 0, (size_t)c->g.ncell * sizeof(double), c->stream));
     return IZEM_OK;
   }
   if (!c->cfg.vis || c->cfg.ndim != 3)
@@ -1496,7 +1505,7 @@ int izem_gpu_set_les(izem_ctx* c, int enable, double mu_sgs_factor, double sc_sg
     return ctx_fail(c, IZEM_ERR_ARG, "LES parameters out of range", cudaSuccess);
   if (!c->les) {
     CK(cudaMalloc(&c->les, 4 * (size_t)c->g.ncell * sizeof(double)));
-    CK(cudaMemset(c->les, 0, 4 * (size_t)c->g.ncell * sizeof(double)));
+    CK(cudaMemsetAsync(c->les, 0, 4 * (size_t)c->g.ncell * sizeof(double), c->stream));
   }
   double cs2 = mu_sgs_factor;
   cs2 = cs2 * cs2 / c->adi.sqgmr;
@@ -1506,7 +1515,7 @@ int izem_gpu_set_les(izem_ctx* c, int enable, double mu_sgs_factor, double sc_sg
   c->les_pr_sgs_i = 1.0 / pr_sgs;
   if (!c->cfg.eglib && !c->mu_sgs) {   // viscflux_LES_xyz hands mu_SGS to the time step
     CK(cudaMalloc(&c->mu_sgs, (size_t)c->g.ncell * sizeof(double)));
-    CK(cudaMemset(c->mu_sgs, 0, (size_t)c->g.ncell * sizeof(double)));
+    CK(cudaMemsetAsync(c->mu_sgs, 0, (size_t)c->g.ncell * sizeof(double), c->stream));
   }
   c->les_pw = percent_weight_sgs;
   c->les_on = true;
@@ -1590,7 +1599,7 @@ int izem_gpu_chem_autotune(const izem_mech* mech, int n, const double* T, const 
   for (float& x : ms) x = 1e30f;   // untimed candidates never win
   int best = chem_variant();
   do {
-    if (chem_upload_mech(mech) != cudaSuccess) { rc = IZEM_ERR_CUDA; break; }
+    if (chem_upload_mech(mech, s) != cudaSuccess) { rc = IZEM_ERR_CUDA; break; }
     if (cudaMalloc(&T0, ns * 8) || cudaMalloc(&Y0, (size_t)ns * 72) || cudaMalloc(&r, ns * 8) ||
         cudaMalloc(&d, ns * 8) || cudaMalloc(&Tw, ns * 8) || cudaMalloc(&Yw, (size_t)ns * 72) ||
         cudaMalloc(&counter, sizeof(unsigned)) || cudaMalloc(&st, sizeof(ChemStats))) { rc = IZEM_ERR_NOMEM; break; }

@@ -148,7 +148,7 @@ cudaError_t mlp_ensure(izem_mlp* m, int rows) {
   m->splits = (nchunks + m->split_chunks - 1) / m->split_chunks;
   cudaError_t e;
   if ((e = cudaMalloc(&m->xa, M * 16 * 2)) || (e = cudaMalloc(&m->xt, 128 * M * 2)) ||
-      (e = cudaMemset(m->xt, 0, 128 * M * 2)) ||
+      (e = cudaMemsetAsync(m->xt, 0, 128 * M * 2, m->s)) ||
       (e = cudaMalloc(&m->gout, M * 16 * 4)) || (e = cudaMalloc(&m->goa, M * 16 * 2)) ||
       (e = cudaMalloc(&m->got, M * 16 * 2)) ||
       (e = cudaMalloc(&m->dza[0], M * H * 2)) || (e = cudaMalloc(&m->dza[1], M * H * 2)) ||
@@ -403,8 +403,9 @@ int izem_mlp_create(izem_mlp** out) {
            cudaMalloc(&m->mW[l], nw * 4) || cudaMalloc(&m->vW[l], nw * 4) || cudaMalloc(&m->mb[l], nb * 4) ||
            cudaMalloc(&m->vb[l], nb * 4) || cudaMalloc(&m->gW[l], nw * 4) || cudaMalloc(&m->gb[l], nb * 4));
     if (ok) {
-      cudaMemset(m->mW[l], 0, nw * 4); cudaMemset(m->vW[l], 0, nw * 4);
-      cudaMemset(m->mb[l], 0, nb * 4); cudaMemset(m->vb[l], 0, nb * 4);
+      // on the handle's stream, which is not ordered after the default one
+      ok = !(cudaMemsetAsync(m->mW[l], 0, nw * 4, m->s) || cudaMemsetAsync(m->vW[l], 0, nw * 4, m->s) ||
+             cudaMemsetAsync(m->mb[l], 0, nb * 4, m->s) || cudaMemsetAsync(m->vb[l], 0, nb * 4, m->s));
     }
   }
   ok = ok && cudaMalloc(&m->d_loss, sizeof(double)) == cudaSuccess;
@@ -412,7 +413,8 @@ int izem_mlp_create(izem_mlp** out) {
     ok = cudaMalloc(&m->blob[l], (size_t)LIN[l] * LOUT[l] * 2) == cudaSuccess &&
          cudaMalloc(&m->wt[l], (size_t)LIN[l] * LOUT[l] * 2) == cudaSuccess &&
          cudaMalloc(&m->wn[l], (size_t)LIN[l] * LOUT[l] * 2) == cudaSuccess;
-  ok = ok && cudaMalloc(&m->d_err, sizeof(int)) == cudaSuccess && cudaMemset(m->d_err, 0, sizeof(int)) == cudaSuccess;
+  ok = ok && cudaMalloc(&m->d_err, sizeof(int)) == cudaSuccess &&
+       cudaMemsetAsync(m->d_err, 0, sizeof(int), m->s) == cudaSuccess && cudaStreamSynchronize(m->s) == cudaSuccess;
   if (!ok) {
     izem_mlp_destroy(m);   // frees what was allocated (cudaFree of a null pointer is a no-op)
     return IZEM_ERR_NOMEM;
@@ -452,8 +454,9 @@ int izem_mlp_set_params(izem_mlp* m, const float* const* W, const float* const* 
   m->blob_dirty = true;
   for (int l = 0; l < NL; ++l) {
     const size_t nw = (size_t)LIN[l] * LOUT[l];
-    if (cudaMemcpy(m->W[l], W[l], nw * 4, cudaMemcpyHostToDevice) != cudaSuccess) return IZEM_ERR_CUDA;
-    if (cudaMemcpy(m->b[l], b[l], LOUT[l] * 4, cudaMemcpyHostToDevice) != cudaSuccess) return IZEM_ERR_CUDA;
+    if (cudaMemcpyAsync(m->W[l], W[l], nw * 4, cudaMemcpyHostToDevice, m->s) != cudaSuccess ||
+        cudaMemcpyAsync(m->b[l], b[l], LOUT[l] * 4, cudaMemcpyHostToDevice, m->s) != cudaSuccess)
+      return IZEM_ERR_CUDA;
   }
   if (mlp_weight_copies(m) != cudaSuccess) return IZEM_ERR_CUDA;
   return cudaStreamSynchronize(m->s) == cudaSuccess ? IZEM_OK : IZEM_ERR_CUDA;
@@ -480,7 +483,7 @@ int izem_gpu_reactor_rhs(const izem_mech* mech, int n, const double* T, const do
                          double* zdot, int device_ptrs) {
   if (!mech || n <= 0 || !T || !rho || !Y || !zdot || !chem_mech_valid(mech)) return IZEM_ERR_ARG;
   (void)cudaGetLastError();
-  if (chem_upload_mech(mech) != cudaSuccess) return IZEM_ERR_CUDA;
+  if (chem_upload_mech(mech, 0) != cudaSuccess) return IZEM_ERR_CUDA;
   if (device_ptrs) {
     if (chem_launch_rhs(n, T, rho, Y, zdot, 0) != cudaSuccess) return IZEM_ERR_CUDA;
     return cudaStreamSynchronize(0) == cudaSuccess ? IZEM_OK : IZEM_ERR_CUDA;
@@ -490,8 +493,9 @@ int izem_gpu_reactor_rhs(const izem_mech* mech, int n, const double* T, const do
   int rc = IZEM_OK;
   if (cudaMalloc(&dT, n8) || cudaMalloc(&dr, n8) || cudaMalloc(&dY, 9 * n8) || cudaMalloc(&dz, 10 * n8)) {
     rc = IZEM_ERR_NOMEM;
-  } else if (cudaMemcpy(dT, T, n8, cudaMemcpyHostToDevice) || cudaMemcpy(dr, rho, n8, cudaMemcpyHostToDevice) ||
-             cudaMemcpy(dY, Y, 9 * n8, cudaMemcpyHostToDevice) || chem_launch_rhs(n, dT, dr, dY, dz, 0) ||
+  } else if (cudaMemcpyAsync(dT, T, n8, cudaMemcpyHostToDevice, 0) ||
+             cudaMemcpyAsync(dr, rho, n8, cudaMemcpyHostToDevice, 0) ||
+             cudaMemcpyAsync(dY, Y, 9 * n8, cudaMemcpyHostToDevice, 0) || chem_launch_rhs(n, dT, dr, dY, dz, 0) ||
              cudaMemcpy(zdot, dz, 10 * n8, cudaMemcpyDeviceToHost)) {
     rc = IZEM_ERR_CUDA;
   }
@@ -539,8 +543,8 @@ int izem_mlp_grads(izem_mlp* m, int M, const float* x, const float* t, double* l
     return IZEM_ERR_NOMEM;
   }
   int rc = IZEM_OK;
-  if (cudaMemcpy(dx, x, (size_t)M * IN * 4, cudaMemcpyHostToDevice) != cudaSuccess ||
-      cudaMemcpy(dt, t, (size_t)M * OUT * 4, cudaMemcpyHostToDevice) != cudaSuccess)
+  if (cudaMemcpyAsync(dx, x, (size_t)M * IN * 4, cudaMemcpyHostToDevice, m->s) != cudaSuccess ||
+      cudaMemcpyAsync(dt, t, (size_t)M * OUT * 4, cudaMemcpyHostToDevice, m->s) != cudaSuccess)
     rc = IZEM_ERR_CUDA;
   if (rc == IZEM_OK) {
     if (cudaMemsetAsync(m->d_loss, 0, sizeof(double), m->s) != cudaSuccess ||
@@ -670,7 +674,7 @@ int izem_gpu_psr_batch_mlp(izem_mlp* m, izem_mlp* m2, const izem_mech* mech, int
     if (cudaMalloc(&m->g_list, (size_t)n * sizeof(int)) != cudaSuccess) return IZEM_ERR_NOMEM;
     m->g_list_cap = n;
   }
-  if (chem_upload_mech(mech) != cudaSuccess) return IZEM_ERR_CUDA;
+  if (chem_upload_mech(mech, s) != cudaSuccess) return IZEM_ERR_CUDA;
   cudaMemcpyAsync(m->d_norm, m->norm, sizeof(m->norm), cudaMemcpyHostToDevice, s);
   if (m2) cudaMemcpyAsync(m2->d_norm, m2->norm, sizeof(m2->norm), cudaMemcpyHostToDevice, s);
   const size_t kk = mech->kk;
