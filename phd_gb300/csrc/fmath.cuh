@@ -354,4 +354,21 @@ __device__ __forceinline__ double fm_div(double a, double x) {
   const double q = a * y;
   return fma(fma(-x, q, a), y, q);
 }
+
+// 1 / (a b) and what the roundings of the product and of the reciprocal leave
+// over; fm_over takes x / (a b) from it with one rounding beyond those of x.
+// Mole fractions X_k = (rho Y_k / W_k) / (rho W_i) of many species share it: rms
+// error 0.60 units of 2^-53 (two roundings), 0.74 as one quotient a species
+// (three), 0.85 as plain products with a reciprocal (four).
+struct fm_pair {
+  double hi, lo;
+};
+__device__ __forceinline__ fm_pair fm_rcp_prod(double a, double b) {
+  const double p = a * b;
+  fm_pair r;
+  r.hi = fm_rcp(p);
+  r.lo = fma(-fma(a, b, -p), r.hi, fma(-p, r.hi, 1.0)) * r.hi;
+  return r;
+}
+__device__ __forceinline__ double fm_over(double x, const fm_pair& r) { return fma(x, r.hi, x * r.lo); }
 #endif  // __CUDACC__

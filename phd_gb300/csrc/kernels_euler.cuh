@@ -72,7 +72,7 @@ __global__ void k_prim(Geo g, const double* __restrict__ v, const double* __rest
   double rho_i = fm_rcp(rho);
   double ux = v[nc + p] * rho_i, vy = v[2 * nc + p] * rho_i, wz = v[3 * nc + p] * rho_i;
   double Wi = W_i[p];
-  const double TW = T[p] * Wi, rw = rho * Wi;
+  const double TW = T[p] * Wi;
   double P = rho * TW;
   if (P <= 0.0) atomicExch(&st->neg_pressure, 1);
   // gamma = cp / (cp - gam2 W_i); one reciprocal for the mole fractions
@@ -81,18 +81,14 @@ __global__ void k_prim(Geo g, const double* __restrict__ v, const double* __rest
   const double cpp = cp[p];
   double cs = sqrt(fm_div(cpp, cpp - c_thd.gam2 * Wi) * TW);
   double ht = 0.0;
-  // X_k = (rho Y_k / W_k) / (rho W_i) with the reciprocal's rounding and the
-  // product's carried along: second derivatives of X see its last bits (rms
-  // error 0.60 units of 2^-53; 0.74 as one quotient a species, 0.85 as plain
-  // products)
-  const double rw_i = fm_rcp(rw);
-  const double rw_lo = fma(-fma(rho, Wi, -rw), rw_i, fma(-rw, rw_i, 1.0)) * rw_i;
+  // the roundings of 1 / (rho W_i) carried along: second derivatives of the
+  // mole fractions see their last bits
+  const fm_pair rw_i = fm_rcp_prod(rho, Wi);
 #pragma unroll
   for (int l = 0; l < NRV; ++l) {
     double rY = v[(IZEM_NIV + l) * nc + p];
     ht = fma(ha[l * nc + p], rY, ht);
-    const double a = rY * c_thd.Wc_i[l];
-    if (Xa) Xa[l * nc + p] = fma(a, rw_i, a * rw_lo);
+    if (Xa) Xa[l * nc + p] = fm_over(rY * c_thd.Wc_i[l], rw_i);
   }
   ht = ht * rho_i;
   ht = ht + 0.5 * (ux * ux + vy * vy + wz * wz);

@@ -370,9 +370,9 @@ __global__ void k_dtv(Geo g, Metrics mt, const double* __restrict__ v, const dou
     const long long p = gid(g, c[0], c[1], c[2]);
     const double rho = v[p], Tp = T[p], Wi = W_i[p];
     double X[NRV];
-    const double rw_i = fm_rcp(rho * Wi);
+    const fm_pair rw_i = fm_rcp_prod(rho, Wi);
 #pragma unroll
-    for (int l = 0; l < NRV; ++l) X[l] = v[(IZEM_NIV + l) * nc + p] * c_thd.Wc_i[l] * rw_i;
+    for (int l = 0; l < NRV; ++l) X[l] = fm_over(v[(IZEM_NIV + l) * nc + p] * c_thd.Wc_i[l], rw_i);
     const double lt1 = fm_log(Tp * c_thd.tinf);
     const double lt2 = lt1 * lt1, lt3 = lt2 * lt1;
     const double P = rho * Tp * Wi;
