@@ -1511,7 +1511,8 @@ __global__ void __launch_bounds__(kChemThreads, MINB) k_psr_batch(int n, double*
 // an ensemble (x2 may be null); rows are 16 BF16 values, written as two
 // 16-byte stores.  Launched with at least 32 threads per block.  Bound by the
 // FP64 pipe, where a library logarithm takes 36 slots: with the fixed-point one
-// 0.87 -> 0.20 ms a million reactors.
+// 0.87 -> 0.25 ms a million reactors (0.05 of it the pressure's, which is the
+// library's near 1 atm).
 // fmax(x, 0) by the bit pattern (a NaN gives 0 there too)
 __device__ __forceinline__ double c_clamp0(double x) {
   const long long b = __double_as_longlong(x);
