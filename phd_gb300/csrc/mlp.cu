@@ -130,10 +130,30 @@ constexpr int part_floats(int layers) { return layers == 0 ? 0 : part_floats(lay
 constexpr int kPartFloats = part_floats(NL);
 static_assert(NL == mlptt::WG_LAYERS, "layers of the batched weight-gradient launch");
 
+constexpr int kTileN = 32;   // columns a tile of the forward and input-gradient GEMMs (k_tgemm)
+
+// The shared memory of the training step's kernels, above the default limit of
+// a launch.  The limit is the current device's, so every handle raises it for
+// its own.
+cudaError_t mlp_train_attributes() {
+  auto raise = [](const void* kern, int nt) {
+    return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)mlptt::tg_smem_bytes(nt));
+  };
+  cudaError_t e;
+  if ((e = raise((const void*)mlptt::k_tgemm<kTileN, mlptt::TG_FWD_GELU>, kTileN)) ||
+      (e = raise((const void*)mlptt::k_tgemm<OUTP, mlptt::TG_FWD_LOSS>, OUTP)) ||
+      (e = raise((const void*)mlptt::k_tgemm<kTileN, mlptt::TG_BWD_GELU>, kTileN)) ||
+      (e = raise((const void*)mlptt::k_tg_wgrad, mlptt::WG_NT)))
+    return e;
+  return cudaSuccess;
+}
+
 // Training buffers for batches of up to `rows` rows (rounded up to 128).
 cudaError_t mlp_ensure(izem_mlp* m, int rows) {
   rows = (rows + 127) / 128 * 128;
   if (rows <= m->cap) return cudaSuccess;
+  cudaError_t e = mlp_train_attributes();
+  if (e != cudaSuccess) return e;
   cudaFree(m->xa); cudaFree(m->xt); cudaFree(m->gout); cudaFree(m->goa); cudaFree(m->got);
   cudaFree(m->dza[0]); cudaFree(m->dza[1]); cudaFree(m->part);
   for (int l = 0; l < NL - 1; ++l) {
@@ -146,7 +166,6 @@ cudaError_t mlp_ensure(izem_mlp* m, int rows) {
   const int nchunks = rows / mlptt::KCMAX;
   m->split_chunks = nchunks / 32 > 1 ? nchunks / 32 : 1;
   m->splits = (nchunks + m->split_chunks - 1) / m->split_chunks;
-  cudaError_t e;
   if ((e = cudaMalloc(&m->xa, M * 16 * 2)) || (e = cudaMalloc(&m->xt, 128 * M * 2)) ||
       (e = cudaMemsetAsync(m->xt, 0, 128 * M * 2, m->s)) ||
       (e = cudaMalloc(&m->gout, M * 16 * 4)) || (e = cudaMalloc(&m->goa, M * 16 * 2)) ||
@@ -182,19 +201,10 @@ cudaError_t step_launch(void (*kern)(Args), dim3 grid, int threads, uint32_t sme
 
 template <int NT, int MODE>
 cudaError_t tg_launch(const mlptt::TgArgs& a, int mt, int nt, int splits, cudaStream_t s) {
-  static bool attr = false;
-  cudaError_t e;
-  if (!attr) {
-    if ((e = cudaFuncSetAttribute(mlptt::k_tgemm<NT, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)mlptt::tg_smem_bytes(NT))) != cudaSuccess)
-      return e;
-    attr = true;
-  }
   return step_launch(mlptt::k_tgemm<NT, MODE>, dim3(mt, nt, splits), mlptt::GT_THREADS, mlptt::tg_smem_bytes(NT), s, a);
 }
 
 constexpr float kBeta1 = 0.9f, kBeta2 = 0.999f;   // Adam
-constexpr int kTileN = 32;   // columns a tile of the forward and input-gradient GEMMs (k_tgemm)
 
 // CTAs over which the weight gradients split a batch of M rows
 int mlp_splits(const izem_mlp* m, int M) { return (M / mlptt::KCMAX + m->split_chunks - 1) / m->split_chunks; }
@@ -286,13 +296,6 @@ cudaError_t mlp_backward(izem_mlp* m, int M) {
     w.err = m->d_err;
     b.first[l + 1] = b.first[l] + w.RA / 128 * ((LOUT[l] + mlptt::WG_NT - 1) / mlptt::WG_NT);
   }
-  static bool attr = false;
-  if (!attr) {
-    if ((e = cudaFuncSetAttribute(mlptt::k_tg_wgrad, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)mlptt::tg_smem_bytes(mlptt::WG_NT))) != cudaSuccess)
-      return e;
-    attr = true;
-  }
   return step_launch(mlptt::k_tg_wgrad, dim3(b.first[NL], splits), mlptt::GT_THREADS, mlptt::tg_smem_bytes(mlptt::WG_NT),
                      m->s, b);
 }
@@ -355,13 +358,6 @@ cudaError_t mlp_infer_tc(izem_mlp* m, int M, const __nv_bfloat16* x, float* y, c
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
     m->blob_dirty = false;
   }
-  static bool attr = false;
-  if (!attr) {
-    if ((e = cudaFuncSetAttribute(mlptc::k_mlp_tc, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)mlptc::SMEM_BYTES)) != cudaSuccess)
-      return e;
-    attr = true;
-  }
   int dev = 0, sms = 0;
   if ((e = cudaGetDevice(&dev)) || (e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev))) return e;
   const int ntiles = (M + mlptc::TM - 1) / mlptc::TM;
@@ -396,7 +392,9 @@ int izem_mlp_create(izem_mlp** out) {
     delete m;
     return IZEM_ERR_CUDA;
   }
-  bool ok = true;
+  // the inference kernel's shared memory on this device (mlp_train_attributes)
+  bool ok = cudaFuncSetAttribute(mlptc::k_mlp_tc, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)mlptc::SMEM_BYTES) == cudaSuccess;
   for (int l = 0; l < NL && ok; ++l) {
     const size_t nw = (size_t)LIN[l] * LOUT[l], nb = LOUT[l];
     ok = !(cudaMalloc(&m->W[l], nw * 4) || cudaMalloc(&m->b[l], nb * 4) || cudaMalloc(&m->Wb[l], nw * 2) ||
