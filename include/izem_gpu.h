@@ -488,6 +488,12 @@ int  izem_gpu_fp64_rate(double* gflops);
  * when it stopped waiting (always, on a working device); the context stays
  * usable. */
 int  izem_gpu_wait_selftest(int polls, int* gave_up);
+/* The same for the barrier of the Newton solve's cooperative launch (no
+ * counterpart in the reference): a solve of no points whose blocks wait for one
+ * more than there are, `polls` times (1 .. 2^20).  Returns IZEM_ERR_TIMEOUT, as
+ * a solve that gives up does (always, on a working device); the state is
+ * untouched and the context stays usable. */
+int  izem_gpu_newton_wait_selftest(izem_ctx* ctx, int polls);
 /* allow = 0 makes the chemistry kernels walk the mechanism's tables even
  * for the shipped mechanism (to compare the two forms); allow = 1 (the
  * default) uses the generated form whenever it applies.  Takes effect at

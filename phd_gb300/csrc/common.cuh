@@ -65,6 +65,11 @@ static __constant__ DevThd c_thd;
 constexpr int kNewtonXBlocksMax = 8;
 constexpr int kNewtonSlots = 10 * kNewtonXBlocksMax;
 
+// Polls of a Newton solve's barrier before it gives up: 1.4 s (0.16 us a poll)
+// on a barrier that some block never reaches.  An iteration over 8.4 million
+// points takes 1 ms, over as many as the GPU's memory holds some 30.
+constexpr int kNewtonPolls = 1 << 23;
+
 // Shared state of one Newton solve (k_newton_solve); all zero between solves.
 struct NewtonShared {
   unsigned long long max[3][kNewtonSlots];   // per slot max dT^2 (bit pattern of a non-negative double), iteration mod 3

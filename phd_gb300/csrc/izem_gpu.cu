@@ -222,26 +222,39 @@ void drop_graphs(izem_ctx* c) {
 // blocks as the points need or the GPU holds at once; the same inside a
 // captured graph and launched directly.
 template <int NRV>
-int enq_newton(izem_ctx* c, int ghost, double eps, int itmax, int check_negT) {
+int launch_newton(izem_ctx* c, int ghost, long long n, int threads, unsigned blocks, double eps, int itmax,
+                  int check_negT, int polls, unsigned absent) {
   const Geo& g = c->g;
   const int d0 = ghost == 2 ? 7 : (ghost ? 1 : 0), d1 = ghost == 2 ? 8 : (ghost ? 6 : 0);
-  const long long n = ghost == 2 ? 2LL * g.n[1] * g.n[2] : (ghost ? slab_count(g) - g.nint : g.nint);
-  const int nxb = g.n[0] / c->newton_bx, threads = tb(c, n);
+  const int nxb = g.n[0] / c->newton_bx;
   int per_sm = 0;
   CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_newton_solve<NRV>, threads, 0));
   cudaLaunchAttribute at{};
   at.id = cudaLaunchAttributeCooperative;
   at.val.cooperative = 1;
   cudaLaunchConfig_t cfg{};
-  cfg.gridDim = dim3((unsigned)std::min<long long>((long long)per_sm * c->nsm, grid_for(n, threads)));
+  cfg.gridDim = dim3((unsigned)std::min<long long>((long long)per_sm * c->nsm, blocks));
   cfg.blockDim = dim3(threads);
   cfg.stream = c->stream;
   cfg.attrs = &at;
   cfg.numAttrs = 1;
   return launch(c, ghost == 2 ? "newton_plane" : (ghost ? "newton_ghost" : "newton"), [&] {
     cudaLaunchKernelEx(&cfg, k_newton_solve<NRV>, g, ghost, n, (const double*)c->v, c->T, c->cp, c->ha, c->d_status,
-                       check_negT, c->newton_bx, d0, d1, nxb, eps, itmax);
+                       check_negT, c->newton_bx, d0, d1, nxb, eps, itmax, polls, absent);
   });
+}
+template <int NRV>
+int enq_newton(izem_ctx* c, int ghost, double eps, int itmax, int check_negT) {
+  const Geo& g = c->g;
+  const long long n = ghost == 2 ? 2LL * g.n[1] * g.n[2] : (ghost ? slab_count(g) - g.nint : g.nint);
+  const int threads = tb(c, n);
+  return launch_newton<NRV>(c, ghost, n, threads, grid_for(n, threads), eps, itmax, check_negT, kNewtonPolls, 0);
+}
+// A solve of no points, one block an SM, whose barrier waits for a block that
+// the grid does not have.
+template <int NRV>
+int newton_wait_selftest(izem_ctx* c, int polls) {
+  return launch_newton<NRV>(c, 0, 0, 32, (unsigned)c->nsm, 1.0, 1, 0, polls, 1);
 }
 
 template <int NRV>
@@ -1683,6 +1696,12 @@ int izem_gpu_kernel_times(izem_ctx* c, int max_kernels, char* names, int name_le
     if (ms) ms[q] = c->kt_ms[q];
   }
   return IZEM_OK;
+}
+
+int izem_gpu_newton_wait_selftest(izem_ctx* c, int polls) {
+  if (!c || polls < 1 || polls > (1 << 20)) return IZEM_ERR_ARG;
+  int rc = IZEM_DISPATCH(c, newton_wait_selftest, c, polls);
+  return rc ? rc : read_status(c);
 }
 
 int izem_gpu_synchronize(izem_ctx* c) {

@@ -224,15 +224,14 @@ __device__ __forceinline__ void newton_point(const Geo& g, int ghost, long long 
   atomic_max_nonneg_warp(&maxdf[dom], nan ? 0.0 : df2);
 }
 
-// Barrier of a cooperative launch: thread 0 waits, a bounded number of polls,
-// until `target` blocks have arrived.  Returns false when it gave up.
-__device__ inline bool grid_barrier(unsigned* arrived, unsigned target) {
+// Barrier of a cooperative launch: thread 0 waits, at most `polls` polls (one or
+// more), until `target` blocks have arrived.  Returns false when it gave up.
+__device__ inline bool grid_barrier(unsigned* arrived, unsigned target, int polls) {
   __shared__ int through;
   __syncthreads();
   if (threadIdx.x == 0) {
     __threadfence();
     atomicAdd(arrived, 1u);
-    int polls = 1 << 26;
     while (*(volatile unsigned*)arrived < target && --polls) {}
     __threadfence();
     through = polls != 0;
@@ -253,11 +252,15 @@ __device__ inline bool grid_barrier(unsigned* arrived, unsigned target) {
 // microseconds on small blocks, where the launches of a loop of an iteration
 // and a test were most of the time: a step of the 400 x 11 shock tube took
 // 0.96 ms so and takes 0.85, of 64^3 2.94 and 2.83, of 256 x 256 x 128 the same.
+// A barrier that some block does not reach gives up after `polls` polls, sets the
+// timeout flag and ends the solve.  `absent` blocks are waited for beyond those
+// of the grid: 0, but for the test of that path.
 template <int NRV>
 __global__ void __launch_bounds__(128) k_newton_solve(Geo g, int ghost, long long n, const double* __restrict__ v,
                                                       double* __restrict__ T, double* __restrict__ cp,
                                                       double* __restrict__ ha, DevStatus* st, int check_negT, int bx,
-                                                      int d0, int d1, int nxb, double eps, int itmax) {
+                                                      int d0, int d1, int nxb, double eps, int itmax,
+                                                      int polls, unsigned absent) {
   __shared__ int done[kNewtonSlots], last;
   NewtonShared& sh = st->newton;
   for (int q = threadIdx.x; q < kNewtonSlots; q += blockDim.x) done[q] = 0;
@@ -269,7 +272,7 @@ __global__ void __launch_bounds__(128) k_newton_solve(Geo g, int ghost, long lon
     unsigned long long* mx = sh.max[it % 3];
     for (long long idx = blockIdx.x * (long long)blockDim.x + threadIdx.x; idx < n; idx += step)
       newton_point<NRV>(g, ghost, idx, v, T, cp, ha, st, check_negT, bx, done, mx);
-    if (!grid_barrier(&sh.arrived, (unsigned)it * gridDim.x)) {
+    if (!grid_barrier(&sh.arrived, (unsigned)it * gridDim.x + absent, polls)) {
       if (threadIdx.x == 0) atomicExch(&st->timeout, 1);
       break;
     }

@@ -69,6 +69,7 @@ def load_library(path=None):
         "izem_gpu_kernel_times": (C.c_int, [P, C.c_int, C.c_char_p, C.c_int, C.POINTER(C.c_int), _dp,
                                             C.POINTER(C.c_int)]),
         "izem_gpu_synchronize": (C.c_int, [P]),
+        "izem_gpu_newton_wait_selftest": (C.c_int, [P, C.c_int]),
         "izem_metrics_dscalar": (C.c_int, [C.c_int, C.c_int, _dp, _dp]),
         "izem_gpu_set_mechanism": (C.c_int, [P, C.POINTER(IzemMech)]),
         "izem_gpu_chem_step": (C.c_int, [P, C.c_double, C.c_double, C.c_int, _dp]),
@@ -438,6 +439,12 @@ class IzemGPU:
 
     def synchronize(self):
         self._check(self.lib.izem_gpu_synchronize(self.h), "synchronize")
+
+    def newton_wait_selftest(self, polls=4096):
+        """A Newton solve of no points whose barrier cannot be reached: raises
+        IzemError (IZEM_ERR_TIMEOUT) after `polls` polls
+        (izem_gpu_newton_wait_selftest)."""
+        self._check(self.lib.izem_gpu_newton_wait_selftest(self.h, int(polls)), "newton_wait_selftest")
 
 
 CHEM_BDF, CHEM_MLP = 0, 1
