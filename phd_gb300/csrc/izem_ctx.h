@@ -48,7 +48,7 @@ struct izem_ctx {
   // one block) and the block-edge faces as seen by the right block
   int sensor_bx = 0;
   int newton_bx = 0;   // x-block size of the Newton stopping test (nx: one block)
-  int nsm = 0;         // SMs of the context's device (the host-transfer kernel's grid)
+  int nsm = 0;         // SMs that the context may use (launch shapes, the Newton solve's grid)
   int sensor_type = 0;          // IZEM_SENSOR_ADAMS_SHARIFF or IZEM_SENSOR_DUCROS
   double ducros_treduc = 0.2;   // DUCROS_TREDUC
   double* fhat_edge = nullptr;

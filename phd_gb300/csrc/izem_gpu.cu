@@ -10,6 +10,7 @@
 #include <string>
 #include <vector>
 #include <algorithm>
+#include <cuda.h>
 #include <cuda_runtime.h>
 
 #include "common.cuh"
@@ -799,15 +800,38 @@ int izem_gpu_init(const izem_cfg* cfg, const izem_thd* thd, const izem_adi* adi,
 
 }  // extern "C"
 
+// SMs that the current CUDA context may use: the device's, or those of the
+// partition that a green context was given.  A cooperative launch (the Newton
+// solve) must fit into them at once; one sized by the device's fails there.
+// Called with a context current (the stream's creation makes one).
+static cudaError_t context_sms(int* n) {
+  int dev = 0;
+  cudaError_t e;
+  if ((e = cudaGetDevice(&dev)) || (e = cudaDeviceGetAttribute(n, cudaDevAttrMultiProcessorCount, dev))) return e;
+  auto entry = [](const char* name, unsigned version) -> void* {
+    void* f = nullptr;
+    cudaDriverEntryPointQueryResult found;
+    if (cudaGetDriverEntryPointByVersion(name, &f, version, cudaEnableDefault, &found) != cudaSuccess) {
+      (void)cudaGetLastError();
+      return nullptr;
+    }
+    return found == cudaDriverEntryPointSuccess ? f : nullptr;
+  };
+  const auto current = (CUresult(*)(CUcontext*))entry("cuCtxGetCurrent", 4000);
+  const auto resource = (CUresult(*)(CUcontext, CUdevResource*, CUdevResourceType))entry("cuCtxGetDevResource", 12040);
+  CUcontext ctx = nullptr;
+  CUdevResource r{};
+  if (current && resource && current(&ctx) == CUDA_SUCCESS && ctx &&
+      resource(ctx, &r, CU_DEV_RESOURCE_TYPE_SM) == CUDA_SUCCESS && r.sm.smCount > 0)
+    *n = std::min(*n, (int)r.sm.smCount);
+  return cudaSuccess;
+}
+
 int ctx_alloc(izem_ctx* c) {
   const Geo& g = c->g;
   const int nv = c->nv, nrv = c->cfg.nrv;
   CK(cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking));
-  {
-    int dev = 0;
-    CK(cudaGetDevice(&dev));
-    CK(cudaDeviceGetAttribute(&c->nsm, cudaDevAttrMultiProcessorCount, dev));
-  }
+  CK(context_sms(&c->nsm));
   // All set-up work goes to the context's stream, here and in the setters below:
   // the stream is non-blocking, so that nothing orders its kernels after a copy or
   // a fill on the default stream, and both may return before they are done.
