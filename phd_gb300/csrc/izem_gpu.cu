@@ -61,7 +61,9 @@ int face_share(const izem_ctx* c, long long faces) {
 // the FP64 pipe is full.  Limits of 8, 16 and 32 warps are alike.  Gradients and
 // divergence of the 400 x 11 shock tube 22.3 -> 9.9 and 22.4 -> 9.2 us, of 33 x
 // 40 x 21 35 -> 29 and 37 -> 27; a pass of the former 15.95 -> 14.23 ms, a step
-// of the latter 6.8 -> 6.6.
+// of the latter 6.8 -> 6.6.  The periodic wrap of the latter (4 warps an SM) 27
+// -> 11 us with eight rows; of 256 x 256 x 128 (160) 238 -> 253 with eight, and
+// of its four LES components 33 -> 51 with four: one row there.
 int rows_for(const izem_ctx* c, long long n, int parts) {
   const long long warps = (n + 31) / 32, fit = 32LL * c->nsm / warps;
   return fit >= parts ? parts : (fit < 2 ? 1 : (int)fit);
@@ -342,9 +344,9 @@ int enq_visc(izem_ctx* c) {
               })))
     return rc;
   long long ns = slab_count(g) - g.nint;
-  if ((rc = launch(c, "visc_wrap", [&] { k_wrap_periodic<<<dim3(grid_for(ns, tb(c, ns)), 8), tb(c, ns), 0, c->stream>>>(g, nderiv, c->fd); })))
+  if ((rc = launch(c, "visc_wrap", [&] { k_wrap_periodic<<<dim3(grid_for(ns, tb(c, ns)), rows_for(c, ns, 8)), tb(c, ns), 0, c->stream>>>(g, nderiv, c->fd); })))
     return rc;
-  if (les && (rc = launch(c, "les_wrap", [&] { k_wrap_periodic<<<dim3(grid_for(ns, tb(c, ns)), 4), tb(c, ns), 0, c->stream>>>(g, 4, c->les); })))
+  if (les && (rc = launch(c, "les_wrap", [&] { k_wrap_periodic<<<dim3(grid_for(ns, tb(c, ns)), rows_for(c, ns, 4)), tb(c, ns), 0, c->stream>>>(g, 4, c->les); })))
     return rc;
   const long long ns_all = slab_count(g);
   const int tv = tb_or(c, c->tb_visc, ns_all);
