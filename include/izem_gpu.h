@@ -177,6 +177,11 @@ typedef struct izem_ctx izem_ctx;
  * Supported: ng = 3 (WENO5) or ng = 4 (WENO7), two or nine species, in 3-D
  * or 2-D; ndim = 2 needs nz = 1 (no z sweep, no z derivatives); EGLIB
  * transport in 3-D.  Other configurations return IZEM_ERR_ARG.
+ * The species data (thd, adi), EGLIB's linking data (izem_gpu_set_eglib) and the
+ * mechanism are constants of the process on its device: the set given last, by
+ * any context or batch call, holds for all.  Several contexts of one set may run
+ * at once, from several threads; contexts of different sets may not be used in
+ * turn, only one after the other.
  * Replaces the allocations at module_solver.f90:736-739 and the per-call
  * temporaries of module_weno.f90:588-607, module_viscflux.f90:1708-1714. */
 int  izem_gpu_init(const izem_cfg* cfg, const izem_thd* thd, const izem_adi* adi,
@@ -246,7 +251,10 @@ int  izem_gpu_nr_flux(izem_ctx* ctx);
 
 /* EGLIB linking data for cfg.eglib = 1 (init_eglib + EGINI,
  * module_eg_lib.f90:44-96, eglib/EGini.f:58-301); call once after
- * izem_gpu_init and before any viscous flux. */
+ * izem_gpu_init and before any viscous flux.  Tabulates the data's functions of
+ * the temperature for this context (2.5 ms, 12.7 MB with nine species); setting
+ * other data tabulates them anew.  See izem_gpu_init for contexts with different
+ * data. */
 int  izem_gpu_set_eglib(izem_ctx* ctx, const izem_eglib* eglib);
 
 /* upd_prim_var_domain + comm_cons + upd_boundaries + upd_prim_var_ghost
@@ -385,6 +393,8 @@ int  izem_mlp_set_norm(izem_mlp* m, const float* norm);
 int  izem_mlp_forward(izem_mlp* m, int M, const float* x, float* y);
 int  izem_mlp_grads(izem_mlp* m, int M, const float* x, const float* t, double* loss,
                     float* const* gW, float* const* gb);
+/* Host arrays (device_ptrs = 0) are copied to the device on every call; of that
+ * memory the handle keeps up to 64 MB for the next call, until it is destroyed. */
 int  izem_mlp_train(izem_mlp* m, long long n, const float* x, const float* t, int device_ptrs,
                     int epochs, int batch, float lr, unsigned seed, double* losses);
 /* Surrogate chemistry step on independent reactors with the per-cell error

@@ -534,8 +534,8 @@ HD void ck_fun_fast(double rho, const double* z, double* zp) {
 // Right-hand-side policies of the BDF driver: the generic form, which walks
 // the uploaded mechanism's tables, and the generated form of the mechanism
 // the library was built with (chem_gen.cuh, phd_gb300/mechgen.py), which
-// performs the same operations in the same order with the tables as
-// literals.  chem_upload_mech picks the generated form when the uploaded
+// performs the same operations in the same order with that mechanism's numbers
+// in literals and constant tables of its own.  chem_upload_mech picks the generated form when the uploaded
 // mechanism is that one.
 template <int KK>
 struct RhsTables {

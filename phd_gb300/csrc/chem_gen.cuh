@@ -1,7 +1,8 @@
 // Generated by phd_gb300/mechgen.py from phd_gb300/data/h2_sandiego12.inp -- do not edit.
 // The constant-volume reactor right-hand side of this mechanism (9 species,
-// 12 reactions) as straight-line code: the expressions and operation order of
-// fun_tpart / fun_cpart in chem.cu with the mechanism's tables as literals.
+// 12 reactions): the expressions and operation order of fun_tpart / fun_cpart
+// in chem.cu, the composition part straight-line code with the mechanism's numbers
+// as literals, the Arrhenius and NASA terms loops over constant tables.
 #pragma once
 
 namespace chem_gen {

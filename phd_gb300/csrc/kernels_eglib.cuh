@@ -10,9 +10,11 @@
 // (conductivity and rescaled thermal diffusion ratios, a direct
 // factorisation of Lambda_[e]) and EGSDR1 (rho times the flux diffusion
 // matrix, two stationary steps on L_[00] and the mass-conservation
-// projection), in the reference's operation order.  EGSL2 and EGSK2, also
-// called there, only produce values that the reference discards (the
-// conductivity is recomputed by EGSLCT2 and the volume viscosity is set to
+// projection).  The formulas are the reference's, the order of operations is
+// not: what depends on the temperature alone comes from a table (eg_table.cuh),
+// and rho D is applied to the driving forces and never formed (EgPoint).  EGSL2
+// and EGSK2, also called there, only produce values that the reference discards
+// (the conductivity is recomputed by EGSLCT2 and the volume viscosity is set to
 // zero, module_eg_lib.f90:288).
 //
 // The species gradients keep the fitted-transport layout of fd
@@ -166,10 +168,6 @@ inline void eg_prepare(const izem_eglib& L, const izem_thd& t, const izem_adi& a
 }
 
 #include "eg_table.cuh"
-
-// packed symmetric index of EGLIB (0-based, i <= j)
-template <int N>
-__host__ __device__ constexpr int egs(int i, int j) { return N * i - (i * (i + 1)) / 2 + j; }
 
 // Species cp of egvars (module_eg_lib.f90:170-240): NASA-7 with the linear
 // extrapolation outside [Tpolymin, Tpolymax], in erg/g/K.

@@ -194,7 +194,10 @@ __device__ __forceinline__ void newton_point(const Geo& g, int ghost, long long 
   if (done[dom]) return;
   const long long nc = g.ncell;
   const long long p = gid(g, i, j, k);
-  // F = e(T) - e of the conserved state, with the sums over rho Y_k
+  // F = e(T) - e of the conserved state, with the sums over rho Y_k: the species
+  // sums first, then the kinetic and the total energy.  Of the orders of equal
+  // cost it is the one for which the time step after an RK3 step has the oracle's
+  // bits (tests/test_gpu_strang.py compares them)
   const double rho_i = fm_rcp(v[p]);
   const double v2 = v[nc + p], v3 = v[2 * nc + p], v4 = v[3 * nc + p];
   double F = 0.0;

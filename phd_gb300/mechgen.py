@@ -1,5 +1,5 @@
 """Mechanism compiler: the constant-volume reactor right-hand side of one
-CHEMKIN mechanism as straight-line CUDA code.
+CHEMKIN mechanism as CUDA code of its own.
 
 The chemistry kernels evaluate CHEMKIN's rate expressions (CKCVBS, CKHMS,
 CKRATT, CKRATX, CKWYR; chemkin/vode.f) for whatever mechanism the caller
@@ -7,8 +7,11 @@ uploads, walking its reaction tables at run time.  Species concentrations,
 rates of progress and production rates are then indexed by table entries,
 so they live in local memory, and every term costs a table load and a
 branch.  For a mechanism known when the library is built this module writes
-the same expressions, in the same operation order, with the table entries
-as literals: reaction loops unrolled, indices fixed, absent terms dropped.
+the same expressions, in the same operation order, for its reactions alone:
+in the composition part the reaction loops are unrolled, indices fixed, absent
+terms dropped and the table entries literals; the Arrhenius and NASA terms of
+the temperature part stay loops, over constant tables, since unrolled they
+push the integrator out of the instruction cache.
 The arithmetic is the generic form's (fun_tpart / fun_cpart in chem.cu),
 operation for operation, so a host build of the two gives identical bits.
 
@@ -109,8 +112,9 @@ def generate(m, name="h2air9", source="phd_gb300/data/h2_sandiego12.inp"):
     w = L.append
     w("// Generated by phd_gb300/mechgen.py from %s -- do not edit." % source)
     w("// The constant-volume reactor right-hand side of this mechanism (%d species," % kk)
-    w("// %d reactions) as straight-line code: the expressions and operation order of" % m.ii)
-    w("// fun_tpart / fun_cpart in chem.cu with the mechanism's tables as literals.")
+    w("// %d reactions): the expressions and operation order of fun_tpart / fun_cpart" % m.ii)
+    w("// in chem.cu, the composition part straight-line code with the mechanism's numbers")
+    w("// as literals, the Arrhenius and NASA terms loops over constant tables.")
     w("#pragma once")
     w("")
     w("namespace chem_gen {")
